@@ -244,6 +244,27 @@ __device__ __forceinline__ double cell_width2(const DeviceScalars* s, const Batc
     return ldexp(b.w2[b.uid[i]], -2 * (level - kBatchUidDigits));
 }
 
+// m r^-3 from r^2 (FP64): the hardware's approximate 1/sqrt y (about 20 bits),
+// corrected by the binomial series of (1 - e)^(-3/2), e = 1 - r^2 y^2, to its
+// second-order term; e^3 is below 2^-57.  Seven FP64 instructions.  y has so
+// few bits that y^2 is exact, so e carries one rounding.  For r^2 in
+// normal_range(); m_over_r3_any() takes the rest.
+__device__ __forceinline__ double m_over_r3(double m, double r2) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+    const double t = __dmul_rn(y, y);
+    const double e = __fma_rn(-r2, t, 1.0);
+    const double w = __dmul_rn(__dmul_rn(m, y), t);
+    return __fma_rn(w, __dmul_rn(e, __fma_rn(1.875, e, 1.5)), w);
+}
+__device__ __forceinline__ bool normal_range(double x) {  // positive, normal and finite
+    return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u;
+}
+__device__ __forceinline__ double m_over_r3_any(double m, double r2) {
+    const double inv = rsqrt(r2);
+    return m * (inv * inv * inv);
+}
+
 // Number of radix passes (top bytes of the key) a sort should take, from the
 // histogram of shared leading digits of neighbouring sorted codes: the fewest
 // passes that leave at most n / 32 neighbouring pairs tied; 8 without data.
