@@ -18,36 +18,150 @@
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;
+constexpr int kTile = 256;    // sources staged in shared memory at a time
 
-__global__ void __launch_bounds__(kThreads)
-allpairs_fp64(const double2* __restrict__ pos, const double* __restrict__ mass, int64_t n,
-              const int64_t* __restrict__ targets, int64_t k, double eps2, double2* __restrict__ acc) {
-    __shared__ double2 sp[kThreads];
-    __shared__ double sm[kThreads];
-    const int64_t t = blockIdx.x * (int64_t)kThreads + threadIdx.x;
-    const int64_t me = t < k ? targets[t] : -1;
-    const double2 p = me >= 0 ? pos[me] : make_double2(0.0, 0.0);
-    double ax = 0.0, ay = 0.0;
-    for (int64_t base = 0; base < n; base += kThreads) {
-        const int64_t j = base + threadIdx.x;
-        sp[threadIdx.x] = j < n ? pos[j] : make_double2(0.0, 0.0);
-        sm[threadIdx.x] = j < n ? mass[j] : 0.0;
+using nb::m_over_r3;
+using nb::normal_range;
+
+// Pair weight w of a_i += w (p_j - p_i).  kCpuLaw: the law of
+// Simulation::force, m / (d (d^2 + eps2)) (Simulation.cpp:74-80, G applied
+// with the kick); otherwise Plummer's m (d^2 + eps2)^-3/2.
+template <bool kCpuLaw>
+__device__ __forceinline__ double pair_weight(double m, double r2, double eps2) {
+    return kCpuLaw ? nb::m_over_r_s(m, r2, r2 + eps2) : m_over_r3(m, r2 + eps2);
+}
+// The same for any r2: zero, subnormal or infinite squares.
+template <bool kCpuLaw>
+__device__ __forceinline__ double pair_weight_any(double m, double r2, double eps2) {
+    if (kCpuLaw) return m / (sqrt(r2) * (r2 + eps2));
+    const double inv = 1.0 / sqrt(r2 + eps2);
+    return m * inv * inv * inv;
+}
+
+// Sums the sources [s0, s1) for the block's targets, kPer per thread: target
+// b of a thread is p[b], and self[b] its own source index, which is left out.
+// 13 FP64 instructions per pair (22 with the CPU law), each two issue cycles:
+// the FP64 pipe is the bound (1 / sqrt and its division took some 35: 65,536
+// targets of 1,048,576 bodies with their copies 205 -> 70 ms; a step of 20,011
+// bodies 0.92 -> 0.38 ms).  Several targets per thread share the loads and
+// the loop.  Only a tile that holds one of the warp's own sources tests for
+// it; a tile whose sums are not finite (a square that is zero, subnormal or
+// infinite) is summed again with full-range functions.
+template <bool kCpuLaw, int kPer>
+__device__ __forceinline__ void sum_sources(const double2* __restrict__ pos,
+                                            const double* __restrict__ mass, int64_t s0, int64_t s1,
+                                            double eps2, const double2 (&p)[kPer],
+                                            const int64_t (&self)[kPer], double (&ax)[kPer],
+                                            double (&ay)[kPer]) {
+    __shared__ double2 sp[kTile];
+    __shared__ double sm[kTile];
+    for (int64_t base = s0; base < s1; base += kTile) {
+        const int lim = (int)min((int64_t)kTile, s1 - base);
+        for (int q = threadIdx.x; q < lim; q += kThreads) {
+            sp[q] = pos[base + q];
+            sm[q] = mass[base + q];
+        }
         __syncthreads();
-        const int lim = (int)min((int64_t)kThreads, n - base);
-        for (int q = 0; q < lim; ++q) {
-            if (base + q == me) continue;
-            const double dx = sp[q].x - p.x;
-            const double dy = sp[q].y - p.y;
-            const double d2 = dx * dx + dy * dy + eps2;
-            const double inv_r = 1.0 / sqrt(d2);
-            const double a = sm[q] * inv_r * inv_r * inv_r;
-            ax += dx * a;
-            ay += dy * a;
+        double bx[kPer], by[kPer];
+        bool own = false, odd = false;
+#pragma unroll
+        for (int b = 0; b < kPer; ++b) {
+            bx[b] = ax[b];
+            by[b] = ay[b];
+            own |= self[b] >= base && self[b] < base + lim;
+        }
+        if (!__any_sync(0xffffffffu, own)) {
+#pragma unroll 4
+            for (int q = 0; q < lim; ++q)
+#pragma unroll
+                for (int b = 0; b < kPer; ++b) {
+                    const double dx = sp[q].x - p[b].x, dy = sp[q].y - p[b].y;
+                    const double w = pair_weight<kCpuLaw>(sm[q], fma(dx, dx, dy * dy), eps2);
+                    bx[b] = fma(dx, w, bx[b]);
+                    by[b] = fma(dy, w, by[b]);
+                }
+        } else {
+            for (int q = 0; q < lim; ++q)
+#pragma unroll
+                for (int b = 0; b < kPer; ++b) {
+                    const double dx = sp[q].x - p[b].x, dy = sp[q].y - p[b].y;
+                    const double w = pair_weight<kCpuLaw>(sm[q], fma(dx, dx, dy * dy), eps2);
+                    if (base + q != self[b]) {
+                        bx[b] = fma(dx, w, bx[b]);
+                        by[b] = fma(dy, w, by[b]);
+                    }
+                }
+        }
+#pragma unroll
+        for (int b = 0; b < kPer; ++b) odd |= !(isfinite(bx[b]) && isfinite(by[b]));
+        if (odd) {
+            for (int q = 0; q < lim; ++q)
+#pragma unroll 1
+                for (int b = 0; b < kPer; ++b) {
+                    const double dx = sp[q].x - p[b].x, dy = sp[q].y - p[b].y;
+                    if (base + q == self[b]) continue;
+                    const double w = pair_weight_any<kCpuLaw>(sm[q], fma(dx, dx, dy * dy), eps2);
+                    ax[b] += dx * w;
+                    ay[b] += dy * w;
+                }
+        } else {
+#pragma unroll
+            for (int b = 0; b < kPer; ++b) {
+                ax[b] = bx[b];
+                ay[b] = by[b];
+            }
         }
         __syncthreads();
     }
-    if (t < k) acc[t] = make_double2(ax, ay);
+}
+
+// Block (x, y) sums targets x * kThreads * kPer.. over source chunk y: few
+// targets split the sources so that the grid fills the GPU, and the partial
+// sums are added in chunk order (deterministic).  targets == nullptr: target
+// i is body i.
+template <bool kCpuLaw, int kPer>
+__global__ void __launch_bounds__(kThreads)
+allpairs_partial(const double2* __restrict__ pos, const double* __restrict__ mass, int64_t n,
+                 const int64_t* __restrict__ targets, int64_t k, int64_t chunk, double eps2,
+                 double2* __restrict__ partial) {
+    const int64_t first = blockIdx.x * (int64_t)(kThreads * kPer) + threadIdx.x;
+    double2 p[kPer];
+    int64_t self[kPer];
+    double ax[kPer], ay[kPer];
+#pragma unroll
+    for (int b = 0; b < kPer; ++b) {
+        const int64_t i = min(first + b * kThreads, k - 1);
+        self[b] = targets ? targets[i] : i;
+        p[b] = pos[self[b]];
+        ax[b] = ay[b] = 0.0;
+    }
+    const int64_t s0 = blockIdx.y * chunk, s1 = min(n, s0 + chunk);
+    sum_sources<kCpuLaw, kPer>(pos, mass, s0, s1, eps2, p, self, ax, ay);
+#pragma unroll
+    for (int b = 0; b < kPer; ++b) {
+        const int64_t i = first + b * kThreads;
+        if (i < k) partial[blockIdx.y * k + i] = make_double2(ax[b], ay[b]);
+    }
+}
+
+// Target i's partial sums added in chunk order (loads of eight in flight).
+__device__ __forceinline__ double2 fold_partial(const double2* __restrict__ partial, int chunks,
+                                                int64_t k, int64_t i) {
+    double ax = 0.0, ay = 0.0;
+#pragma unroll 8
+    for (int c = 0; c < chunks; ++c) {
+        const double2 a = partial[c * k + i];
+        ax += a.x;
+        ay += a.y;
+    }
+    return make_double2(ax, ay);
+}
+
+__global__ void allpairs_fold(const double2* __restrict__ partial, int chunks, int64_t k,
+                              double2* __restrict__ acc) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < k) acc[i] = fold_partial(partial, chunks, k, i);
 }
 
 // NB_MODE_ALLPAIRS, stage 1 (AllPairs.cpp:31-35): b = a with x += v dt (or a
@@ -63,96 +177,72 @@ __global__ void allpairs_drift(nb::BodyBuffers a, nb::BodyBuffers b, int64_t n, 
     b.orig[i] = a.orig[i];
 }
 
-// Stage 2 (AllPairs.cpp:38-49): every body sums all others (each pair is
-// evaluated from both sides: twice the reference's pair evaluations, no
-// atomics).  kCpuLaw: the law of Simulation::force,
-// a = m (p_j - p_i) / (d (d^2 + eps2)) (Simulation.cpp:74-80, G applied with
-// the kick); otherwise Plummer's a = m (p_j - p_i) (d^2 + eps2)^-3/2.  Block
-// (x, y) sums targets x*256.. over source chunk y; small systems split the
-// sources into chunks so that the grid fills the GPU, and the partial sums
-// are added in chunk order by the kick (deterministic).
-template <bool kCpuLaw>
-__global__ void __launch_bounds__(kThreads)
-allpairs_partial(const double2* __restrict__ pos, const double* __restrict__ mass, int64_t n,
-                 int64_t chunk, double eps2, double2* __restrict__ partial) {
-    __shared__ double2 sp[kThreads];
-    __shared__ double sm[kThreads];
-    const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
-    const double2 p = i < n ? pos[i] : make_double2(0.0, 0.0);
-    const int64_t s0 = blockIdx.y * chunk, s1 = min(n, s0 + chunk);
-    double ax = 0.0, ay = 0.0;
-    for (int64_t base = s0; base < s1; base += kThreads) {
-        const int64_t j = base + threadIdx.x;
-        sp[threadIdx.x] = j < s1 ? pos[j] : make_double2(0.0, 0.0);
-        sm[threadIdx.x] = j < s1 ? mass[j] : 0.0;
-        __syncthreads();
-        const int lim = (int)min((int64_t)kThreads, s1 - base);
-        for (int q = 0; q < lim; ++q) {
-            if (base + q == i) continue;
-            const double dx = sp[q].x - p.x;
-            const double dy = sp[q].y - p.y;
-            const double r2 = dx * dx + dy * dy;
-            double a;
-            if (kCpuLaw) {
-                a = sm[q] / (sqrt(r2) * (r2 + eps2));
-            } else {
-                const double inv_r = 1.0 / sqrt(r2 + eps2);
-                a = sm[q] * inv_r * inv_r * inv_r;
-            }
-            ax += dx * a;
-            ay += dy * a;
-        }
-        __syncthreads();
-    }
-    if (i < n) partial[blockIdx.y * n + i] = make_double2(ax, ay);
-}
-
+// Stage 2 (AllPairs.cpp:38-49): every body sums all others (allpairs_partial;
+// each pair is evaluated from both sides: twice the reference's pair
+// evaluations, no atomics), then the kick.
 __global__ void allpairs_kick(const double2* __restrict__ partial, int chunks, int64_t n,
                               double2* __restrict__ vel, double2* __restrict__ acc_out,
                               double G_dt, int kick, unsigned long long* __restrict__ body_terms) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double ax = 0.0, ay = 0.0;
-    for (int c = 0; c < chunks; ++c) {
-        const double2 a = partial[c * n + i];
-        ax += a.x;
-        ay += a.y;
-    }
-    if (acc_out) acc_out[i] = make_double2(ax, ay);
+    const double2 a = fold_partial(partial, chunks, n, i);
+    if (acc_out) acc_out[i] = a;
     if (kick) {
         double2 v = vel[i];
-        v.x += ax * G_dt;
-        v.y += ay * G_dt;
+        v.x += a.x * G_dt;
+        v.y += a.y * G_dt;
         vel[i] = v;
     }
     if (threadIdx.x == 0)
         atomicAdd(body_terms, (unsigned long long)min((int64_t)blockDim.x, n - i) * (n - 1));
 }
 
+// Two targets per thread share each source's load; below this many targets
+// one per thread fills the GPU better.
+constexpr int64_t kTwoPerThread = 16384;
+
+inline int64_t target_blocks(int64_t k) {
+    const int64_t per = kThreads * (k >= kTwoPerThread ? 2 : 1);
+    return (k + per - 1) / per;
+}
+
+// Source chunks for k targets and n sources: four waves of eight blocks per
+// SM, so that the last wave costs little (and the partial sums, 16 bytes per
+// target and chunk, stay below 20 MB), with chunks of at least 32 sources.
+inline int source_chunks(int64_t k, int64_t n, int sm_count) {
+    const int64_t want = (int64_t)sm_count * 8 * 4 / target_blocks(k);
+    return (int)std::max<int64_t>(1, std::min<int64_t>({want, n / 32, 256}));
+}
+
+template <bool kCpuLaw>
+void launch_partial(const double2* pos, const double* mass, int64_t n, const int64_t* targets,
+                    int64_t k, int chunks, double eps2, double2* partial, cudaStream_t st) {
+    const dim3 grid((unsigned)target_blocks(k), (unsigned)chunks);
+    const int64_t chunk = (n + chunks - 1) / chunks;
+    if (k >= kTwoPerThread)
+        allpairs_partial<kCpuLaw, 2><<<grid, kThreads, 0, st>>>(pos, mass, n, targets, k, chunk, eps2,
+                                                               partial);
+    else
+        allpairs_partial<kCpuLaw, 1><<<grid, kThreads, 0, st>>>(pos, mass, n, targets, k, chunk, eps2,
+                                                               partial);
+}
+
 }  // namespace
 
-int nb::allpairs_chunks(int64_t n, int sm_count) {
-    const int64_t xblocks = (n + kThreads - 1) / kThreads;
-    const int64_t want = (int64_t)sm_count * 8;  // blocks to fill the GPU a few times over
-    int64_t chunks = (want + xblocks - 1) / xblocks;
-    chunks = std::min<int64_t>(chunks, std::max<int64_t>(1, n / kThreads));
-    return (int)std::max<int64_t>(1, std::min<int64_t>(chunks, 64));
-}
+int nb::allpairs_chunks(int64_t n, int sm_count) { return source_chunks(n, n, sm_count); }
 
 void nb::launch_allpairs_step(nb_ctx* c, const BodyBuffers& a, const BodyBuffers& b, bool integrate,
                               bool store_acc) {
     const unsigned blocks = (unsigned)((c->n + kThreads - 1) / kThreads);
     const int chunks = allpairs_chunks(c->n, c->sm_count);
-    const int64_t chunk = (c->n + chunks - 1) / chunks;
     c->launches += 3;
     allpairs_drift<<<blocks, kThreads, 0, c->stream>>>(a, b, c->n, integrate ? c->p.timestep : 0.0);
-    const dim3 grid(blocks, (unsigned)chunks);
     if (c->p.flags & NB_FLAG_CPU_LAW)
-        allpairs_partial<true><<<grid, kThreads, 0, c->stream>>>(b.pos, b.mass, c->n, chunk,
-                                                                c->p.epsilon_squared, c->ap_partial);
+        launch_partial<true>(b.pos, b.mass, c->n, nullptr, c->n, chunks, c->p.epsilon_squared,
+                             c->ap_partial, c->stream);
     else
-        allpairs_partial<false><<<grid, kThreads, 0, c->stream>>>(b.pos, b.mass, c->n, chunk,
-                                                                 c->p.epsilon_squared, c->ap_partial);
+        launch_partial<false>(b.pos, b.mass, c->n, nullptr, c->n, chunks, c->p.epsilon_squared,
+                              c->ap_partial, c->stream);
     allpairs_kick<<<blocks, kThreads, 0, c->stream>>>(c->ap_partial, chunks, c->n, b.vel,
                                                        store_acc ? c->acc : nullptr,
                                                        c->p.G * c->p.timestep, integrate ? 1 : 0,
@@ -172,25 +262,30 @@ extern "C" int nb_allpairs_accelerations(int32_t device, uint64_t n, const doubl
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(device);
-    double2 *dpos = nullptr, *dacc = nullptr;
+    double2 *dpos = nullptr, *dacc = nullptr, *dpart = nullptr;
     double* dmass = nullptr;
     int64_t* dtgt = nullptr;
     cudaStream_t st = nullptr;
-    int rc = NB_OK;
+    int rc = NB_OK, sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int chunks = source_chunks((int64_t)k, (int64_t)n, sms > 0 ? sms : 1);
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc(&dpos, n * sizeof(double2)) != cudaSuccess ||
         cudaMalloc(&dmass, n * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&dtgt, k * sizeof(int64_t)) != cudaSuccess ||
-        cudaMalloc(&dacc, k * sizeof(double2)) != cudaSuccess) {
+        cudaMalloc(&dacc, k * sizeof(double2)) != cudaSuccess ||
+        (chunks > 1 && cudaMalloc(&dpart, k * chunks * sizeof(double2)) != cudaSuccess)) {
         rc = NB_ERR_NOMEM;
     }
     if (rc == NB_OK) {
         cudaMemcpyAsync(dpos, pos_xy, n * sizeof(double2), cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(dmass, mass, n * sizeof(double), cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(dtgt, targets, k * sizeof(int64_t), cudaMemcpyHostToDevice, st);
-        const unsigned blocks = (unsigned)((k + kThreads - 1) / kThreads);
-        allpairs_fp64<<<blocks, kThreads, 0, st>>>(dpos, dmass, (int64_t)n, dtgt, (int64_t)k,
-                                                   epsilon_squared, dacc);
+        launch_partial<false>(dpos, dmass, (int64_t)n, dtgt, (int64_t)k, chunks, epsilon_squared,
+                              chunks > 1 ? dpart : dacc, st);
+        if (chunks > 1)
+            allpairs_fold<<<(unsigned)((k + kThreads - 1) / kThreads), kThreads, 0, st>>>(
+                dpart, chunks, (int64_t)k, dacc);
         cudaMemcpyAsync(acc_xy, dacc, k * sizeof(double2), cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess)
             rc = NB_ERR_CUDA;
@@ -199,6 +294,7 @@ extern "C" int nb_allpairs_accelerations(int32_t device, uint64_t n, const doubl
     cudaFree(dmass);
     cudaFree(dtgt);
     cudaFree(dacc);
+    cudaFree(dpart);
     if (st) cudaStreamDestroy(st);
     cudaSetDevice(prev);
     return rc;

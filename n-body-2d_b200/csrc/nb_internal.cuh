@@ -257,6 +257,17 @@ __device__ __forceinline__ double m_over_r3(double m, double r2) {
     const double w = __dmul_rn(__dmul_rn(m, y), t);
     return __fma_rn(w, __dmul_rn(e, __fma_rn(1.875, e, 1.5)), w);
 }
+// m / (sqrt(r2) s), s > 0 normal (FP64): approximate 1/sqrt and reciprocal, then
+// the same series for the exponent -1/2, with e = 1 - r2 (s u)^2.
+__device__ __forceinline__ double m_over_r_s(double m, double r2, double s) {
+    double y, z;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(s));
+    const double u = __dmul_rn(y, z), v = __dmul_rn(s, u);
+    const double e = __fma_rn(-__dmul_rn(r2, v), v, 1.0);
+    const double w = __dmul_rn(m, u);
+    return __fma_rn(w, __dmul_rn(e, __fma_rn(0.375, e, 0.5)), w);
+}
 __device__ __forceinline__ bool normal_range(double x) {  // positive, normal and finite
     return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u;
 }
