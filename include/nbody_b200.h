@@ -266,11 +266,12 @@ NB_API int nb_debug_groups(nb_ctx* ctx, int32_t* first_body, int32_t* last_body,
 
 NB_API int nb_get_stats(nb_ctx* ctx, nb_stats* out);
 
-/* Device time of each phase of the most recent graph-launched step, from CUDA
- * events recorded inside the step graph (the GPU counterpart of the phase
+/* Device time of each phase of the most recent graph-launched step, from
+ * device timestamps that its kernels write (the GPU counterpart of the phase
  * StopWatches of the reference CPU backend, src/Simulation/src/BarnesHut.cpp:
- * 22-25, 52-64).  Writes up to max values to ms and returns the number of
- * phases (>= 0) or a negative NB_* status.  Phase k is named by
+ * 22-25, 52-64); 0 for a phase that the context's mode does not have, -1
+ * before the first step.  Writes up to max values to ms and returns the number
+ * of phases (>= 0) or a negative NB_* status.  Phase k is named by
  * nb_phase_name(k). */
 NB_API int nb_phase_times(nb_ctx* ctx, double* ms, int max);
 NB_API const char* nb_phase_name(int phase);

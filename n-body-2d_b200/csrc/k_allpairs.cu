@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(kThreads)
 allpairs_partial(const double2* __restrict__ pos, const double* __restrict__ mass, int64_t n,
                  const int64_t* __restrict__ targets, int64_t k, int64_t chunk, double eps2,
                  double2* __restrict__ partial) {
+    nb::chain_begin();
     const int64_t first = blockIdx.x * (int64_t)(kThreads * kPer) + threadIdx.x;
     double2 p[kPer];
     int64_t self[kPer];
@@ -166,7 +167,15 @@ __global__ void allpairs_fold(const double2* __restrict__ partial, int chunks, i
 
 // NB_MODE_ALLPAIRS, stage 1 (AllPairs.cpp:31-35): b = a with x += v dt (or a
 // plain copy when only accelerations are wanted).
-__global__ void allpairs_drift(nb::BodyBuffers a, nb::BodyBuffers b, int64_t n, double dt) {
+__global__ void allpairs_drift(nb::BodyBuffers a, nb::BodyBuffers b, int64_t n, double dt,
+                               nb::DeviceScalars* __restrict__ s, unsigned long long* mark) {
+    nb::chain_begin();
+    nb::mark_start(mark);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s->cell_terms = 0;
+        s->body_terms = 0;
+        s->stack_hw = 0;
+    }
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double2 p = a.pos[i], v = a.vel[i];
@@ -182,7 +191,9 @@ __global__ void allpairs_drift(nb::BodyBuffers a, nb::BodyBuffers b, int64_t n, 
 // evaluations, no atomics), then the kick.
 __global__ void allpairs_kick(const double2* __restrict__ partial, int chunks, int64_t n,
                               double2* __restrict__ vel, double2* __restrict__ acc_out,
-                              double G_dt, int kick, unsigned long long* __restrict__ body_terms) {
+                              double G_dt, int kick, unsigned long long* __restrict__ body_terms,
+                              unsigned long long* end) {
+    nb::chain_begin();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double2 a = fold_partial(partial, chunks, n, i);
@@ -195,6 +206,7 @@ __global__ void allpairs_kick(const double2* __restrict__ partial, int chunks, i
     }
     if (threadIdx.x == 0)
         atomicAdd(body_terms, (unsigned long long)min((int64_t)blockDim.x, n - i) * (n - 1));
+    nb::mark_end(end);
 }
 
 // Two targets per thread share each source's load; below this many targets
@@ -216,15 +228,13 @@ inline int source_chunks(int64_t k, int64_t n, int sm_count) {
 
 template <bool kCpuLaw>
 void launch_partial(const double2* pos, const double* mass, int64_t n, const int64_t* targets,
-                    int64_t k, int chunks, double eps2, double2* partial, cudaStream_t st) {
+                    int64_t k, int chunks, double eps2, double2* partial, cudaStream_t st,
+                    bool chained) {
     const dim3 grid((unsigned)target_blocks(k), (unsigned)chunks);
     const int64_t chunk = (n + chunks - 1) / chunks;
-    if (k >= kTwoPerThread)
-        allpairs_partial<kCpuLaw, 2><<<grid, kThreads, 0, st>>>(pos, mass, n, targets, k, chunk, eps2,
-                                                               partial);
-    else
-        allpairs_partial<kCpuLaw, 1><<<grid, kThreads, 0, st>>>(pos, mass, n, targets, k, chunk, eps2,
-                                                               partial);
+    nb::chain_launch(st, chained,
+                     k >= kTwoPerThread ? allpairs_partial<kCpuLaw, 2> : allpairs_partial<kCpuLaw, 1>,
+                     grid, kThreads, 0, pos, mass, n, targets, k, chunk, eps2, partial);
 }
 
 }  // namespace
@@ -236,17 +246,17 @@ void nb::launch_allpairs_step(nb_ctx* c, const BodyBuffers& a, const BodyBuffers
     const unsigned blocks = (unsigned)((c->n + kThreads - 1) / kThreads);
     const int chunks = allpairs_chunks(c->n, c->sm_count);
     c->launches += 3;
-    allpairs_drift<<<blocks, kThreads, 0, c->stream>>>(a, b, c->n, integrate ? c->p.timestep : 0.0);
+    chain_launch(c->stream, false, allpairs_drift, blocks, kThreads, 0, a, b, c->n,
+                 integrate ? c->p.timestep : 0.0, c->scal, mark_of(c, 7));
     if (c->p.flags & NB_FLAG_CPU_LAW)
         launch_partial<true>(b.pos, b.mass, c->n, nullptr, c->n, chunks, c->p.epsilon_squared,
-                             c->ap_partial, c->stream);
+                             c->ap_partial, c->stream, true);
     else
         launch_partial<false>(b.pos, b.mass, c->n, nullptr, c->n, chunks, c->p.epsilon_squared,
-                              c->ap_partial, c->stream);
-    allpairs_kick<<<blocks, kThreads, 0, c->stream>>>(c->ap_partial, chunks, c->n, b.vel,
-                                                       store_acc ? c->acc : nullptr,
-                                                       c->p.G * c->p.timestep, integrate ? 1 : 0,
-                                                       &c->scal->body_terms);
+                              c->ap_partial, c->stream, true);
+    chain_launch(c->stream, true, allpairs_kick, blocks, kThreads, 0, c->ap_partial, chunks, c->n,
+                 b.vel, store_acc ? c->acc : nullptr, c->p.G * c->p.timestep, integrate ? 1 : 0,
+                 &c->scal->body_terms, mark_of(c, kPhases));
 }
 
 extern "C" int nb_allpairs_accelerations(int32_t device, uint64_t n, const double* mass,
@@ -282,7 +292,7 @@ extern "C" int nb_allpairs_accelerations(int32_t device, uint64_t n, const doubl
         cudaMemcpyAsync(dmass, mass, n * sizeof(double), cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(dtgt, targets, k * sizeof(int64_t), cudaMemcpyHostToDevice, st);
         launch_partial<false>(dpos, dmass, (int64_t)n, dtgt, (int64_t)k, chunks, epsilon_squared,
-                              chunks > 1 ? dpart : dacc, st);
+                              chunks > 1 ? dpart : dacc, st, false);
         if (chunks > 1)
             allpairs_fold<<<(unsigned)((k + kThreads - 1) / kThreads), kThreads, 0, st>>>(
                 dpart, chunks, (int64_t)k, dacc);

@@ -430,7 +430,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __restrict__ acc_out,
             float2* __restrict__ acc32, int n, Tree t, DeviceScalars* __restrict__ s, Batch bt,
             float eps2, float theta2, int leaf_size, double G_dt, double dt, int kick,
-            float band2) {
+            float band2, unsigned long long* mark, unsigned long long* end) {
+    chain_begin();
+    mark_start(mark);
     __shared__ WarpLists lists[kWarpsPerBlock];
     const int lane = threadIdx.x & 31;
     WarpLists& L = lists[threadIdx.x >> 5];
@@ -496,11 +498,13 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
     if (lane == 0) {
         atomicAdd(&s->cell_terms, cells_total);
         atomicAdd(&s->body_terms, pairs_total);
+        if (end) atomicMax(end, global_ns());
     }
 }
 
 template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft>
-void launch_split_soft(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc, float eps2) {
+void launch_split_soft(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc, bool chained,
+                       float eps2) {
     int& grid = c->split_blocks[(kQuad ? 1 : 0) + (kLearned ? 2 : 0) + (kBPL == 1 ? 4 : 0) +
                                 (kBPL == 4 ? 16 : 0) +
                                 (kZeroSoft ? 8 : 0)];
@@ -515,21 +519,23 @@ void launch_split_soft(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_ac
     }
     const float theta2 = (float)(c->p.theta * c->p.theta);
     const int leaf = c->p.leaf_size > 0 ? c->p.leaf_size : kDefaultLeaf;
-    force_split<kQuad, kBPL, kLearned, kZeroSoft><<<grid, 32 * kWarpsPerBlock, 0, c->stream>>>(
-        b.pos, b.vel, store_acc ? c->acc : nullptr, c->acc32, (int)c->n, c->tree, c->scal, c->batch,
-        eps2, theta2, leaf, c->p.G * c->p.timestep, c->p.timestep, kick ? 1 : 0,
-        band_theta(c) * band_theta(c));
+    chain_launch(c->stream, chained, force_split<kQuad, kBPL, kLearned, kZeroSoft>, grid,
+                 32 * kWarpsPerBlock, 0, b.pos, b.vel, store_acc ? c->acc : nullptr, c->acc32,
+                 (int)c->n, c->tree, c->scal, c->batch, eps2, theta2, leaf, c->p.G * c->p.timestep,
+                 c->p.timestep, kick ? 1 : 0, band_theta(c) * band_theta(c), mark_of(c, 7),
+                 kLearned ? nullptr : mark_of(c, kPhases));
 }
 
 // eps2 = 0 takes the variant whose terms skip coincident FP32 points
 template <bool kQuad, int kBPL, bool kLearned>
-void launch_split_kernel(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc) {
+void launch_split_kernel(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc,
+                         bool chained) {
     // eps2 below the smallest normal float is treated like eps2 = 0
     const float eps2 = (float)c->p.epsilon_squared;
     if (eps2 >= FLT_MIN)
-        launch_split_soft<kQuad, kBPL, kLearned, false>(c, b, kick, store_acc, eps2);
+        launch_split_soft<kQuad, kBPL, kLearned, false>(c, b, kick, store_acc, chained, eps2);
     else
-        launch_split_soft<kQuad, kBPL, kLearned, true>(c, b, kick, store_acc, eps2);
+        launch_split_soft<kQuad, kBPL, kLearned, true>(c, b, kick, store_acc, chained, eps2);
 }
 
 }  // namespace
@@ -540,23 +546,22 @@ int split_group_size(const nb_ctx* c) {
     return 32 * (c->bpl == 1 ? 1 : c->bpl == 4 ? 4 : kBodiesPerLane);
 }
 
-void launch_force_split(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc) {
+void launch_force_split(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc, bool chained) {
     c->launches += 1;
-    cudaMemsetAsync(&c->scal->group_ticket, 0, sizeof(unsigned), c->stream);
     if (c->p.flags & NB_FLAG_LEARNED) {  // the correction kernel assumes groups of 64
         if (c->p.flags & NB_FLAG_QUADRUPOLE)  // the network corrects the quadrupole walk
-            launch_split_kernel<true, kBodiesPerLane, true>(c, b, kick, store_acc);
+            launch_split_kernel<true, kBodiesPerLane, true>(c, b, kick, store_acc, chained);
         else
-            launch_split_kernel<false, kBodiesPerLane, true>(c, b, kick, store_acc);
+            launch_split_kernel<false, kBodiesPerLane, true>(c, b, kick, store_acc, chained);
     }
     else if (c->p.flags & NB_FLAG_QUADRUPOLE)
-        c->bpl == 1   ? launch_split_kernel<true, 1, false>(c, b, kick, store_acc)
-        : c->bpl == 4 ? launch_split_kernel<true, 4, false>(c, b, kick, store_acc)
-                      : launch_split_kernel<true, kBodiesPerLane, false>(c, b, kick, store_acc);
+        c->bpl == 1   ? launch_split_kernel<true, 1, false>(c, b, kick, store_acc, chained)
+        : c->bpl == 4 ? launch_split_kernel<true, 4, false>(c, b, kick, store_acc, chained)
+                      : launch_split_kernel<true, kBodiesPerLane, false>(c, b, kick, store_acc, chained);
     else
-        c->bpl == 1   ? launch_split_kernel<false, 1, false>(c, b, kick, store_acc)
-        : c->bpl == 4 ? launch_split_kernel<false, 4, false>(c, b, kick, store_acc)
-                      : launch_split_kernel<false, kBodiesPerLane, false>(c, b, kick, store_acc);
+        c->bpl == 1   ? launch_split_kernel<false, 1, false>(c, b, kick, store_acc, chained)
+        : c->bpl == 4 ? launch_split_kernel<false, 4, false>(c, b, kick, store_acc, chained)
+                      : launch_split_kernel<false, kBodiesPerLane, false>(c, b, kick, store_acc, chained);
 }
 
 }  // namespace nb

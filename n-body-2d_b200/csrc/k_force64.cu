@@ -94,7 +94,10 @@ template <int kG, bool kTerms>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 7)
 force_fp64(const double2* __restrict__ pos, const double* __restrict__ mass, double2* __restrict__ vel,
            double2* __restrict__ acc_out, int n, Tree t, DeviceScalars* __restrict__ s, double eps2,
-           double theta_sq, double G_dt, int kick, uint2* __restrict__ terms_out) {
+           double theta_sq, double G_dt, int kick, uint2* __restrict__ terms_out,
+           unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     static_assert(kG >= 1 && kG <= 32 && (kG & (kG - 1)) == 0, "a power of two of bodies per warp");
     constexpr int kSlots = 32 / kG;
     // At kG = 32 more than half of a group's entries act on some 9 bodies each:
@@ -451,23 +454,27 @@ force_fp64(const double2* __restrict__ pos, const double* __restrict__ mass, dou
 template <int kG, bool kTerms>
 void launch_walk64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc) {
     const int64_t groups = (c->n + kG - 1) / kG;
-    force_fp64<kG, kTerms><<<(unsigned)((groups + kWarpsPerBlock - 1) / kWarpsPerBlock),
-                             kWarpsPerBlock * 32, 0, c->stream>>>(
-        b.pos, b.mass, b.vel, store_acc ? c->acc : nullptr, (int)c->n, c->tree, c->scal,
-        c->p.epsilon_squared, c->p.theta * c->p.theta, c->p.G * c->p.timestep, kick ? 1 : 0,
-        kTerms ? c->dbg_terms : nullptr);
+    chain_launch(c->stream, true, force_fp64<kG, kTerms>,
+                 (unsigned)((groups + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0,
+                 b.pos, b.mass, b.vel, store_acc ? c->acc : nullptr, (int)c->n, c->tree, c->scal,
+                 c->p.epsilon_squared, c->p.theta * c->p.theta, c->p.G * c->p.timestep, kick ? 1 : 0,
+                 kTerms ? c->dbg_terms : nullptr, mark_of(c, 7));
 }
 
 // Drift, CU:489-495.
 __global__ void drift_kernel(double2* __restrict__ pos, const double2* __restrict__ vel, int64_t n,
-                             double dt) {
+                             double dt, unsigned long long* mark, unsigned long long* end) {
+    chain_begin();
+    mark_start(mark);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double2 p = pos[i];
-    const double2 v = vel[i];
-    p.x += v.x * dt;
-    p.y += v.y * dt;
-    pos[i] = p;
+    if (i < n) {
+        double2 p = pos[i];
+        const double2 v = vel[i];
+        p.x += v.x * dt;
+        p.y += v.y * dt;
+        pos[i] = p;
+    }
+    mark_end(end);
 }
 
 // CU:498-506, plus the optional accelerations.
@@ -556,7 +563,8 @@ void launch_force_fp64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_ac
 
 void launch_drift(nb_ctx* c, const BodyBuffers& b) {
     c->launches += 1;
-    drift_kernel<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(b.pos, b.vel, c->n, c->p.timestep);
+    chain_launch(c->stream, true, drift_kernel, blocks_for(c->n, 256), 256, 0, b.pos, b.vel, c->n,
+                 c->p.timestep, mark_of(c, 8), mark_of(c, kPhases));
 }
 
 void launch_scatter(nb_ctx* c, const BodyBuffers& b, double2* out_pos, double2* out_vel,

@@ -426,7 +426,9 @@ __global__ void __launch_bounds__(kCorrWarps * 32, 5)
 mlp_correct_kick(const InferW* __restrict__ Wg, Tree t, const DeviceScalars* __restrict__ s,
                  double2* __restrict__ pos, double2* __restrict__ vel,
                  const float2* __restrict__ acc32, double2* __restrict__ acc_out, int n,
-                 float eps2, double G_dt, double dt, int kick) {
+                 float eps2, double G_dt, double dt, int kick, unsigned long long* mark,
+                 unsigned long long* end) {
+    mark_start(mark);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CorrSmem& S = *reinterpret_cast<CorrSmem*>(smem_raw);
     {
@@ -537,6 +539,7 @@ mlp_correct_kick(const InferW* __restrict__ Wg, Tree t, const DeviceScalars* __r
             }
         }
     }
+    mark_end(end);
 }
 
 // ---- the network on the 5th-generation tensor cores (tcgen05) --------------
@@ -1225,7 +1228,8 @@ void launch_mlp_correct(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_a
     mlp_correct_kick<<<c->sm_count * c->corr_blocks_per_sm, kCorrWarps * 32, smem, c->stream>>>(
         static_cast<const InferW*>(c->mlp_infer), c->tree, c->scal, b.pos, b.vel, c->acc32,
         store_acc ? c->acc : nullptr, (int)c->n, (float)c->p.epsilon_squared,
-        c->p.G * c->p.timestep, c->p.timestep, kick ? 1 : 0);
+        c->p.G * c->p.timestep, c->p.timestep, kick ? 1 : 0,
+        mark_of(c, 8), mark_of(c, kPhases));
 }
 
 void launch_mlp_samples(nb_ctx* c, const BodyBuffers& b, const int* pick, int npick, float* X,

@@ -30,13 +30,23 @@ __device__ __forceinline__ double warp_max(double v) {
 // by) and resets the counters of the tie pass; the histogram of the last tree
 // is consumed.  Without `adaptive` (or with a forced count) no histogram is
 // used.
-__device__ __forceinline__ void start_sort(DeviceScalars* s, int64_t n, int adaptive) {
+// Also resets what the later kernels of a step count in, and in a new step the
+// interaction counters.
+__device__ __forceinline__ void start_sort(DeviceScalars* s, int64_t n, int adaptive,
+                                           int new_step) {
     int passes = adaptive ? choose_sort_passes(s->lcp_hist, n) : 8;
     if (s->sort_passes_forced > 0) passes = min(s->sort_passes_forced, 8);
     s->sort_passes = passes;
     for (int d = 0; d <= 32; ++d) s->lcp_hist[d] = 0;
     s->tie_count[0] = 0;
     s->tie_count[1] = 0;
+    s->nstart = 0;
+    s->group_ticket = 0;
+    if (new_step) {
+        s->cell_terms = 0;
+        s->body_terms = 0;
+        s->stack_hw = 0;
+    }
 }
 
 // Exact FP64 min/max of all positions, reduced per block, then folded and
@@ -71,7 +81,9 @@ __device__ __forceinline__ void box_fold(double& xmin, double& xmax, double& ymi
 
 __global__ void __launch_bounds__(kBoxThreads)
 bbox_kernel(const double2* __restrict__ pos, int64_t n, double* __restrict__ partials,
-            DeviceScalars* __restrict__ s, int adaptive) {
+            DeviceScalars* __restrict__ s, int adaptive, int new_step, unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     double xmin = INFINITY, xmax = -INFINITY, ymin = INFINITY, ymax = -INFINITY;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -150,7 +162,7 @@ bbox_kernel(const double2* __restrict__ pos, int64_t n, double* __restrict__ par
             wsq *= 0.25;
         }
         s->bbox_ticket = 0;
-        start_sort(s, n, adaptive);
+        start_sort(s, n, adaptive, new_step);
     }
 }
 
@@ -164,6 +176,24 @@ __device__ __forceinline__ uint64_t expand_bits_2d(uint32_t v) {
     return x;
 }
 
+// What a sort counts in: the digit histograms, the tile counters and the
+// status words of the passes it will run.
+struct SortState {
+    uint32_t* hist = nullptr;     // nullptr: nothing to reset
+    unsigned* tile_counter = nullptr;
+    uint32_t* status = nullptr;
+    int tiles = 0;
+};
+
+__device__ __forceinline__ void reset_sort(const SortState& z, int passes) {
+    if (!z.hist) return;
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x, per_pass = 256 * (int64_t)z.tiles;
+    for (int64_t k = t0; k < 8 * 256; k += step) z.hist[k] = 0;
+    if (t0 < 8) z.tile_counter[t0] = 0;
+    for (int64_t k = (8 - passes) * per_pass + t0; k < 8 * per_pass; k += step) z.status[k] = 0;
+}
+
 // CU:117-132: code from (p - min) * (1 / width), quantised to 32 bits per axis
 // with round-down; x bits land on odd positions.  val = current slot.  The
 // codes go to the buffer the first radix pass reads: pass k reads buffer
@@ -172,7 +202,9 @@ __device__ __forceinline__ uint64_t expand_bits_2d(uint32_t v) {
 __global__ void morton_kernel(const double2* __restrict__ pos, int64_t n,
                               const DeviceScalars* __restrict__ s, uint64_t* __restrict__ key0,
                               uint64_t* __restrict__ key1, uint32_t* __restrict__ val0,
-                              uint32_t* __restrict__ val1) {
+                              uint32_t* __restrict__ val1, SortState z) {
+    chain_begin();
+    reset_sort(z, s->sort_passes);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bool odd = s->sort_passes & 1;
@@ -204,7 +236,9 @@ __device__ __forceinline__ double from_ordered(unsigned long long o) {
 }
 
 __global__ void __launch_bounds__(256)
-bbox_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b) {
+bbox_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b, unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     const int lane = threadIdx.x & 31;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i - lane < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -235,9 +269,11 @@ bbox_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b) {
 
 // Squares every universe's box as the single-universe path does, and resets
 // the reduction slots for the next step.
-__global__ void bbox_batch_finish(Batch b, DeviceScalars* __restrict__ s, int64_t n) {
+__global__ void bbox_batch_finish(Batch b, DeviceScalars* __restrict__ s, int64_t n,
+                                  int new_step) {
+    chain_begin();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u == 0) start_sort(s, n, 1);
+    if (u == 0) start_sort(s, n, 1, new_step);
     if (u >= b.nuni) return;
     unsigned long long* e = b.boxbits + 4 * u;
     double x0 = from_ordered(e[0]), x1 = from_ordered(~e[1]);
@@ -265,7 +301,10 @@ __global__ void bbox_batch_finish(Batch b, DeviceScalars* __restrict__ s, int64_
 __global__ void morton_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b,
                                     const DeviceScalars* __restrict__ s,
                                     uint64_t* __restrict__ key0, uint64_t* __restrict__ key1,
-                                    uint32_t* __restrict__ val0, uint32_t* __restrict__ val1) {
+                                    uint32_t* __restrict__ val0, uint32_t* __restrict__ val1,
+                                    SortState z) {
+    chain_begin();
+    reset_sort(z, s->sort_passes);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bool odd = s->sort_passes & 1;
@@ -467,7 +506,10 @@ constexpr int kHistRows = 4;
 
 __global__ void __launch_bounds__(kSortThreads)
 onesweep_histogram(const uint64_t* __restrict__ key0, const uint64_t* __restrict__ key1, int64_t n,
-                   const DeviceScalars* __restrict__ s, uint32_t* __restrict__ hist) {
+                   const DeviceScalars* __restrict__ s, uint32_t* __restrict__ hist,
+                   unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     // the Morton pass wrote the codes where the first radix pass reads them
     const uint64_t* __restrict__ key = (s->sort_passes & 1) ? key1 : key0;
     const int dmin = 8 - s->sort_passes;  // digits below are not sorted by a pass
@@ -529,6 +571,7 @@ __device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid) {
 // Exclusive scan of each digit position's 256 bins (block d = position d).
 __global__ void __launch_bounds__(kSortThreads)
 onesweep_bins(uint32_t* __restrict__ hist) {
+    chain_begin();
     __shared__ uint32_t warp_tot[kWarps];
     uint32_t* row = hist + 256 * blockIdx.x;
     const uint32_t v = row[threadIdx.x];
@@ -601,6 +644,7 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
               const uint32_t* __restrict__ bins, uint32_t* __restrict__ status,
               unsigned* __restrict__ tile_counter, unsigned* __restrict__ err,
               const int32_t* __restrict__ passes) {
+    chain_begin();
     if (passes && shift < 64 - 8 * *passes) return;
     __shared__ uint32_t whist[kWarps][256];
     __shared__ uint32_t tile_start[256];
@@ -737,6 +781,7 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
 __global__ void __launch_bounds__(256)
 tie_mark(const uint64_t* __restrict__ key, int64_t n, DeviceScalars* __restrict__ s,
          uint2* __restrict__ small, uint2* __restrict__ big) {
+    chain_begin();
     const int passes = s->sort_passes;
     if (passes >= 8) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -788,6 +833,7 @@ tie_mark(const uint64_t* __restrict__ key, int64_t n, DeviceScalars* __restrict_
 __global__ void __launch_bounds__(256)
 tie_sort_small(uint64_t* __restrict__ key, uint32_t* __restrict__ val,
                const uint2* __restrict__ small, const DeviceScalars* __restrict__ s) {
+    chain_begin();
     if (s->sort_passes >= 8) return;
     const unsigned count = s->tie_count[0];
     const int lane = threadIdx.x & 31;
@@ -818,6 +864,7 @@ __global__ void __launch_bounds__(128)
 tie_sort_big(uint64_t* __restrict__ key0, uint32_t* __restrict__ val0, uint64_t* __restrict__ key1,
              uint32_t* __restrict__ val1, const uint2* __restrict__ big,
              const DeviceScalars* __restrict__ s) {
+    chain_begin();
     const int passes = s->sort_passes;
     if (passes >= 8) return;
     __shared__ uint32_t off[4][256];
@@ -894,7 +941,10 @@ tie_sort_big(uint64_t* __restrict__ key0, uint32_t* __restrict__ val0, uint64_t*
 // writes the FP32 source record of each body relative to the box centre.
 __global__ void gather_kernel(const uint32_t* __restrict__ order, int64_t n, BodyBuffers src,
                               BodyBuffers dst, float4* __restrict__ body4,
-                              const DeviceScalars* __restrict__ s, Batch bt) {
+                              const DeviceScalars* __restrict__ s, Batch bt,
+                              unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t j = __ldg(order + i);
@@ -917,29 +967,35 @@ inline unsigned blocks_for(int64_t n, int threads) {
 
 }  // namespace
 
-void launch_bbox(nb_ctx* c, const double2* pos) {
+void launch_bbox(nb_ctx* c, const double2* pos, bool new_step) {
     if (c->batch.nuni > 0) {
         c->launches += 2;
-        bbox_batch_kernel<<<2 * c->sm_count * 8, 256, 0, c->stream>>>(pos, c->n, c->batch);
-        bbox_batch_finish<<<blocks_for(c->batch.nuni, 128), 128, 0, c->stream>>>(c->batch, c->scal,
-                                                                                c->n);
+        chain_launch(c->stream, false, bbox_batch_kernel, 2 * c->sm_count * 8, 256, 0, pos, c->n,
+                     c->batch, mark_of(c, 0));
+        chain_launch(c->stream, true, bbox_batch_finish, blocks_for(c->batch.nuni, 128), 128, 0,
+                     c->batch, c->scal, c->n, new_step);
         return;
     }
     c->launches += 1;
-    bbox_kernel<<<c->bbox_blocks, kBoxThreads, 0, c->stream>>>(pos, c->n, c->bbox_partials, c->scal,
-                                                               1);
+    chain_launch(c->stream, false, bbox_kernel, c->bbox_blocks, kBoxThreads, 0, pos, c->n,
+                 c->bbox_partials, c->scal, 1, new_step, mark_of(c, 0));
 }
 
 void launch_morton(nb_ctx* c, const double2* pos) {
     c->launches += 1;
+    SortState z;
+    z.hist = c->sort.hist;
+    z.tile_counter = c->sort.tile_counter;
+    z.status = c->sort.status;
+    z.tiles = c->sort.tiles;
     if (c->batch.nuni > 0) {
-        morton_batch_kernel<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(
-            pos, c->n, c->batch, c->scal, c->sort.key[0], c->sort.key[1], c->sort.val[0],
-            c->sort.val[1]);
+        chain_launch(c->stream, true, morton_batch_kernel, blocks_for(c->n, 256), 256, 0, pos, c->n,
+                     c->batch, c->scal, c->sort.key[0], c->sort.key[1], c->sort.val[0],
+                     c->sort.val[1], z);
         return;
     }
-    morton_kernel<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(
-        pos, c->n, c->scal, c->sort.key[0], c->sort.key[1], c->sort.val[0], c->sort.val[1]);
+    chain_launch(c->stream, true, morton_kernel, blocks_for(c->n, 256), 256, 0, pos, c->n, c->scal,
+                 c->sort.key[0], c->sort.key[1], c->sort.val[0], c->sort.val[1], z);
 }
 
 // One radix pass over two tiles of keys in which only the second tile runs:
@@ -983,31 +1039,27 @@ unsigned sort_timeout_probe(cudaStream_t st) {
     return flags;
 }
 
+// The Morton pass has reset the histograms, tile counters and status words.
 void launch_sort(nb_ctx* c) {
     const int tiles = c->sort.tiles;
     c->launches += 2 + 8 + 3;
-    // histograms, per-pass status words and tile counters start at zero
-    cudaMemsetAsync(c->sort.hist, 0, sizeof(uint32_t) * 8 * 256, c->stream);
-    cudaMemsetAsync(c->sort.status, 0, sizeof(uint32_t) * 8 * 256 * (size_t)tiles, c->stream);
-    cudaMemsetAsync(c->sort.tile_counter, 0, sizeof(unsigned) * 8, c->stream);
-    onesweep_histogram<<<4 * c->sm_count, kSortThreads, 0, c->stream>>>(
-        c->sort.key[0], c->sort.key[1], c->n, c->scal, c->sort.hist);
-    onesweep_bins<<<8, kSortThreads, 0, c->stream>>>(c->sort.hist);
+    chain_launch(c->stream, true, onesweep_histogram, 4 * c->sm_count, kSortThreads, 0,
+                 c->sort.key[0], c->sort.key[1], c->n, c->scal, c->sort.hist, mark_of(c, 1));
+    chain_launch(c->stream, true, onesweep_bins, 8, kSortThreads, 0, c->sort.hist);
     for (int pass = 0; pass < 8; ++pass) {
         const int src = pass & 1, dst = src ^ 1;
-        onesweep_pass<<<tiles, kSortThreads, 0, c->stream>>>(
-            c->sort.key[src], c->sort.val[src], c->sort.key[dst], c->sort.val[dst], c->n, 8 * pass,
-            c->sort.hist + 256 * pass, c->sort.status + (size_t)pass * 256 * tiles,
-            c->sort.tile_counter + pass, &c->scal->error, &c->scal->sort_passes);
+        chain_launch(c->stream, true, onesweep_pass, tiles, kSortThreads, 0, c->sort.key[src],
+                     c->sort.val[src], c->sort.key[dst], c->sort.val[dst], c->n, 8 * pass,
+                     c->sort.hist + 256 * pass, c->sort.status + (size_t)pass * 256 * tiles,
+                     c->sort.tile_counter + pass, &c->scal->error, &c->scal->sort_passes);
     }
     // keys tied in the sorted top bytes, in order of their low bytes
-    tie_mark<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->sort.key[0], c->n, c->scal,
-                                                           c->sort.ties_small, c->sort.ties_big);
-    tie_sort_small<<<c->sm_count * 8, 256, 0, c->stream>>>(c->sort.key[0], c->sort.val[0],
-                                                          c->sort.ties_small, c->scal);
-    tie_sort_big<<<c->sm_count, 128, 0, c->stream>>>(c->sort.key[0], c->sort.val[0],
-                                                     c->sort.key[1], c->sort.val[1],
-                                                     c->sort.ties_big, c->scal);
+    chain_launch(c->stream, true, tie_mark, blocks_for(c->n, 256), 256, 0, c->sort.key[0], c->n,
+                 c->scal, c->sort.ties_small, c->sort.ties_big);
+    chain_launch(c->stream, true, tie_sort_small, c->sm_count * 8, 256, 0, c->sort.key[0],
+                 c->sort.val[0], c->sort.ties_small, c->scal);
+    chain_launch(c->stream, true, tie_sort_big, c->sm_count, 128, 0, c->sort.key[0], c->sort.val[0],
+                 c->sort.key[1], c->sort.val[1], c->sort.ties_big, c->scal);
 }
 
 void launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* const key[2],
@@ -1015,8 +1067,10 @@ void launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* const key[2
                             uint32_t* counts, uint32_t* totals, double* partials, int bbox_blocks,
                             DeviceScalars* scal, cudaStream_t st) {
     const int tiles = (int)((n + kSortTile - 1) / kSortTile);
-    bbox_kernel<<<bbox_blocks, kBoxThreads, 0, st>>>(pos, n, partials, scal, 0);  // all 8 passes
-    morton_kernel<<<blocks_for(n, 256), 256, 0, st>>>(pos, n, scal, key[0], key[1], val[0], val[1]);
+    bbox_kernel<<<bbox_blocks, kBoxThreads, 0, st>>>(pos, n, partials, scal, 0, 0,
+                                                      nullptr);  // all 8 passes
+    morton_kernel<<<blocks_for(n, 256), 256, 0, st>>>(pos, n, scal, key[0], key[1], val[0], val[1],
+                                                    SortState());
     for (int pass = 0; pass < 8; ++pass) {
         const int src = pass & 1, dst = src ^ 1;
         const int shift = 8 * pass;
@@ -1031,8 +1085,8 @@ void launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* const key[2
 
 void launch_gather(nb_ctx* c, const BodyBuffers& src, const BodyBuffers& dst, float4* body4) {
     c->launches += 1;
-    gather_kernel<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->sort.val[0], c->n, src, dst,
-                                                                body4, c->scal, c->batch);
+    chain_launch(c->stream, true, gather_kernel, blocks_for(c->n, 256), 256, 0, c->sort.val[0], c->n,
+                 src, dst, body4, c->scal, c->batch, mark_of(c, 2));
 }
 
 }  // namespace nb

@@ -122,7 +122,10 @@ __device__ __forceinline__ unsigned thermometer(int c) {
 __global__ void __launch_bounds__(kThreads)
 tree_lcp(const uint64_t* __restrict__ key, int n, int tiles, uint8_t* __restrict__ lcp8,
          int32_t* __restrict__ tile_first, int32_t* __restrict__ tile_last,
-         unsigned* __restrict__ lcp_hist) {
+         unsigned* __restrict__ lcp_hist,
+         unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     __shared__ unsigned hist[33];
     __shared__ int sfirst[kAnsvLevels], slast[kAnsvLevels];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -179,6 +182,7 @@ tree_lcp(const uint64_t* __restrict__ key, int n, int tiles, uint8_t* __restrict
 constexpr int kTileScanThreads = 1024;
 __global__ void __launch_bounds__(kTileScanThreads)
 tree_ansv_tiles(int tiles, int32_t* __restrict__ tile_first, int32_t* __restrict__ tile_last) {
+    chain_begin();
     __shared__ int wagg[kTileScanThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t* last = tile_last + blockIdx.x * tiles;
@@ -237,6 +241,7 @@ __global__ void __launch_bounds__(kThreads)
 tree_ansv(const uint8_t* __restrict__ lcp8, int n, int tiles,
           const int32_t* __restrict__ tile_first, const int32_t* __restrict__ tile_last,
           int32_t* __restrict__ flag, int4* __restrict__ bnd) {
+    chain_begin();
     // masks[r][v]: row r's ballot of "level < v" (v = 1..30; 0 elsewhere).
     // rlast[r][v]: after the scan, the last boundary with a level below v in
     // rows 8p..r of r's part p (-1 if none), rfirst[r][v] the first in rows
@@ -357,7 +362,10 @@ __device__ int block_exclusive(int v, int* wsum, int* total) {
 // kScanItems items [w 32 kScanItems, (w + 1) 32 kScanItems) of the tile,
 // lane l the items 32 k + l of them.
 __global__ void __launch_bounds__(kThreads)
-scan_reduce(const int32_t* __restrict__ in, int n, int32_t* __restrict__ block_sums) {
+scan_reduce(const int32_t* __restrict__ in, int n, int32_t* __restrict__ block_sums,
+         unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     __shared__ int wsum[kThreads / 32];
     __shared__ int total;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -377,6 +385,7 @@ scan_reduce(const int32_t* __restrict__ in, int n, int32_t* __restrict__ block_s
 constexpr int kSumsThreads = 1024;
 __global__ void __launch_bounds__(kSumsThreads)
 scan_block_sums(int32_t* __restrict__ block_sums, int blocks, int32_t* __restrict__ total_out) {
+    chain_begin();
     __shared__ int wsum[kSumsThreads / 32];
     __shared__ int total;
     int carry = 0;
@@ -396,6 +405,7 @@ scan_block_sums(int32_t* __restrict__ block_sums, int blocks, int32_t* __restric
 __global__ void __launch_bounds__(kThreads)
 scan_apply(const int32_t* __restrict__ in, int n, const int32_t* __restrict__ block_sums,
            int32_t* __restrict__ out, int32_t* __restrict__ index_of) {
+    chain_begin();
     __shared__ int wsum[kThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int base = blockIdx.x * kScanTile + warp * 32 * kScanItems + lane;
@@ -488,6 +498,7 @@ tree_link(const uint64_t* __restrict__ key, const uint8_t* __restrict__ lcp8, in
           const double2* __restrict__ pos, const double* __restrict__ mass, Tree t,
           DeviceScalars* __restrict__ s, const double4* __restrict__ prefix, Batch bt,
           float accept_scale, int gsize, int fill) {
+    chain_begin();
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     const int cells = s->cells;
     if (id >= cells) {
@@ -581,6 +592,7 @@ tree_link(const uint64_t* __restrict__ key, const uint8_t* __restrict__ lcp8, in
 // A tree without internal cells: one body, or all bodies in one level-30 leaf.
 __global__ void tree_trivial_root(const double2* __restrict__ pos, const double* __restrict__ mass,
                                   int n, Tree t, DeviceScalars* __restrict__ s, int gsize) {
+    chain_begin();
     if (s->cells != 0) return;
     if (gsize > 0) t.gcount[0] = (n + gsize - 1) / gsize;  // groups of the root leaf
     s->root = ~0;
@@ -746,7 +758,10 @@ __device__ __forceinline__ int arrive_acq_rel(int* counter) {
 template <bool kSplit, bool kSecond>
 __global__ void tree_moments(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
                              const double* __restrict__ mass, Tree t, Batch bt,
-                             float accept_scale) {
+                             float accept_scale,
+         unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int cells = s->cells;
     if (k >= s->nstart) return;
@@ -816,7 +831,10 @@ constexpr int kWarpItems = 32 * kScanItems;
 // Phase 1: per tile of kScanTile bodies, the total.
 __global__ void __launch_bounds__(kThreads)
 prefix_reduce(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
-              const DeviceScalars* __restrict__ s, Batch bt, double4* __restrict__ tiles) {
+              const DeviceScalars* __restrict__ s, Batch bt, double4* __restrict__ tiles,
+         unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
     __shared__ double4 red[kThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int base = blockIdx.x * kScanTile + warp * kWarpItems + lane;
@@ -864,6 +882,7 @@ __device__ double4 block_exclusive_d4(double4 v, double4* part, double4& total) 
 // Phase 2: exclusive scan of the tile totals (one block, chunks of
 // kThreads * kScanItems tiles in order); tiles[ntiles] = the grand total.
 __global__ void __launch_bounds__(kThreads) prefix_tiles_scan(double4* __restrict__ tiles, int ntiles) {
+    chain_begin();
     __shared__ double4 part[kThreads];
     double4 carry = make_double4(0.0, 0.0, 0.0, 0.0);
     for (int c0 = 0; c0 < ntiles; c0 += kScanTile) {
@@ -892,6 +911,7 @@ __global__ void __launch_bounds__(kThreads)
 prefix_apply(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
              const DeviceScalars* __restrict__ s, Batch bt, const double4* __restrict__ tiles,
              int ntiles, double4* __restrict__ prefix) {
+    chain_begin();
     __shared__ double4 wtot[kThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int base = blockIdx.x * kScanTile + warp * kWarpItems + lane;
@@ -1008,6 +1028,7 @@ __device__ __forceinline__ void add_shifted(float m, float dx, float dy, const f
 __global__ void __launch_bounds__(kThreads)
 learned_features(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
                  const double* __restrict__ mass, Tree t, Batch bt) {
+    chain_begin();
     int id = blockIdx.x * blockDim.x + threadIdx.x;
     const int cells = s->cells;
     if (id >= cells || !direct_cell(t, id)) return;
@@ -1146,6 +1167,7 @@ __device__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const i
 __global__ void tree_groups_write(int n, int gsize, int fill, Tree t,
                                   const DeviceScalars* __restrict__ s, Batch bt,
                                   const uint64_t* __restrict__ key) {
+    chain_begin();
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     const int cells = s->cells;
     if (id >= n) return;
@@ -1184,6 +1206,7 @@ __global__ void tree_groups_write(int n, int gsize, int fill, Tree t,
 // Root reference of each universe: the cell whose body range is exactly the
 // universe's (found like a child cell in tree_link), or its single leaf.
 __global__ void batch_roots(const uint64_t* __restrict__ key, Tree t, Batch bt) {
+    chain_begin();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= bt.nuni) return;
     const int a = bt.off[u], b = bt.off[u + 1] - 1;
@@ -1208,11 +1231,12 @@ inline unsigned blocks_for(int64_t n, int threads) {
 void launch_batch_roots(nb_ctx* c) {
     if (c->batch.nuni == 0) return;
     c->launches += 1;
-    batch_roots<<<blocks_for(c->batch.nuni, 128), 128, 0, c->stream>>>(c->sort.key[0], c->tree,
-                                                                      c->batch);
+    chain_launch(c->stream, true, batch_roots, blocks_for(c->batch.nuni, 128), 128, 0,
+                 c->sort.key[0], c->tree, c->batch);
 }
 
-void launch_groups(nb_ctx* c) {
+// chained: the kernel before is the linking pass, on the same stream
+void launch_groups(nb_ctx* c, bool chained) {
     const int n = (int)c->n;
     const int sblocks = (int)blocks_for(n, kScanTile);
     c->launches += 4;
@@ -1222,12 +1246,14 @@ void launch_groups(nb_ctx* c) {
     // learned correction keeps groups of whole cells, whose residuals it fits.
     // The linking pass counted every cell's groups; scan, then write them.
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
-    scan_reduce<<<sblocks, kThreads, 0, c->stream>>>(c->tree.gcount, n, c->scan.block_sums);
-    scan_block_sums<<<1, kSumsThreads, 0, c->stream>>>(c->scan.block_sums, sblocks, &c->scal->groups);
-    scan_apply<<<sblocks, kThreads, 0, c->stream>>>(c->tree.gcount, n, c->scan.block_sums,
-                                                     c->tree.gbase, nullptr);
-    tree_groups_write<<<blocks_for(n, kThreads), kThreads, 0, c->stream>>>(
-        n, gsize, fill, c->tree, c->scal, c->batch, c->sort.key[0]);
+    chain_launch(c->stream, chained, scan_reduce, sblocks, kThreads, 0, c->tree.gcount, n,
+                 c->scan.block_sums, mark_of(c, 6));
+    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, c->scan.block_sums, sblocks,
+                 &c->scal->groups);
+    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, c->tree.gcount, n,
+                 c->scan.block_sums, c->tree.gbase, nullptr);
+    chain_launch(c->stream, true, tree_groups_write, blocks_for(n, kThreads), kThreads, 0, n, gsize,
+                 fill, c->tree, c->scal, c->batch, c->sort.key[0]);
 }
 
 // SPLIT without quadrupoles takes its monopoles from prefix sums over the
@@ -1250,12 +1276,12 @@ void launch_prefix_sums(nb_ctx* c, const BodyBuffers& b) {
     {  // the prefix sums need only the sorted bodies
         const int ptiles = (int)blocks_for(n, kScanTile);
         c->launches += 3;
-        prefix_reduce<<<ptiles, kThreads, 0, c->stream>>>(b.pos, b.mass, n, c->scal, c->batch,
-                                                          c->tree.prefix_tiles);
-        prefix_tiles_scan<<<1, kThreads, 0, c->stream>>>(c->tree.prefix_tiles, ptiles);
-        prefix_apply<<<ptiles, kThreads, 0, c->stream>>>(b.pos, b.mass, n, c->scal, c->batch,
-                                                         c->tree.prefix_tiles, ptiles,
-                                                         c->tree.prefix);
+        chain_launch(c->stream, true, prefix_reduce, ptiles, kThreads, 0, b.pos, b.mass, n, c->scal,
+                     c->batch, c->tree.prefix_tiles, mark_of(c, 3));
+        chain_launch(c->stream, true, prefix_tiles_scan, 1, kThreads, 0, c->tree.prefix_tiles,
+                     ptiles);
+        chain_launch(c->stream, true, prefix_apply, ptiles, kThreads, 0, b.pos, b.mass, n, c->scal,
+                     c->batch, c->tree.prefix_tiles, ptiles, c->tree.prefix);
     }
 }
 
@@ -1267,36 +1293,33 @@ void launch_tree(nb_ctx* c, const BodyBuffers& b, bool prefix_done) {
     Tree& t = c->tree;
     const int tiles = (int)blocks_for(n, kAnsvTile);
     c->launches += 8;
-    tree_lcp<<<tiles, kThreads, 0, c->stream>>>(key, n, tiles, t.lcp8, t.ansv_first, t.ansv_last,
-                                                c->scal->lcp_hist);
-    tree_ansv_tiles<<<kAnsvLevels, kTileScanThreads, 0, c->stream>>>(tiles, t.ansv_first,
-                                                                     t.ansv_last);
-    tree_ansv<<<tiles, kThreads, 0, c->stream>>>(t.lcp8, n, tiles, t.ansv_first, t.ansv_last,
-                                                 t.flag, t.bnd);
+    chain_launch(c->stream, true, tree_lcp, tiles, kThreads, 0, key, n, tiles, t.lcp8, t.ansv_first,
+                 t.ansv_last, c->scal->lcp_hist, mark_of(c, 4));
+    chain_launch(c->stream, true, tree_ansv_tiles, kAnsvLevels, kTileScanThreads, 0, tiles,
+                 t.ansv_first, t.ansv_last);
+    chain_launch(c->stream, true, tree_ansv, tiles, kThreads, 0, t.lcp8, n, tiles, t.ansv_first,
+                 t.ansv_last, t.flag, t.bnd);
     const int sblocks = (int)blocks_for(n, kScanTile);
-    scan_reduce<<<sblocks, kThreads, 0, c->stream>>>(t.flag, n, c->scan.block_sums);
-    scan_block_sums<<<1, kSumsThreads, 0, c->stream>>>(c->scan.block_sums, sblocks, &c->scal->cells);
-    scan_apply<<<sblocks, kThreads, 0, c->stream>>>(t.flag, n, c->scan.block_sums, t.cell_of,
-                                                     t.rep_of);
-    cudaMemsetAsync(&c->scal->nstart, 0, sizeof(int32_t), c->stream);
+    chain_launch(c->stream, true, scan_reduce, sblocks, kThreads, 0, t.flag, n, c->scan.block_sums,
+                 nullptr);
+    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, c->scan.block_sums, sblocks,
+                 &c->scal->cells);
+    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, t.flag, n, c->scan.block_sums,
+                 t.cell_of, t.rep_of);
     // SPLIT: the cells count their target groups as they link
     const int gsize = c->p.mode == NB_MODE_SPLIT ? split_group_size(c) : 0;
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
-    if (mono)
-        tree_link<true><<<blocks_for(n, kThreads), kThreads, 0, c->stream>>>(
-            key, t.lcp8, n, b.pos, b.mass, t, c->scal, t.prefix, c->batch, split_accept_scale(c),
-            gsize, fill);
-    else
-        tree_link<false><<<blocks_for(n, kThreads), kThreads, 0, c->stream>>>(
-            key, t.lcp8, n, b.pos, b.mass, t, c->scal, nullptr, c->batch, 0.f, gsize, fill);
-    tree_trivial_root<<<1, 1, 0, c->stream>>>(b.pos, b.mass, n, t, c->scal, gsize);
+    chain_launch(c->stream, true, mono ? tree_link<true> : tree_link<false>, blocks_for(n, kThreads),
+                 kThreads, 0, key, t.lcp8, n, b.pos, b.mass, t, c->scal, mono ? t.prefix : nullptr,
+                 c->batch, mono ? split_accept_scale(c) : 0.f, gsize, fill);
+    chain_launch(c->stream, true, tree_trivial_root, 1, 1, 0, b.pos, b.mass, n, t, c->scal, gsize);
 }
 
-void launch_features(nb_ctx* c, const BodyBuffers& b) {
+void launch_features(nb_ctx* c, const BodyBuffers& b, bool chained) {
     const int cap = (int)(c->n > 1 ? c->n - 1 : 1);
     c->launches += 1;
-    learned_features<<<blocks_for(cap, kThreads), kThreads, 0, c->stream>>>(c->scal, b.pos, b.mass,
-                                                                           c->tree, c->batch);
+    chain_launch(c->stream, chained, learned_features, blocks_for(cap, kThreads), kThreads, 0, c->scal,
+                 b.pos, b.mass, c->tree, c->batch);
 }
 
 void launch_moments(nb_ctx* c, const BodyBuffers& b, bool split) {
@@ -1309,15 +1332,15 @@ void launch_moments(nb_ctx* c, const BodyBuffers& b, bool split) {
     const unsigned blocks = blocks_for(cap, kThreads);
     if (second) {
         c->launches += 1;
-        tree_moments<true, true><<<blocks, kThreads, 0, c->stream>>>(c->scal, b.pos, b.mass, c->tree,
-                                                                     c->batch, accept_scale);
+        chain_launch(c->stream, true, tree_moments<true, true>, blocks, kThreads, 0, c->scal, b.pos,
+                     b.mass, c->tree, c->batch, accept_scale, mark_of(c, 5));
     } else if (split) {
         // monopoles: the prefix sums ran before the tree, and the linking
         // pass wrote every cell's record from them
     } else {
         c->launches += 1;
-        tree_moments<false, false><<<blocks, kThreads, 0, c->stream>>>(c->scal, b.pos, b.mass,
-                                                                       c->tree, c->batch, 0.f);
+        chain_launch(c->stream, true, tree_moments<false, false>, blocks, kThreads, 0, c->scal, b.pos,
+                     b.mass, c->tree, c->batch, 0.f, mark_of(c, 5));
     }
 }
 

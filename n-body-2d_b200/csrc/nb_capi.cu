@@ -237,77 +237,67 @@ const char* const kPhaseNames[nb::kPhases] = {"bbox+morton", "sort", "gather", "
 
 // Enqueues one step reading the state from buf[parity]; leaves it in the
 // other buffer.  integrate=false stops after the force pass (no kick/drift).
-// timed=true records the phase events between stages.
+// timed=true: the kernels write the phases' times (scal->marks).
 void enqueue_step(nb_ctx* c, int parity, bool integrate, bool store_acc, bool timed = false) {
     const nb::BodyBuffers& A = c->buf[parity];
     const nb::BodyBuffers& B = c->buf[parity ^ 1];
-    // External records become event nodes of the captured graph, so the
-    // events carry timestamps from every replay of the step.
-    auto mark = [&](int k) {
-        if (timed) cudaEventRecordWithFlags(c->phase_ev[k], c->stream, cudaEventRecordExternal);
-    };
-    mark(0);
-    // cell_terms, body_terms and stack_hw start every force pass at zero
-    cudaMemsetAsync(&c->scal->cell_terms, 0, 3 * sizeof(unsigned long long), c->stream);
+    c->marks_on = timed;
     if (c->p.mode == NB_MODE_ALLPAIRS) {
         // AllPairsSim: drift into the other buffer, then the all-pairs kick there
-        for (int k = 1; k < 8; ++k) mark(k);
         nb::launch_allpairs_step(c, A, B, integrate, store_acc);
-        mark(8);
-        mark(9);
+        c->marks_on = false;
         return;
     }
-    nb::launch_bbox(c, A.pos);
+    nb::launch_bbox(c, A.pos, true);
     nb::launch_morton(c, A.pos);
-    mark(1);
     nb::launch_sort(c);
-    mark(2);
     const bool split = c->p.mode == NB_MODE_SPLIT;
     nb::launch_gather(c, A, B, split ? c->tree.body4 : nullptr);
-    mark(3);
     nb::launch_prefix_sums(c, B);  // SPLIT monopoles only
-    mark(4);
     nb::launch_tree(c, B, true);
     nb::launch_batch_roots(c);
-    mark(5);
-    // the target groups need only the tree: they are built on the side stream
-    // while the moments run (two branches of the captured graph)
-    if (split) {
-        cudaEventRecord(c->fork_ev, c->stream);
-        cudaStreamWaitEvent(c->side_stream, c->fork_ev, 0);
+    // the target groups need only the tree: with quadrupoles, whose moments
+    // climb the tree, they are built on the side stream meanwhile (two branches
+    // of the captured graph)
+    const bool fork = split && (c->p.flags & NB_FLAG_QUADRUPOLE);
+    auto on_side = [&](cudaEvent_t forked, cudaEvent_t joined, auto&& launch) {
+        cudaEventRecord(forked, c->stream);
+        cudaStreamWaitEvent(c->side_stream, forked, 0);
         cudaStream_t main_stream = c->stream;
         c->stream = c->side_stream;
-        nb::launch_groups(c);
+        launch();
         c->stream = main_stream;
-        cudaEventRecord(c->join_ev, c->side_stream);
-    }
+        cudaEventRecord(joined, c->side_stream);
+    };
+    if (fork) on_side(c->fork_ev, c->join_ev, [&] { nb::launch_groups(c, false); });
+    else if (split) nb::launch_groups(c, true);
     nb::launch_moments(c, B, split);
-    mark(6);
-    if (split) cudaStreamWaitEvent(c->stream, c->join_ev, 0);
-    mark(7);
+    if (fork) cudaStreamWaitEvent(c->stream, c->join_ev, 0);
     if (split && (c->p.flags & NB_FLAG_LEARNED)) {
         // the features need only the monopoles, and only the correction reads
         // them: they are built on the side stream while the walk runs
-        cudaEventRecord(c->feat_fork_ev, c->stream);
-        cudaStreamWaitEvent(c->side_stream, c->feat_fork_ev, 0);
-        cudaStream_t main_stream = c->stream;
-        c->stream = c->side_stream;
-        nb::launch_features(c, B);
-        c->stream = main_stream;
-        cudaEventRecord(c->feat_join_ev, c->side_stream);
-        nb::launch_force_split(c, B, integrate, store_acc);  // FP32 accelerations + band lists
-        mark(8);
+        on_side(c->feat_fork_ev, c->feat_join_ev, [&] { nb::launch_features(c, B, false); });
+        nb::launch_force_split(c, B, integrate, store_acc, false);  // FP32 accelerations + band lists
         cudaStreamWaitEvent(c->stream, c->feat_join_ev, 0);
         nb::launch_mlp_correct(c, B, integrate, store_acc);  // learned term, kick, drift
     } else if (split) {
-        nb::launch_force_split(c, B, integrate, store_acc);  // kick and drift fused
-        mark(8);
+        nb::launch_force_split(c, B, integrate, store_acc, !fork);  // kick and drift fused
     } else {
         nb::launch_force_fp64(c, B, integrate, store_acc);
-        mark(8);
         if (integrate) nb::launch_drift(c, B);
     }
-    mark(9);
+    c->marks_on = false;
+}
+
+// The phases that the context's steps have, as bits.
+unsigned active_phases(const nb_ctx* c) {
+    if (c->p.mode == NB_MODE_ALLPAIRS) return 1u << 7;
+    if (c->p.mode == NB_MODE_FP64) return 1u | 2u | 4u | 16u | 32u | 128u | 256u;
+    // with quadrupoles the groups are built while the moments run, as part of them
+    unsigned a = 1u | 2u | 4u | 16u | 128u;
+    a |= (c->p.flags & NB_FLAG_QUADRUPOLE) ? 32u : 8u | 64u;
+    if (c->p.flags & NB_FLAG_LEARNED) a |= 256u;
+    return a;
 }
 
 int capture_graph(nb_ctx* c, int parity) {
@@ -449,8 +439,6 @@ int create_context(const nb_params* p, uint64_t n, const double* mass, const dou
         cudaEventCreateWithFlags(&c->copied, cudaEventDisableTiming) != cudaSuccess) {
         rc = NB_ERR_CUDA;
     }
-    for (auto& e : c->phase_ev)
-        if (rc == NB_OK && cudaEventCreate(&e) != cudaSuccess) rc = NB_ERR_CUDA;
     if (rc == NB_OK) rc = alloc_all(c);
     if (rc == NB_OK && counts) rc = alloc_batch(c, nuni, counts);
     if (rc == NB_OK) rc = nb_upload(c, mass, pos_xy, vel_xy);
@@ -509,8 +497,6 @@ int nb_destroy(nb_ctx* c) {
         if (u.used) cudaEventDestroy(u.used);
     }
     if (c->up_stream) cudaStreamDestroy(c->up_stream);
-    for (auto& e : c->phase_ev)
-        if (e) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return NB_OK;
@@ -723,7 +709,7 @@ int nb_debug_morton(nb_ctx* c, uint64_t* codes, int32_t* order, double* box_out)
     if (!c) return NB_ERR_INVALID;
     DeviceGuard guard(c->device);
     const nb::BodyBuffers& A = c->buf[c->parity];
-    nb::launch_bbox(c, A.pos);
+    nb::launch_bbox(c, A.pos, false);
     nb::launch_morton(c, A.pos);
     nb::launch_sort(c);
     NB_CUDA(c, cudaGetLastError());
@@ -863,11 +849,16 @@ int nb_phase_times(nb_ctx* c, double* ms, int max) {
     if (!c || (!ms && max > 0)) return -NB_ERR_INVALID;
     DeviceGuard guard(c->device);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return -NB_ERR_CUDA;
-    for (int k = 0; k < nb::kPhases && k < max; ++k) {
-        float t = 0.f;
-        ms[k] = cudaEventElapsedTime(&t, c->phase_ev[k], c->phase_ev[k + 1]) == cudaSuccess ? t : -1.0;
-    }
-    cudaGetLastError();
+    unsigned long long t[nb::kPhases + 1];
+    if (cudaMemcpy(t, c->scal->marks, sizeof(t), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return -NB_ERR_CUDA;
+    const unsigned active = active_phases(c);
+    const bool stepped = t[nb::kPhases] != 0;
+    // a phase lasts until the next one that the steps have begins
+    for (int k = nb::kPhases - 1; k >= 0; --k)
+        if (!((active >> k) & 1u) || t[k] > t[k + 1]) t[k] = t[k + 1];
+    for (int k = 0; k < nb::kPhases && k < max; ++k)
+        ms[k] = stepped ? (double)(t[k + 1] - t[k]) * 1e-6 : -1.0;
     return nb::kPhases;
 }
 
@@ -1004,14 +995,14 @@ int nb_mlp_samples(nb_ctx* c, uint64_t ntargets, uint64_t seed, uint64_t capacit
     // sorted bodies, tree and moments of the current state, without integrating
     const nb::BodyBuffers& A = c->buf[c->parity];
     const nb::BodyBuffers& B = c->buf[c->parity ^ 1];
-    nb::launch_bbox(c, A.pos);
+    nb::launch_bbox(c, A.pos, false);
     nb::launch_morton(c, A.pos);
     nb::launch_sort(c);
     nb::launch_gather(c, A, B, c->tree.body4);
     nb::launch_tree(c, B);
     nb::launch_moments(c, B, true);
-    nb::launch_features(c, B);
-    nb::launch_groups(c);
+    nb::launch_features(c, B, true);
+    nb::launch_groups(c, true);
     NB_CUDA(c, cudaGetLastError());
     c->parity ^= 1;
     // target groups: a seeded uniform choice (splitmix64), reduced modulo the

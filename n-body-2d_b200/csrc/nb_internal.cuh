@@ -54,6 +54,9 @@ struct DeviceScalars {
     // sort.  sort_passes_forced != 0 overrides the choice (tests).
     int32_t sort_passes;
     int32_t sort_passes_forced;
+    // start of each phase of the last graph-launched step, and its end (ns of
+    // the device's global timer)
+    unsigned long long marks[kPhases + 1];
     unsigned lcp_hist[33];    // neighbouring codes sharing d leading 2-bit digits (d = 32: equal)
     unsigned tie_count[2];    // tie groups of <= 32 keys / of more keys, this step
 };
@@ -177,7 +180,7 @@ struct nb_ctx {
     cudaEvent_t staged = nullptr;        // the download's scatter into the staging buffers is done
     cudaEvent_t copied = nullptr;        // the staging buffers have been copied out (free again)
     cudaStream_t up_stream = nullptr;    // nb_upload_async: host-to-device copies
-    cudaEvent_t phase_ev[nb::kPhases + 1] = {};
+    bool marks_on = false;          // the kernels being enqueued write scal->marks
     int parity = 0;                 // which BodyBuffers holds the state
     nb::BodyBuffers buf[2];
     nb::SortBuffers sort;
@@ -291,8 +294,59 @@ __device__ __forceinline__ int choose_sort_passes(const unsigned* hist, int64_t 
     return 8;
 }
 
+// ---- the step's kernel chain ----------------------------------------------
+// A step is a chain of some 30 kernels, most of them a few microseconds long
+// below a million bodies, so the gaps between them count.  Its kernels are
+// launched with programmatic stream serialization: each begins with
+// chain_begin(), which lets the next kernel's blocks be launched as soon as all
+// blocks of this one run, and then waits until the kernel before has
+// completed and its writes are visible.  Nothing is read or written before
+// that wait, so the order of memory accesses is that of plain launches.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// chained = false: an ordinary launch (the first kernel of a step, or one that
+// follows a copy, an event or another stream).
+template <typename... Ps, typename... As>
+inline void chain_launch(cudaStream_t st, bool chained, void (*kernel)(Ps...), dim3 grid,
+                         dim3 block, size_t smem, As... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Ps>(args)...);
+}
+
+// Phase times: the first kernel of phase k writes marks[k] (mark_start), the
+// last kernel of the step raises marks[kPhases] to the end of its last block
+// (mark_end).  Event nodes in the graph cost 2.6 us each and cut the chain.
+inline unsigned long long* mark_of(const nb_ctx* c, int k) {
+    return c->marks_on ? &c->scal->marks[k] : nullptr;
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void mark_start(unsigned long long* mark) {
+    if (mark && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *mark = global_ns();
+}
+// Only the grid's last blocks can be the last to end.
+__device__ __forceinline__ void mark_end(unsigned long long* mark) {
+    if (mark && threadIdx.x == 0 && blockIdx.x + 2048 >= gridDim.x) atomicMax(mark, global_ns());
+}
+
 // Kernel launchers (all enqueue on ctx->stream, no host synchronisation).
-void launch_bbox(nb_ctx* c, const double2* pos);
+// new_step: the interaction counters start at zero
+void launch_bbox(nb_ctx* c, const double2* pos, bool new_step);
 void launch_morton(nb_ctx* c, const double2* pos);
 void launch_batch_roots(nb_ctx* c);   // per-universe root cells after the tree build
 void launch_sort(nb_ctx* c);
@@ -304,7 +358,7 @@ void launch_prefix_sums(nb_ctx* c, const BodyBuffers& b);
 void launch_tree(nb_ctx* c, const BodyBuffers& b, bool prefix_done = false);
 void launch_moments(nb_ctx* c, const BodyBuffers& b, bool split);
 // learned mode: second and third moments and the BF16 feature records
-void launch_features(nb_ctx* c, const BodyBuffers& b);
+void launch_features(nb_ctx* c, const BodyBuffers& b, bool chained);
 int split_group_size(const nb_ctx* c);   // bodies per SPLIT traversal group
 void launch_mlp_correct(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc);
 size_t mlp_infer_bytes();
@@ -323,8 +377,8 @@ size_t mlp_train_image_bytes();
 int mlp_grad_tc_device(const float* params, const float* X, const float* Yt, const int64_t* idx,
                        int64_t n, float* grad, float* loss, void* image, unsigned* err,
                        int sm_count, cudaStream_t st);
-void launch_groups(nb_ctx* c);
-void launch_force_split(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc);
+void launch_groups(nb_ctx* c, bool chained);
+void launch_force_split(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc, bool chained);
 void launch_force_fp64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc);
 void launch_drift(nb_ctx* c, const BodyBuffers& b);
 void launch_upload_check(nb_ctx* c, const BodyBuffers& b, unsigned* bad);
