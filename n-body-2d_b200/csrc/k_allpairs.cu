@@ -234,7 +234,7 @@ void launch_partial(const double2* pos, const double* mass, int64_t n, const int
     const int64_t chunk = (n + chunks - 1) / chunks;
     nb::chain_launch(st, chained,
                      k >= kTwoPerThread ? allpairs_partial<kCpuLaw, 2> : allpairs_partial<kCpuLaw, 1>,
-                     grid, kThreads, 0, pos, mass, n, targets, k, chunk, eps2, partial);
+                     grid, kThreads, 0, 1, pos, mass, n, targets, k, chunk, eps2, partial);
 }
 
 }  // namespace
@@ -246,7 +246,7 @@ void nb::launch_allpairs_step(nb_ctx* c, const BodyBuffers& a, const BodyBuffers
     const unsigned blocks = (unsigned)((c->n + kThreads - 1) / kThreads);
     const int chunks = allpairs_chunks(c->n, c->sm_count);
     c->launches += 3;
-    chain_launch(c->stream, false, allpairs_drift, blocks, kThreads, 0, a, b, c->n,
+    chain_launch(c->stream, false, allpairs_drift, blocks, kThreads, 0, 1, a, b, c->n,
                  integrate ? c->p.timestep : 0.0, c->scal, mark_of(c, 7));
     if (c->p.flags & NB_FLAG_CPU_LAW)
         launch_partial<true>(b.pos, b.mass, c->n, nullptr, c->n, chunks, c->p.epsilon_squared,
@@ -254,7 +254,7 @@ void nb::launch_allpairs_step(nb_ctx* c, const BodyBuffers& a, const BodyBuffers
     else
         launch_partial<false>(b.pos, b.mass, c->n, nullptr, c->n, chunks, c->p.epsilon_squared,
                               c->ap_partial, c->stream, true);
-    chain_launch(c->stream, true, allpairs_kick, blocks, kThreads, 0, c->ap_partial, chunks, c->n,
+    chain_launch(c->stream, true, allpairs_kick, blocks, kThreads, 0, 1, c->ap_partial, chunks, c->n,
                  b.vel, store_acc ? c->acc : nullptr, c->p.G * c->p.timestep, integrate ? 1 : 0,
                  &c->scal->body_terms, mark_of(c, kPhases));
 }

@@ -520,7 +520,7 @@ void launch_split_soft(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_ac
     const float theta2 = (float)(c->p.theta * c->p.theta);
     const int leaf = c->p.leaf_size > 0 ? c->p.leaf_size : kDefaultLeaf;
     chain_launch(c->stream, chained, force_split<kQuad, kBPL, kLearned, kZeroSoft>, grid,
-                 32 * kWarpsPerBlock, 0, b.pos, b.vel, store_acc ? c->acc : nullptr, c->acc32,
+                 32 * kWarpsPerBlock, 0, 1, b.pos, b.vel, store_acc ? c->acc : nullptr, c->acc32,
                  (int)c->n, c->tree, c->scal, c->batch, eps2, theta2, leaf, c->p.G * c->p.timestep,
                  c->p.timestep, kick ? 1 : 0, band_theta(c) * band_theta(c), mark_of(c, 7),
                  kLearned ? nullptr : mark_of(c, kPhases));

@@ -455,7 +455,7 @@ template <int kG, bool kTerms>
 void launch_walk64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc) {
     const int64_t groups = (c->n + kG - 1) / kG;
     chain_launch(c->stream, true, force_fp64<kG, kTerms>,
-                 (unsigned)((groups + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0,
+                 (unsigned)((groups + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, 1,
                  b.pos, b.mass, b.vel, store_acc ? c->acc : nullptr, (int)c->n, c->tree, c->scal,
                  c->p.epsilon_squared, c->p.theta * c->p.theta, c->p.G * c->p.timestep, kick ? 1 : 0,
                  kTerms ? c->dbg_terms : nullptr, mark_of(c, 7));
@@ -563,7 +563,7 @@ void launch_force_fp64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_ac
 
 void launch_drift(nb_ctx* c, const BodyBuffers& b) {
     c->launches += 1;
-    chain_launch(c->stream, true, drift_kernel, blocks_for(c->n, 256), 256, 0, b.pos, b.vel, c->n,
+    chain_launch(c->stream, true, drift_kernel, blocks_for(c->n, 256), 256, 0, 1, b.pos, b.vel, c->n,
                  c->p.timestep, mark_of(c, 8), mark_of(c, kPhases));
 }
 

@@ -6,10 +6,15 @@
 // the sort is a project-written stable LSD radix sort over all 64 key bits,
 // so its order equals cub::DeviceRadixSort::SortPairs at CU:692 (any stable
 // sort of (code, current index) gives the same permutation).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "nb_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace nb {
 namespace {
@@ -26,18 +31,23 @@ __device__ __forceinline__ double warp_max(double v) {
     return v;
 }
 
-// Chooses this step's radix passes (the top bytes of the key the sort orders
-// by) and resets the counters of the tie pass; the histogram of the last tree
-// is consumed.  Without `adaptive` (or with a forced count) no histogram is
-// used.
-// Also resets what the later kernels of a step count in, and in a new step the
-// interaction counters.
-__device__ __forceinline__ void start_sort(DeviceScalars* s, int64_t n, int adaptive,
-                                           int new_step) {
-    int passes = adaptive ? choose_sort_passes(s->lcp_hist, n) : 8;
-    if (s->sort_passes_forced > 0) passes = min(s->sort_passes_forced, 8);
+// This step's radix passes (the top bytes of the key the sort orders by), from
+// the histogram of the last tree.  Without `adaptive` (or with a forced count)
+// no histogram is used.  One warp.
+__device__ __forceinline__ int sort_passes_of(const DeviceScalars* s, int64_t n, int adaptive) {
+    const int forced = s->sort_passes_forced;
+    if (forced > 0) return min(forced, 8);
+    return adaptive ? choose_sort_passes(s->lcp_hist, n) : 8;
+}
+
+// Consumes the histogram and resets what the later kernels of a step count in,
+// and in a new step the interaction counters.  One warp.
+__device__ __forceinline__ void start_sort(DeviceScalars* s, int passes, int new_step) {
+    const int lane = threadIdx.x & 31;
+    s->lcp_hist[lane] = 0;
+    if (lane != 0) return;
     s->sort_passes = passes;
-    for (int d = 0; d <= 32; ++d) s->lcp_hist[d] = 0;
+    s->lcp_hist[32] = 0;
     s->tie_count[0] = 0;
     s->tie_count[1] = 0;
     s->nstart = 0;
@@ -76,6 +86,43 @@ __device__ __forceinline__ void box_fold(double& xmin, double& xmax, double& ymi
             ymin = fmin(ymin, red[2][w]);
             ymax = fmax(ymax, red[3][w]);
         }
+    }
+}
+
+// The squared root box of the extremes (host squaring, CU:665-677) and the
+// Morton kernel's scale factors (CU:122-123).
+struct RootBox {
+    double x0, x1, y0, y1, inv_w, inv_h;
+};
+__device__ __forceinline__ RootBox square_box(double bx0, double bx1, double by0, double by1) {
+    const double x_range = bx1 - bx0;
+    const double y_range = by1 - by0;
+    if (x_range > y_range) {
+        const double mid = (by0 + by1) * 0.5;
+        by0 = mid - x_range * 0.5;
+        by1 = mid + x_range * 0.5;
+    } else {
+        const double mid = (bx0 + bx1) * 0.5;
+        bx0 = mid - y_range * 0.5;
+        bx1 = mid + y_range * 0.5;
+    }
+    return {bx0, bx1, by0, by1, 1.0 / (bx1 - bx0), 1.0 / (by1 - by0)};
+}
+__device__ __forceinline__ void write_box(DeviceScalars* s, const RootBox& b) {
+    s->box[0] = b.x0;
+    s->box[1] = b.x1;
+    s->box[2] = b.y0;
+    s->box[3] = b.y1;
+    s->center[0] = 0.5 * (b.x0 + b.x1);
+    s->center[1] = 0.5 * (b.y0 + b.y1);
+    s->inv_wh[0] = b.inv_w;
+    s->inv_wh[1] = b.inv_h;
+    // CU:717 root width_sq, then CU:216 child_wsq = parent * 0.25 per level.
+    const double w = b.x1 - b.x0;
+    double wsq = w * w;
+    for (int l = 0; l <= kMaxLevel; ++l) {
+        s->wsq[l] = wsq;
+        wsq *= 0.25;
     }
 }
 
@@ -133,36 +180,14 @@ bbox_kernel(const double2* __restrict__ pos, int64_t n, double* __restrict__ par
     }
     __syncthreads();  // red[] is reused
     box_fold(bx0, bx1, by0, by1, red);
+    if (threadIdx.x < 32) {
+        const int passes = sort_passes_of(s, n, adaptive);
+        __syncwarp();
+        start_sort(s, passes, new_step);
+    }
     if (threadIdx.x == 0) {
-        const double x_range = bx1 - bx0;
-        const double y_range = by1 - by0;
-        if (x_range > y_range) {
-            const double mid = (by0 + by1) * 0.5;
-            by0 = mid - x_range * 0.5;
-            by1 = mid + x_range * 0.5;
-        } else {
-            const double mid = (bx0 + bx1) * 0.5;
-            bx0 = mid - y_range * 0.5;
-            bx1 = mid + y_range * 0.5;
-        }
-        s->box[0] = bx0;
-        s->box[1] = bx1;
-        s->box[2] = by0;
-        s->box[3] = by1;
-        s->center[0] = 0.5 * (bx0 + bx1);
-        s->center[1] = 0.5 * (by0 + by1);
-        // the Morton kernel's scale factors (CU:122-123), divided once here
-        s->inv_wh[0] = 1.0 / (bx1 - bx0);
-        s->inv_wh[1] = 1.0 / (by1 - by0);
-        // CU:717 root width_sq, then CU:216 child_wsq = parent * 0.25 per level.
-        const double w = bx1 - bx0;
-        double wsq = w * w;
-        for (int l = 0; l <= kMaxLevel; ++l) {
-            s->wsq[l] = wsq;
-            wsq *= 0.25;
-        }
+        write_box(s, square_box(bx0, bx1, by0, by1));
         s->bbox_ticket = 0;
-        start_sort(s, n, adaptive, new_step);
     }
 }
 
@@ -176,10 +201,10 @@ __device__ __forceinline__ uint64_t expand_bits_2d(uint32_t v) {
     return x;
 }
 
-// What a sort counts in: the digit histograms, the tile counters and the
-// status words of the passes it will run.
+// What the onesweep passes count in: the digit histograms, the tile counters
+// and the status words of the passes that will run.  The Morton pass resets it.
 struct SortState {
-    uint32_t* hist = nullptr;     // nullptr: nothing to reset
+    uint32_t* hist = nullptr;     // nullptr: no onesweep passes follow
     unsigned* tile_counter = nullptr;
     uint32_t* status = nullptr;
     int tiles = 0;
@@ -192,6 +217,15 @@ __device__ __forceinline__ void reset_sort(const SortState& z, int passes) {
     for (int64_t k = t0; k < 8 * 256; k += step) z.hist[k] = 0;
     if (t0 < 8) z.tile_counter[t0] = 0;
     for (int64_t k = (8 - passes) * per_pass + t0; k < 8 * per_pass; k += step) z.status[k] = 0;
+}
+
+__device__ __forceinline__ uint64_t morton_code(double2 p, double x0, double y0, double inv_w,
+                                                double inv_h) {
+    const double nx = (p.x - x0) * inv_w;
+    const double ny = (p.y - y0) * inv_h;
+    const uint32_t ix = __double2uint_rd(fmin(fmax(nx * 4294967296.0, 0.0), 4294967295.0));
+    const uint32_t iy = __double2uint_rd(fmin(fmax(ny * 4294967296.0, 0.0), 4294967295.0));
+    return (expand_bits_2d(ix) << 1) | expand_bits_2d(iy);
 }
 
 // CU:117-132: code from (p - min) * (1 / width), quantised to 32 bits per axis
@@ -210,14 +244,7 @@ __global__ void morton_kernel(const double2* __restrict__ pos, int64_t n,
     const bool odd = s->sort_passes & 1;
     uint64_t* __restrict__ key = odd ? key1 : key0;
     uint32_t* __restrict__ val = odd ? val1 : val0;
-    const double x0 = s->box[0], y0 = s->box[2];
-    const double inv_w = s->inv_wh[0], inv_h = s->inv_wh[1];
-    const double2 p = __ldg(pos + i);
-    const double nx = (p.x - x0) * inv_w;
-    const double ny = (p.y - y0) * inv_h;
-    const uint32_t ix = __double2uint_rd(fmin(fmax(nx * 4294967296.0, 0.0), 4294967295.0));
-    const uint32_t iy = __double2uint_rd(fmin(fmax(ny * 4294967296.0, 0.0), 4294967295.0));
-    key[i] = (expand_bits_2d(ix) << 1) | expand_bits_2d(iy);
+    key[i] = morton_code(__ldg(pos + i), s->box[0], s->box[2], s->inv_wh[0], s->inv_wh[1]);
     val[i] = (uint32_t)i;
 }
 
@@ -273,7 +300,11 @@ __global__ void bbox_batch_finish(Batch b, DeviceScalars* __restrict__ s, int64_
                                   int new_step) {
     chain_begin();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u == 0) start_sort(s, n, 1, new_step);
+    if (u < 32) {
+        const int passes = sort_passes_of(s, n, 1);
+        __syncwarp();
+        start_sort(s, passes, new_step);
+    }
     if (u >= b.nuni) return;
     unsigned long long* e = b.boxbits + 4 * u;
     double x0 = from_ordered(e[0]), x1 = from_ordered(~e[1]);
@@ -307,7 +338,8 @@ __global__ void morton_batch_kernel(const double2* __restrict__ pos, int64_t n, 
     reset_sort(z, s->sort_passes);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const bool odd = s->sort_passes & 1;
+    // (cluster sorts read buffer 0)
+    const bool odd = z.hist && (s->sort_passes & 1);
     uint64_t* __restrict__ key = odd ? key1 : key0;
     uint32_t* __restrict__ val = odd ? val1 : val0;
     const int u = b.uid[i];
@@ -323,11 +355,8 @@ __global__ void morton_batch_kernel(const double2* __restrict__ pos, int64_t n, 
 }
 
 // ---------------------------------------------------------------------------
-// LSD radix sort, 8-bit digits, 8 passes.  Each pass: per-tile digit counts
-// (upsweep), a per-digit scan over tiles, and a stable scatter (downsweep)
-// that ranks keys inside the tile with warp-private histograms and
-// __match_any_sync, stages the tile in shared memory sorted by digit, and
-// writes each digit's run with consecutive threads (coalesced).
+// LSD radix sorts with 8-bit digits: inside clusters of blocks up to
+// kClusterSortMax keys, by onesweep passes over global memory above.
 // ---------------------------------------------------------------------------
 constexpr int kWarps = kSortThreads / 32;
 
@@ -364,119 +393,398 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
     return r;
 }
 
-__global__ void __launch_bounds__(kSortThreads)
-sort_upsweep(const uint64_t* __restrict__ key, int64_t n, int shift, uint32_t* __restrict__ counts,
-             int tiles) {
-    __shared__ uint32_t hist[256];
-    hist[threadIdx.x] = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
+// Lanes holding the same 8-bit digit, from eight ballots (the ballot path
+// keeps this off the pipe that serialises __match_any_sync).
+__device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid) {
+    unsigned peers = __ballot_sync(kFull, valid);
+    if (!valid) peers = 0;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const unsigned m = __ballot_sync(kFull, bit);
+        peers &= bit ? m : ~m;
+    }
+    return valid ? peers : (1u << (threadIdx.x & 31));
+}
+
+// ---------------------------------------------------------------------------
+// Cluster sort, up to kClusterSortMax keys.  There a pass over global memory is
+// a chain of latencies (7 us a pass at 16,384 keys), so one cluster of up to 16
+// blocks keeps all keys in shared memory and scatters them between its blocks'
+// shared memories, with one cluster barrier after the digit counts and one
+// after the scatter.  Box, codes and passes are one kernel.  Same order as the
+// onesweep passes: by the top sort_passes bytes, equal ones in input order.
+// Box to sorted keys, us, with onesweep passes and so: 1,001 bodies 37 and 16,
+// 16,384 49 and 32, 32,768 60 and 44.  With four keys a thread (65,536) a pass
+// takes as long as over global memory; sorting chunks by several clusters and
+// merging them took longer (262,144 bodies 69 and 78).
+// ---------------------------------------------------------------------------
+constexpr int kClusterThreads = 1024;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterMost = 16;  // blocks in a cluster
+static_assert(kClusterSortMax == 2 * kClusterMost * kClusterThreads, "at most two keys per thread");
+
+// Where the codes come from: the bodies (box and codes are made here), or
+// key_in (batched universes, whose codes have been made).
+enum { kSrcBodies, kSrcKeys };
+
+template <int kItems>
+struct ClusterSmem {
+    uint64_t key[kClusterThreads * kItems];  // written by the whole cluster
+    uint32_t val[kClusterThreads * kItems];
+    uint64_t own_key[kClusterThreads * kItems];  // this block's keys by digit
+    uint32_t own_val[kClusterThreads * kItems];
+    uint16_t whist[kClusterWarps][256];  // per warp, then exclusive within its part
+    uint32_t match[kClusterWarps][256];  // per warp and digit: the row's lanes with it
+    uint32_t count[256];                 // this block's digits, read by the whole cluster
+    uint32_t before[4][256], total[4][256];
+    uint32_t off[4][256];                // place of a part's keys among the block's
+    uint32_t base[256];                  // place in the cluster less place in the block
+    uint32_t warp_tot[2][8];
+    double red[4][kClusterWarps];
+    double box[4];                       // this block's extremes, read by the whole cluster
+    int passes;
+};
+
+// Rank of this lane's digit d in the warp's keys so far, row by row: the lanes
+// of the row with the same digit set their bits in the digit's word of match[]
+// (all zero between rows), whist[] counts the rows before.
+__device__ __forceinline__ uint32_t row_rank(uint32_t* match, uint16_t* whist, uint32_t d,
+                                             bool valid, unsigned below) {
+    if (valid) atomicOr(&match[d], 1u << (threadIdx.x & 31));
+    __syncwarp();
+    const unsigned peers = valid ? match[d] : 0u;
+    const uint32_t b = valid ? whist[d] : 0u;
+    __syncwarp();
+    if (valid && (peers & below) == 0) {
+        whist[d] = (uint16_t)(b + __popc(peers));
+        match[d] = 0;
+    }
+    __syncwarp();
+    return b + __popc(peers & below);
+}
+
+// Inclusive scan over the threads of each of the first eight warps; their totals.
+__device__ __forceinline__ uint32_t digit_scan(uint32_t v, uint32_t* warp_tot) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int k = 0; k < kSortTileItems; ++k) {
-        const int64_t i = base + k * kSortThreads + threadIdx.x;
-        const bool valid = i < n;
-        const uint32_t d = valid ? (uint32_t)((__ldg(key + i) >> shift) & 0xFF) : 0x100u + lane;
-        const unsigned peers = __match_any_sync(kFull, d);
-        if (valid && lane == __ffs(peers) - 1) atomicAdd(&hist[d], (uint32_t)__popc(peers));
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, v, o);
+        if (lane >= o) v += t;
     }
-    __syncthreads();
-    counts[(int64_t)threadIdx.x * tiles + blockIdx.x] = hist[threadIdx.x];
+    if (lane == 31) warp_tot[threadIdx.x >> 5] = v;
+    return v;
 }
 
-// Block d turns row d of counts into exclusive offsets and writes its total.
-__global__ void __launch_bounds__(kSortThreads)
-sort_scan_rows(uint32_t* __restrict__ counts, int tiles, uint32_t* __restrict__ totals) {
-    __shared__ uint32_t warp_tot[kWarps];
-    __shared__ uint32_t chunk_total;
-    uint32_t* row = counts + (int64_t)blockIdx.x * tiles;
-    uint32_t carry = 0;
-    for (int b = 0; b < tiles; b += kSortThreads) {
-        const int t = b + threadIdx.x;
-        const uint32_t v = t < tiles ? row[t] : 0;
-        const uint32_t ex = block_exclusive_scan(v, warp_tot, &chunk_total);
-        if (t < tiles) row[t] = carry + ex;
-        carry += chunk_total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+// The two halves of a cluster barrier: what a thread wrote before it arrives
+// is visible to the cluster's threads that have waited.
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kSortThreads)
-sort_downsweep(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ val_in,
-               uint64_t* __restrict__ key_out, uint32_t* __restrict__ val_out, int64_t n, int shift,
-               const uint32_t* __restrict__ counts, const uint32_t* __restrict__ totals, int tiles) {
-    __shared__ uint32_t whist[kWarps][256];
-    __shared__ uint32_t tile_start[256];
-    __shared__ uint32_t goff[256];
-    __shared__ uint32_t warp_tot[kWarps];
-    __shared__ uint64_t skey[kSortTile];
-    __shared__ uint32_t sval[kSortTile];
-
+template <int kItems, int kSrc>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+cluster_sort(const double2* __restrict__ pos, int64_t n, DeviceScalars* __restrict__ s, int adaptive,
+             int new_step, int fixed_passes, const uint64_t* key_in, uint64_t* key_out,
+             uint32_t* __restrict__ val_out, unsigned long long* mark0, unsigned long long* mark1) {
+    chain_begin();
+    mark_start(mark0);
+    constexpr int kTile = kClusterThreads * kItems;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ClusterSmem<kItems>& S = *reinterpret_cast<ClusterSmem<kItems>*>(smem_raw);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int me = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int part = tid >> 8, digit = tid & 255;
+    // a warp's keys: kItems rows of 32; slots from n on (the last chunk's end) stay empty
+    const int slot0 = warp * 32 * kItems + lane;
+    const int64_t first = (int64_t)blockIdx.x * kTile + slot0;
+    uint64_t k_reg[kItems];
+    uint32_t v_reg[kItems], r_reg[kItems];
+    int passes = fixed_passes;
+    if (kSrc == kSrcKeys) {
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) whist[w][tid] = 0;
-    {
-        const uint32_t tot = totals[tid];
-        const uint32_t pre = block_exclusive_scan(tot, warp_tot, nullptr);
-        goff[tid] = pre + counts[(int64_t)tid * tiles + blockIdx.x];
+        for (int k = 0; k < kItems; ++k) k_reg[k] = first + 32 * k < n ? key_in[first + 32 * k] : 0ull;
+        if (passes == 0) passes = s->sort_passes;
+    } else {
+        double2 p[kItems];
+#pragma unroll
+        for (int k = 0; k < kItems; ++k)
+            p[k] = first + 32 * k < n ? __ldg(pos + first + 32 * k) : make_double2(0.0, 0.0);
+        RootBox box;
+        {
+            double v[4] = {INFINITY, -INFINITY, INFINITY, -INFINITY};
+#pragma unroll
+            for (int k = 0; k < kItems; ++k)
+                if (first + 32 * k < n) {
+                    v[0] = fmin(v[0], p[k].x);
+                    v[1] = fmax(v[1], p[k].x);
+                    v[2] = fmin(v[2], p[k].y);
+                    v[3] = fmax(v[3], p[k].y);
+                }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                v[q] = (q & 1) ? warp_max(v[q]) : warp_min(v[q]);
+                if (lane == 0) S.red[q][warp] = v[q];
+            }
+            __syncthreads();
+            if (warp < 4) {  // warp q folds extreme q
+                const double x = S.red[warp][lane];
+                const double f = (warp & 1) ? warp_max(x) : warp_min(x);
+                if (lane == 0) S.box[warp] = f;
+            } else if (warp == 4) {
+                const int chosen = fixed_passes ? fixed_passes : sort_passes_of(s, n, adaptive);
+                if (lane == 0) S.passes = chosen;
+            }
+            cluster.sync();
+            double m[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double x = cluster.map_shared_rank(S.box, min(lane, blocks - 1))[q];
+                m[q] = (q & 1) ? warp_max(x) : warp_min(x);
+            }
+            box = square_box(m[0], m[1], m[2], m[3]);
+            passes = S.passes;
+            if (me == 0 && warp == 0) {  // the cluster has read the histogram
+                start_sort(s, passes, new_step);
+                if (lane == 0) write_box(s, box);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) k_reg[k] = morton_code(p[k], box.x0, box.y0, box.inv_w, box.inv_h);
     }
-    __syncthreads();
+    mark_start(mark1);
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) v_reg[k] = (uint32_t)(first + 32 * k);
+    const unsigned below = lanemask_lt();
+    const int held = (int)max((int64_t)0, min((int64_t)kTile, n - (int64_t)blockIdx.x * kTile));
+#pragma unroll
+    for (int k = lane; k < 256; k += 32) S.match[warp][k] = 0;
+    for (int pass = 8 - passes; pass < 8; ++pass) {
+#pragma unroll
+        for (int k = lane; k < 128; k += 32) reinterpret_cast<uint32_t*>(S.whist[warp])[k] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k)
+            r_reg[k] = row_rank(S.match[warp], S.whist[warp], (uint32_t)(k_reg[k] >> (8 * pass)) & 255u,
+                                first + 32 * k < n, below);
+        __syncthreads();
+        {   // exclusive over the part's warps
+            uint32_t run = 0;
+#pragma unroll
+            for (int w = 0; w < kClusterWarps / 4; ++w) {
+                const uint32_t c = S.whist[part * (kClusterWarps / 4) + w][digit];
+                S.whist[part * (kClusterWarps / 4) + w][digit] = (uint16_t)run;
+                run += c;
+            }
+            S.off[part][digit] = run;
+        }
+        __syncthreads();
+        // places in the block: exclusive scan of its digit counts
+        uint32_t count = 0, inc = 0, mine = 0;
+        if (tid < 256) {
+            count = S.off[0][tid] + S.off[1][tid] + S.off[2][tid] + S.off[3][tid];
+            S.count[tid] = count;
+            inc = digit_scan(count, S.warp_tot[0]);
+        }
+        cluster_arrive();  // (the counts)
+        __syncthreads();
+        if (tid < 256) {
+            mine = inc - count;
+            for (int w = 0; w < warp; ++w) mine += S.warp_tot[0][w];
+            uint32_t off = mine;
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const uint32_t c = S.off[p][tid];
+                S.off[p][tid] = off;
+                off += c;
+            }
+        }
+        __syncthreads();
+        // the block's keys by digit, so that they leave in runs
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            if (first + 32 * k >= n) continue;
+            const uint32_t d = (uint32_t)(k_reg[k] >> (8 * pass)) & 255u;
+            const uint32_t at = S.off[part][d] + S.whist[warp][d] + r_reg[k];
+            S.own_key[at] = k_reg[k];
+            S.own_val[at] = v_reg[k];
+        }
+        cluster_wait();  // every block's counts are there, and its keys in registers
+        {   // this digit in a quarter of the blocks: before this block, and in all
+            uint32_t before = 0, total = 0;
+            for (int c = part; c < blocks; c += 4) {
+                const uint32_t x = cluster.map_shared_rank(S.count, c)[digit];
+                total += x;
+                before += c < me ? x : 0u;
+            }
+            S.before[part][digit] = before;
+            S.total[part][digit] = total;
+        }
+        __syncthreads();
+        if (tid < 256) {  // the digits' bases: exclusive scan of their totals
+            count = S.total[0][tid] + S.total[1][tid] + S.total[2][tid] + S.total[3][tid];
+            inc = digit_scan(count, S.warp_tot[1]);
+        }
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t off = inc - count - mine;
+            for (int w = 0; w < warp; ++w) off += S.warp_tot[1][w];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) off += S.before[p][tid];
+            S.base[tid] = off;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const int j = k * kClusterThreads + tid;
+            if (j >= held) continue;
+            const uint64_t key = S.own_key[j];
+            const uint32_t at = S.base[(uint32_t)(key >> (8 * pass)) & 255u] + (uint32_t)j;
+            cluster.map_shared_rank(S.key, at / kTile)[at % kTile] = key;
+            cluster.map_shared_rank(S.val, at / kTile)[at % kTile] = S.own_val[j];
+        }
+        cluster.sync();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            k_reg[k] = S.key[slot0 + 32 * k];
+            v_reg[k] = S.val[slot0 + 32 * k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k)
+        if (first + 32 * k < n) {
+            key_out[first + 32 * k] = k_reg[k];
+            val_out[first + 32 * k] = v_reg[k];
+        }
+}
 
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    const int64_t seg = base + warp * (32 * kSortTileItems);
-    uint64_t k_reg[kSortTileItems];
-    uint32_t v_reg[kSortTileItems];
-    uint32_t r_reg[kSortTileItems];
+// ---------------------------------------------------------------------------
+// Counting passes (nb_morton_sort_static above kClusterSortMax keys): one
+// kernel counts each tile's digits, the next adds up the counts of the tiles
+// before its own and scatters.  No block waits on another, so the stage needs
+// no error word, which that entry point could not report.
+// ---------------------------------------------------------------------------
+constexpr int kCountThreads = 1024;
+constexpr int kCountItems = kCountTile / kCountThreads;
+constexpr int kCountWarps = kCountThreads / 32;
+
+__global__ void __launch_bounds__(kCountThreads)
+count_digits(const uint64_t* __restrict__ key, int64_t n, int pass, uint16_t* __restrict__ counts) {
+    chain_begin();
+    __shared__ uint32_t hist[4][256];  // one per quarter of the block
+    const int tid = threadIdx.x, part = tid >> 8;
+    hist[part][tid & 255] = 0;
+    const int64_t base = (int64_t)blockIdx.x * kCountTile + tid;
+    uint64_t k[kCountItems];
+#pragma unroll
+    for (int q = 0; q < kCountItems; ++q)
+        k[q] = base + q * kCountThreads < n ? key[base + q * kCountThreads] : 0ull;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kCountItems; ++q)
+        if (base + q * kCountThreads < n)
+            atomicAdd(&hist[part][(uint32_t)(k[q] >> (8 * pass)) & 255u], 1u);
+    __syncthreads();
+    if (tid < 256)
+        counts[(int64_t)blockIdx.x * 256 + tid] =
+            (uint16_t)(hist[0][tid] + hist[1][tid] + hist[2][tid] + hist[3][tid]);
+}
+
+__global__ void __launch_bounds__(kCountThreads, 1)
+count_scatter(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ val_in,
+              uint64_t* __restrict__ key_out, uint32_t* __restrict__ val_out, int64_t n, int pass,
+              const uint16_t* __restrict__ counts, int tiles) {
+    chain_begin();
+    __shared__ uint16_t whist[kCountWarps][256];  // per warp, then exclusive within its part
+    __shared__ uint32_t match[kCountWarps][256];  // per warp and digit: the row's lanes with it
+    // after the ranking, in match[]'s place (48 KB of static shared memory)
+    auto* before = reinterpret_cast<uint32_t(*)[256]>(&match[0][0]);
+    auto* total = reinterpret_cast<uint32_t(*)[256]>(&match[8][0]);
+    auto* off = reinterpret_cast<uint32_t(*)[256]>(&match[16][0]);
+    uint32_t* warp_tot = &match[20][0];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tile = blockIdx.x, part = tid >> 8, digit = tid & 255;
+    // a warp's keys: kCountItems rows of 32
+    const int64_t first = (int64_t)tile * kCountTile + warp * (32 * kCountItems) + lane;
+    uint64_t k_reg[kCountItems];
+    uint32_t v_reg[kCountItems], r_reg[kCountItems];
+#pragma unroll
+    for (int k = 0; k < kCountItems; ++k) {
+        const bool valid = first + 32 * k < n;
+        k_reg[k] = valid ? key_in[first + 32 * k] : 0ull;
+        v_reg[k] = valid ? val_in[first + 32 * k] : 0u;
+    }
+    // two digits in an eighth of the tiles: before this tile, and in all
+    uint32_t lo_before = 0, hi_before = 0, lo_all = 0, hi_all = 0;
+    {
+        const uint32_t* pairs = reinterpret_cast<const uint32_t*>(counts) + (tid & 127);
+#pragma unroll 8
+        for (int q = tid >> 7; q < tiles; q += 8) {
+            const uint32_t x = pairs[q * 128], lo = x & 0xffffu, hi = x >> 16;
+            lo_all += lo;
+            hi_all += hi;
+            lo_before += q < tile ? lo : 0u;
+            hi_before += q < tile ? hi : 0u;
+        }
+    }
+#pragma unroll
+    for (int k = lane; k < 128; k += 32) reinterpret_cast<uint32_t*>(whist[warp])[k] = 0;
+#pragma unroll
+    for (int k = lane; k < 256; k += 32) match[warp][k] = 0;
+    __syncwarp();
     const unsigned below = lanemask_lt();
 #pragma unroll
-    for (int k = 0; k < kSortTileItems; ++k) {
-        const int64_t i = seg + k * 32 + lane;
-        const bool valid = i < n;
-        k_reg[k] = valid ? key_in[i] : 0ull;
-        v_reg[k] = valid ? val_in[i] : 0u;
-        const uint32_t d = valid ? (uint32_t)((k_reg[k] >> shift) & 0xFF) : 0x100u + lane;
-        const unsigned peers = __match_any_sync(kFull, d);
-        const int leader = __ffs(peers) - 1;
-        uint32_t b = 0;
-        if (valid && lane == leader) {
-            b = whist[warp][d];
-            whist[warp][d] = b + __popc(peers);
-        }
-        b = __shfl_sync(kFull, b, leader);
-        r_reg[k] = b + __popc(peers & below);
-        __syncwarp();
-    }
+    for (int k = 0; k < kCountItems; ++k)
+        r_reg[k] = row_rank(match[warp], whist[warp], (uint32_t)(k_reg[k] >> (8 * pass)) & 255u,
+                            first + 32 * k < n, below);
     __syncthreads();
-    {
+    before[tid >> 7][2 * (tid & 127)] = lo_before;
+    before[tid >> 7][2 * (tid & 127) + 1] = hi_before;
+    total[tid >> 7][2 * (tid & 127)] = lo_all;
+    total[tid >> 7][2 * (tid & 127) + 1] = hi_all;
+    {   // exclusive over the part's warps
         uint32_t run = 0;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t c = whist[w][tid];
-            whist[w][tid] = run;
+        for (int w = 0; w < kCountWarps / 4; ++w) {
+            const uint32_t c = whist[part * (kCountWarps / 4) + w][digit];
+            whist[part * (kCountWarps / 4) + w][digit] = (uint16_t)run;
             run += c;
         }
-        tile_start[tid] = block_exclusive_scan(run, warp_tot, nullptr);
+        off[part][digit] = run;
+    }
+    __syncthreads();
+    // the digits' bases: exclusive scan of their totals
+    uint32_t sum = 0, inc = 0;
+    if (tid < 256) {
+#pragma unroll
+        for (int p = 0; p < 8; ++p) sum += total[p][tid];
+        inc = digit_scan(sum, warp_tot);
+    }
+    __syncthreads();
+    if (tid < 256) {
+        uint32_t o = inc - sum;
+        for (int w = 0; w < warp; ++w) o += warp_tot[w];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) o += before[p][tid];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const uint32_t c = off[p][tid];
+            off[p][tid] = o;
+            o += c;
+        }
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kSortTileItems; ++k) {
-        const int64_t i = seg + k * 32 + lane;
-        if (i < n) {
-            const uint32_t d = (uint32_t)((k_reg[k] >> shift) & 0xFF);
-            const uint32_t lp = tile_start[d] + whist[warp][d] + r_reg[k];
-            skey[lp] = k_reg[k];
-            sval[lp] = v_reg[k];
-        }
-    }
-    __syncthreads();
-    const int tile_n = (int)min((int64_t)kSortTile, n - base);
-    for (int p = tid; p < tile_n; p += kSortThreads) {
-        const uint64_t kk = skey[p];
-        const uint32_t d = (uint32_t)((kk >> shift) & 0xFF);
-        const uint32_t gp = goff[d] + (uint32_t)p - tile_start[d];
-        key_out[gp] = kk;
-        val_out[gp] = sval[p];
+    for (int k = 0; k < kCountItems; ++k) {
+        if (first + 32 * k >= n) continue;
+        const uint32_t d = (uint32_t)(k_reg[k] >> (8 * pass)) & 255u;
+        const uint32_t at = off[part][d] + whist[warp][d] + r_reg[k];
+        key_out[at] = k_reg[k];
+        val_out[at] = v_reg[k];
     }
 }
 
@@ -494,6 +802,7 @@ constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kCountMask = (1u << 30) - 1;
 constexpr int kSpinLimit = 1 << 22;
+constexpr int kLook = 4;  // (8: 64 registers spill; 4M sort 296 and 307 us)
 
 // Histograms of the digits the radix passes sort (the top sort_passes bytes;
 // the passes below return at once and need none).  A warp reads rows of 32
@@ -552,31 +861,6 @@ onesweep_histogram(const uint64_t* __restrict__ key0, const uint64_t* __restrict
         const uint32_t v = (&h[0][0])[k];
         if (v) atomicAdd(hist + k, v);
     }
-}
-
-// Lanes holding the same 8-bit digit, from eight ballots (the ballot path
-// keeps this off the pipe that serialises __match_any_sync).
-__device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid) {
-    unsigned peers = __ballot_sync(kFull, valid);
-    if (!valid) peers = 0;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const bool bit = (d >> b) & 1u;
-        const unsigned m = __ballot_sync(kFull, bit);
-        peers &= bit ? m : ~m;
-    }
-    return valid ? peers : (1u << (threadIdx.x & 31));
-}
-
-// Exclusive scan of each digit position's 256 bins (block d = position d).
-__global__ void __launch_bounds__(kSortThreads)
-onesweep_bins(uint32_t* __restrict__ hist) {
-    chain_begin();
-    __shared__ uint32_t warp_tot[kWarps];
-    uint32_t* row = hist + 256 * blockIdx.x;
-    const uint32_t v = row[threadIdx.x];
-    const uint32_t ex = block_exclusive_scan(v, warp_tot, nullptr);
-    row[threadIdx.x] = ex;
 }
 
 __device__ __forceinline__ uint32_t ld_status(const uint32_t* p) {
@@ -641,12 +925,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar) {
 __global__ void __launch_bounds__(kSortThreads, 4)
 onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ val_in,
               uint64_t* __restrict__ key_out, uint32_t* __restrict__ val_out, int64_t n, int shift,
-              const uint32_t* __restrict__ bins, uint32_t* __restrict__ status,
+              const uint32_t* __restrict__ hist, uint32_t* __restrict__ status,
               unsigned* __restrict__ tile_counter, unsigned* __restrict__ err,
               const int32_t* __restrict__ passes) {
     chain_begin();
     if (passes && shift < 64 - 8 * *passes) return;
-    __shared__ uint32_t whist[kWarps][256];
+    __shared__ uint16_t whist[kWarps][256];
     __shared__ uint32_t tile_start[256];
     __shared__ uint32_t goff[256];
     __shared__ uint32_t warp_tot[kWarps];
@@ -699,18 +983,17 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
         const bool valid = li < tile_n;
         k_reg[k] = valid ? skey[li] : 0ull;
         v_reg[k] = valid ? sval[li] : 0u;
-        const uint32_t d = (uint32_t)((k_reg[k] >> shift) & 0xFF);
-        const unsigned peers = digit_peers(d, valid);
-        const int leader = __ffs(peers) - 1;
-        uint32_t b = 0;
-        if (valid && lane == leader) {
-            b = whist[warp][d];
-            whist[warp][d] = b + __popc(peers);
-        }
-        b = __shfl_sync(kFull, b, leader);
-        r_reg[k] = b + __popc(peers & below);
-        __syncwarp();
     }
+    __syncthreads();
+    // the rows' match words take the values' place until the tile is scattered
+    uint32_t* match = sval + warp * 256;
+#pragma unroll
+    for (int k = lane; k < 256; k += 32) match[k] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < kSortTileItems; ++k)
+        r_reg[k] = row_rank(match, whist[warp], (uint32_t)(k_reg[k] >> shift) & 255u,
+                            seg + k * 32 + lane < tile_n, below);
     __syncthreads();
     uint32_t count;
     {
@@ -718,12 +1001,14 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) {
             const uint32_t c = whist[w][tid];
-            whist[w][tid] = run;
+            whist[w][tid] = (uint16_t)run;
             run += c;
         }
         count = run;
         tile_start[tid] = block_exclusive_scan(run, warp_tot, nullptr);
     }
+    // first place of digit tid in the output
+    const uint32_t bin = block_exclusive_scan(hist[tid], warp_tot, nullptr);
     // look-back for digit tid
     uint32_t* st = status + (int64_t)tile * 256 + tid;
     uint32_t excl = 0;
@@ -731,23 +1016,31 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
         st_status(st, kFlagPrefix | count);
     } else {
         st_status(st, kFlagAgg | count);
-        for (int j = tile - 1; j >= 0; --j) {
-            const uint32_t* pj = status + (int64_t)j * 256 + tid;
-            uint32_t v = ld_status(pj);
-            int spins = 0;
-            while ((v & ~kCountMask) == 0) {
-                if (++spins > kSpinLimit) {
-                    atomicOr(err, kErrTimeout);
-                    break;
+        // kLook predecessors' words in flight: when all tiles start together,
+        // a tile meets no inclusive prefix for many tiles back
+        bool found = false;
+        for (int j = tile - 1; j >= 0 && !found; j -= kLook) {
+            uint32_t v[kLook];
+#pragma unroll
+            for (int q = 0; q < kLook; ++q)
+                v[q] = j - q >= 0 ? ld_status(status + (int64_t)(j - q) * 256 + tid) : kFlagPrefix;
+#pragma unroll
+            for (int q = 0; q < kLook; ++q) {
+                if (found) continue;
+                for (int spins = 0; (v[q] & ~kCountMask) == 0;) {
+                    if (++spins > kSpinLimit) {
+                        atomicOr(err, kErrTimeout);
+                        break;
+                    }
+                    v[q] = ld_status(status + (int64_t)(j - q) * 256 + tid);
                 }
-                v = ld_status(pj);
+                excl += v[q] & kCountMask;
+                found = (v[q] & ~kCountMask) == kFlagPrefix;
             }
-            excl += v & kCountMask;
-            if ((v & ~kCountMask) == kFlagPrefix) break;
         }
         st_status(st, kFlagPrefix | (excl + count));
     }
-    goff[tid] = bins[tid] + excl;
+    goff[tid] = bin + excl;
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kSortTileItems; ++k) {
@@ -830,19 +1123,28 @@ tie_mark(const uint64_t* __restrict__ key, int64_t n, DeviceScalars* __restrict_
 // Groups of 2..32 keys: lane l holds key l of the group and counts the keys
 // that go before it (smaller, or equal and earlier).  The keys share their top
 // bytes, so comparing whole keys compares the low bytes.
-__global__ void __launch_bounds__(256)
-tie_sort_small(uint64_t* __restrict__ key, uint32_t* __restrict__ val,
-               const uint2* __restrict__ small, const DeviceScalars* __restrict__ s) {
+// Groups of more than 32 keys (rare: many bodies within 2^-4P of the box
+// width of each other): one warp per group, a stable LSD radix sort of the
+// 8 - P low bytes, 32 keys at a time, between the group's range of the
+// sorted buffers and the same range of the free ping-pong buffers.
+constexpr int kTieWarps = 4;
+
+__global__ void __launch_bounds__(kTieWarps * 32)
+tie_sort(uint64_t* __restrict__ key0, uint32_t* __restrict__ val0, uint64_t* __restrict__ key1,
+         uint32_t* __restrict__ val1, const uint2* __restrict__ small, const uint2* __restrict__ big,
+         const DeviceScalars* __restrict__ s) {
     chain_begin();
-    if (s->sort_passes >= 8) return;
-    const unsigned count = s->tie_count[0];
-    const int lane = threadIdx.x & 31;
-    const unsigned warps = gridDim.x * (blockDim.x >> 5);
-    for (unsigned g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < count; g += warps) {
+    const int passes = s->sort_passes;
+    if (passes >= 8) return;
+    __shared__ uint32_t off[kTieWarps][256];
+    const unsigned nsmall = s->tie_count[0], nbig = s->tie_count[1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned warps = gridDim.x * kTieWarps, me = blockIdx.x * kTieWarps + w;
+    for (unsigned g = me; g < nsmall; g += warps) {
         const uint2 grp = small[g];
         const bool on = lane < (int)grp.y;
-        const uint64_t k = on ? key[grp.x + lane] : ~0ull;
-        const uint32_t v = on ? val[grp.x + lane] : 0u;
+        const uint64_t k = on ? key0[grp.x + lane] : ~0ull;
+        const uint32_t v = on ? val0[grp.x + lane] : 0u;
         int rank = 0;
         for (int j = 0; j < (int)grp.y; ++j) {
             const uint64_t kj = __shfl_sync(kFull, k, j);
@@ -850,28 +1152,12 @@ tie_sort_small(uint64_t* __restrict__ key, uint32_t* __restrict__ val,
         }
         __syncwarp();
         if (on) {
-            key[grp.x + rank] = k;
-            val[grp.x + rank] = v;
+            key0[grp.x + rank] = k;
+            val0[grp.x + rank] = v;
         }
     }
-}
-
-// Groups of more than 32 keys (rare: many bodies within 2^-4P of the box
-// width of each other): one warp per group, a stable LSD radix sort of the
-// 8 - P low bytes, 32 keys at a time, between the group's range of the
-// sorted buffers and the same range of the free ping-pong buffers.
-__global__ void __launch_bounds__(128)
-tie_sort_big(uint64_t* __restrict__ key0, uint32_t* __restrict__ val0, uint64_t* __restrict__ key1,
-             uint32_t* __restrict__ val1, const uint2* __restrict__ big,
-             const DeviceScalars* __restrict__ s) {
-    chain_begin();
-    const int passes = s->sort_passes;
-    if (passes >= 8) return;
-    __shared__ uint32_t off[4][256];
-    const unsigned count = s->tie_count[1];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned below = lanemask_lt();
-    for (unsigned g = blockIdx.x * 4 + w; g < count; g += gridDim.x * 4) {
+    for (unsigned g = me; g < nbig; g += warps) {
         const uint2 grp = big[g];
         const unsigned first = grp.x, size = grp.y;
         for (int d = 0; d < 8 - passes; ++d) {
@@ -967,21 +1253,87 @@ inline unsigned blocks_for(int64_t n, int threads) {
 
 }  // namespace
 
+namespace {
+
+// Launches cluster_sort over n keys with kItems keys per thread.
+template <int kItems, int kSrc>
+cudaError_t launch_cluster(cudaStream_t st, bool chained, int blocks, int cluster, const double2* pos,
+                           int64_t n, DeviceScalars* s, int adaptive, int new_step, int fixed_passes,
+                           const uint64_t* key_in, uint64_t* key_out, uint32_t* val_out,
+                           unsigned long long* mark0, unsigned long long* mark1) {
+    auto* kernel = cluster_sort<kItems, kSrc>;
+    const size_t smem = sizeof(ClusterSmem<kItems>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    return chain_launch(st, chained, kernel, blocks, kClusterThreads, smem, cluster, pos, n, s, adaptive,
+                        new_step, fixed_passes, key_in, key_out, val_out, mark0, mark1);
+}
+
+// As few keys per thread as one cluster allows (a pass ranks them one after
+// the other), then as few blocks as hold them.
+template <int kSrc>
+cudaError_t launch_cluster_sort(cudaStream_t st, bool chained, const double2* pos, int64_t n,
+                                DeviceScalars* s, int adaptive, int new_step, int fixed_passes,
+                                const uint64_t* key_in, uint64_t* key_out, uint32_t* val_out,
+                                unsigned long long* mark0, unsigned long long* mark1) {
+    const int items = n <= (int64_t)kClusterMost * kClusterThreads ? 1 : 2;
+    const int tiles = (int)((n + items * kClusterThreads - 1) / (items * kClusterThreads));
+    int cluster = 1;
+    while (cluster < tiles) cluster *= 2;
+    auto* launch = items == 1 ? launch_cluster<1, kSrc> : launch_cluster<2, kSrc>;
+    return launch(st, chained, cluster, cluster, pos, n, s, adaptive, new_step, fixed_passes, key_in,
+                  key_out, val_out, mark0, mark1);
+}
+
+inline bool by_cluster(const nb_ctx* c) { return c->sort.hist == nullptr; }
+
+}  // namespace
+
+// The largest clusters that the sort launches must fit the device.
+int64_t cluster_sort_size() {
+    auto* kernel = cluster_sort<2, kSrcBodies>;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kClusterMost;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = kClusterMost;
+    cfg.blockDim = kClusterThreads;
+    cfg.dynamicSmemBytes = sizeof(ClusterSmem<2>);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess)
+        clusters = 0;
+    return clusters > 0 ? kClusterSortMax : 0;
+}
+
 void launch_bbox(nb_ctx* c, const double2* pos, bool new_step) {
     if (c->batch.nuni > 0) {
         c->launches += 2;
-        chain_launch(c->stream, false, bbox_batch_kernel, 2 * c->sm_count * 8, 256, 0, pos, c->n,
+        chain_launch(c->stream, false, bbox_batch_kernel, 2 * c->sm_count * 8, 256, 0, 1, pos, c->n,
                      c->batch, mark_of(c, 0));
-        chain_launch(c->stream, true, bbox_batch_finish, blocks_for(c->batch.nuni, 128), 128, 0,
+        chain_launch(c->stream, true, bbox_batch_finish, blocks_for(c->batch.nuni, 128), 128, 0, 1,
                      c->batch, c->scal, c->n, new_step);
         return;
     }
     c->launches += 1;
-    chain_launch(c->stream, false, bbox_kernel, c->bbox_blocks, kBoxThreads, 0, pos, c->n,
+    if (by_cluster(c)) {  // the whole stage
+        launch_cluster_sort<kSrcBodies>(c->stream, false, pos, c->n, c->scal, 1, new_step, 0, nullptr,
+                                        c->sort.key[0], c->sort.val[0], mark_of(c, 0), mark_of(c, 1));
+        return;
+    }
+    chain_launch(c->stream, false, bbox_kernel, c->bbox_blocks, kBoxThreads, 0, 1, pos, c->n,
                  c->bbox_partials, c->scal, 1, new_step, mark_of(c, 0));
 }
 
 void launch_morton(nb_ctx* c, const double2* pos) {
+    if (by_cluster(c) && c->batch.nuni == 0) return;  // launch_bbox has made the codes
     c->launches += 1;
     SortState z;
     z.hist = c->sort.hist;
@@ -989,12 +1341,12 @@ void launch_morton(nb_ctx* c, const double2* pos) {
     z.status = c->sort.status;
     z.tiles = c->sort.tiles;
     if (c->batch.nuni > 0) {
-        chain_launch(c->stream, true, morton_batch_kernel, blocks_for(c->n, 256), 256, 0, pos, c->n,
+        chain_launch(c->stream, true, morton_batch_kernel, blocks_for(c->n, 256), 256, 0, 1, pos, c->n,
                      c->batch, c->scal, c->sort.key[0], c->sort.key[1], c->sort.val[0],
                      c->sort.val[1], z);
         return;
     }
-    chain_launch(c->stream, true, morton_kernel, blocks_for(c->n, 256), 256, 0, pos, c->n, c->scal,
+    chain_launch(c->stream, true, morton_kernel, blocks_for(c->n, 256), 256, 0, 1, pos, c->n, c->scal,
                  c->sort.key[0], c->sort.key[1], c->sort.val[0], c->sort.val[1], z);
 }
 
@@ -1039,53 +1391,68 @@ unsigned sort_timeout_probe(cudaStream_t st) {
     return flags;
 }
 
-// The Morton pass has reset the histograms, tile counters and status words.
+// The sorted keys and permutation end in buffer 0.
 void launch_sort(nb_ctx* c) {
-    const int tiles = c->sort.tiles;
-    c->launches += 2 + 8 + 3;
-    chain_launch(c->stream, true, onesweep_histogram, 4 * c->sm_count, kSortThreads, 0,
-                 c->sort.key[0], c->sort.key[1], c->n, c->scal, c->sort.hist, mark_of(c, 1));
-    chain_launch(c->stream, true, onesweep_bins, 8, kSortThreads, 0, c->sort.hist);
-    for (int pass = 0; pass < 8; ++pass) {
-        const int src = pass & 1, dst = src ^ 1;
-        chain_launch(c->stream, true, onesweep_pass, tiles, kSortThreads, 0, c->sort.key[src],
-                     c->sort.val[src], c->sort.key[dst], c->sort.val[dst], c->n, 8 * pass,
-                     c->sort.hist + 256 * pass, c->sort.status + (size_t)pass * 256 * tiles,
-                     c->sort.tile_counter + pass, &c->scal->error, &c->scal->sort_passes);
+    uint64_t* const* key = c->sort.key;
+    uint32_t* const* val = c->sort.val;
+    c->launches += 2;
+    if (by_cluster(c)) {
+        if (c->batch.nuni > 0) {  // (otherwise launch_bbox has done it)
+            c->launches += 1;
+            launch_cluster_sort<kSrcKeys>(c->stream, true, nullptr, c->n, c->scal, 1, 0, 0, key[0],
+                                          key[0], val[0], mark_of(c, 1), nullptr);
+        }
+    } else {
+        // the Morton pass has reset the histograms, tile counters and status words
+        const int tiles = c->sort.tiles;
+        c->launches += 1 + 8;
+        chain_launch(c->stream, true, onesweep_histogram,
+                     std::min<unsigned>(4 * c->sm_count, blocks_for(c->n, 32 * kHistRows * kWarps)),
+                     kSortThreads, 0, 1, key[0], key[1], c->n, c->scal, c->sort.hist, mark_of(c, 1));
+        for (int pass = 0; pass < 8; ++pass) {
+            const int src = pass & 1, dst = src ^ 1;
+            chain_launch(c->stream, true, onesweep_pass, tiles, kSortThreads, 0, 1, key[src], val[src],
+                         key[dst], val[dst], c->n, 8 * pass, c->sort.hist + 256 * pass,
+                         c->sort.status + (size_t)pass * 256 * tiles, c->sort.tile_counter + pass,
+                         &c->scal->error, &c->scal->sort_passes);
+        }
     }
     // keys tied in the sorted top bytes, in order of their low bytes
-    chain_launch(c->stream, true, tie_mark, blocks_for(c->n, 256), 256, 0, c->sort.key[0], c->n,
-                 c->scal, c->sort.ties_small, c->sort.ties_big);
-    chain_launch(c->stream, true, tie_sort_small, c->sm_count * 8, 256, 0, c->sort.key[0],
-                 c->sort.val[0], c->sort.ties_small, c->scal);
-    chain_launch(c->stream, true, tie_sort_big, c->sm_count, 128, 0, c->sort.key[0], c->sort.val[0],
-                 c->sort.key[1], c->sort.val[1], c->sort.ties_big, c->scal);
+    chain_launch(c->stream, true, tie_mark, blocks_for(c->n, 256), 256, 0, 1, key[0], c->n, c->scal,
+                 c->sort.ties_small, c->sort.ties_big);
+    chain_launch(c->stream, true, tie_sort, std::min<unsigned>(c->sm_count * 16, blocks_for(c->n, 256)),
+                 kTieWarps * 32, 0, 1, key[0], val[0], key[1], val[1], c->sort.ties_small,
+                 c->sort.ties_big, c->scal);
 }
 
-void launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* const key[2],
-                            uint32_t* const val[2], uint64_t* key_out, uint32_t* val_out,
-                            uint32_t* counts, uint32_t* totals, double* partials, int bbox_blocks,
-                            DeviceScalars* scal, cudaStream_t st) {
-    const int tiles = (int)((n + kSortTile - 1) / kSortTile);
-    bbox_kernel<<<bbox_blocks, kBoxThreads, 0, st>>>(pos, n, partials, scal, 0, 0,
-                                                      nullptr);  // all 8 passes
-    morton_kernel<<<blocks_for(n, 256), 256, 0, st>>>(pos, n, scal, key[0], key[1], val[0], val[1],
-                                                    SortState());
-    for (int pass = 0; pass < 8; ++pass) {
+// All 8 passes, so no ties are left.
+cudaError_t launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* const key[2],
+                                   uint32_t* const val[2], uint64_t* key_out, uint32_t* val_out,
+                                   uint16_t* counts, double* partials, int bbox_blocks,
+                                   DeviceScalars* scal, cudaStream_t st) {
+    if (n <= cluster_sort_size())
+        return launch_cluster_sort<kSrcBodies>(st, false, pos, n, scal, 0, 0, 8, nullptr, key_out,
+                                               val_out, nullptr, nullptr);
+    const int tiles = (int)count_tiles(n);
+    cudaError_t e = chain_launch(st, false, bbox_kernel, bbox_blocks, kBoxThreads, 0, 1, pos, n,
+                                 partials, scal, 0, 0, nullptr);
+    if (e == cudaSuccess)
+        e = chain_launch(st, true, morton_kernel, blocks_for(n, 256), 256, 0, 1, pos, n, scal, key[0],
+                         key[1], val[0], val[1], SortState());
+    for (int pass = 0; pass < 8 && e == cudaSuccess; ++pass) {
         const int src = pass & 1, dst = src ^ 1;
-        const int shift = 8 * pass;
-        uint64_t* kd = pass == 7 ? key_out : key[dst];
-        uint32_t* vd = pass == 7 ? val_out : val[dst];
-        sort_upsweep<<<tiles, kSortThreads, 0, st>>>(key[src], n, shift, counts, tiles);
-        sort_scan_rows<<<256, kSortThreads, 0, st>>>(counts, tiles, totals);
-        sort_downsweep<<<tiles, kSortThreads, 0, st>>>(key[src], val[src], kd, vd, n, shift, counts,
-                                                       totals, tiles);
+        e = chain_launch(st, true, count_digits, tiles, kCountThreads, 0, 1, key[src], n, pass, counts);
+        if (e == cudaSuccess)
+            e = chain_launch(st, true, count_scatter, tiles, kCountThreads, 0, 1, key[src], val[src],
+                             pass == 7 ? key_out : key[dst], pass == 7 ? val_out : val[dst], n, pass,
+                             counts, tiles);
     }
+    return e;
 }
 
 void launch_gather(nb_ctx* c, const BodyBuffers& src, const BodyBuffers& dst, float4* body4) {
     c->launches += 1;
-    chain_launch(c->stream, true, gather_kernel, blocks_for(c->n, 256), 256, 0, c->sort.val[0], c->n,
+    chain_launch(c->stream, true, gather_kernel, blocks_for(c->n, 256), 256, 0, 1, c->sort.val[0], c->n,
                  src, dst, body4, c->scal, c->batch, mark_of(c, 2));
 }
 

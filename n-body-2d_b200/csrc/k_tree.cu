@@ -1231,7 +1231,7 @@ inline unsigned blocks_for(int64_t n, int threads) {
 void launch_batch_roots(nb_ctx* c) {
     if (c->batch.nuni == 0) return;
     c->launches += 1;
-    chain_launch(c->stream, true, batch_roots, blocks_for(c->batch.nuni, 128), 128, 0,
+    chain_launch(c->stream, true, batch_roots, blocks_for(c->batch.nuni, 128), 128, 0, 1,
                  c->sort.key[0], c->tree, c->batch);
 }
 
@@ -1246,13 +1246,13 @@ void launch_groups(nb_ctx* c, bool chained) {
     // learned correction keeps groups of whole cells, whose residuals it fits.
     // The linking pass counted every cell's groups; scan, then write them.
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
-    chain_launch(c->stream, chained, scan_reduce, sblocks, kThreads, 0, c->tree.gcount, n,
+    chain_launch(c->stream, chained, scan_reduce, sblocks, kThreads, 0, 1, c->tree.gcount, n,
                  c->scan.block_sums, mark_of(c, 6));
-    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, c->scan.block_sums, sblocks,
+    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, 1, c->scan.block_sums, sblocks,
                  &c->scal->groups);
-    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, c->tree.gcount, n,
+    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, 1, c->tree.gcount, n,
                  c->scan.block_sums, c->tree.gbase, nullptr);
-    chain_launch(c->stream, true, tree_groups_write, blocks_for(n, kThreads), kThreads, 0, n, gsize,
+    chain_launch(c->stream, true, tree_groups_write, blocks_for(n, kThreads), kThreads, 0, 1, n, gsize,
                  fill, c->tree, c->scal, c->batch, c->sort.key[0]);
 }
 
@@ -1276,11 +1276,11 @@ void launch_prefix_sums(nb_ctx* c, const BodyBuffers& b) {
     {  // the prefix sums need only the sorted bodies
         const int ptiles = (int)blocks_for(n, kScanTile);
         c->launches += 3;
-        chain_launch(c->stream, true, prefix_reduce, ptiles, kThreads, 0, b.pos, b.mass, n, c->scal,
+        chain_launch(c->stream, true, prefix_reduce, ptiles, kThreads, 0, 1, b.pos, b.mass, n, c->scal,
                      c->batch, c->tree.prefix_tiles, mark_of(c, 3));
-        chain_launch(c->stream, true, prefix_tiles_scan, 1, kThreads, 0, c->tree.prefix_tiles,
+        chain_launch(c->stream, true, prefix_tiles_scan, 1, kThreads, 0, 1, c->tree.prefix_tiles,
                      ptiles);
-        chain_launch(c->stream, true, prefix_apply, ptiles, kThreads, 0, b.pos, b.mass, n, c->scal,
+        chain_launch(c->stream, true, prefix_apply, ptiles, kThreads, 0, 1, b.pos, b.mass, n, c->scal,
                      c->batch, c->tree.prefix_tiles, ptiles, c->tree.prefix);
     }
 }
@@ -1293,32 +1293,32 @@ void launch_tree(nb_ctx* c, const BodyBuffers& b, bool prefix_done) {
     Tree& t = c->tree;
     const int tiles = (int)blocks_for(n, kAnsvTile);
     c->launches += 8;
-    chain_launch(c->stream, true, tree_lcp, tiles, kThreads, 0, key, n, tiles, t.lcp8, t.ansv_first,
+    chain_launch(c->stream, true, tree_lcp, tiles, kThreads, 0, 1, key, n, tiles, t.lcp8, t.ansv_first,
                  t.ansv_last, c->scal->lcp_hist, mark_of(c, 4));
-    chain_launch(c->stream, true, tree_ansv_tiles, kAnsvLevels, kTileScanThreads, 0, tiles,
+    chain_launch(c->stream, true, tree_ansv_tiles, kAnsvLevels, kTileScanThreads, 0, 1, tiles,
                  t.ansv_first, t.ansv_last);
-    chain_launch(c->stream, true, tree_ansv, tiles, kThreads, 0, t.lcp8, n, tiles, t.ansv_first,
+    chain_launch(c->stream, true, tree_ansv, tiles, kThreads, 0, 1, t.lcp8, n, tiles, t.ansv_first,
                  t.ansv_last, t.flag, t.bnd);
     const int sblocks = (int)blocks_for(n, kScanTile);
-    chain_launch(c->stream, true, scan_reduce, sblocks, kThreads, 0, t.flag, n, c->scan.block_sums,
+    chain_launch(c->stream, true, scan_reduce, sblocks, kThreads, 0, 1, t.flag, n, c->scan.block_sums,
                  nullptr);
-    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, c->scan.block_sums, sblocks,
+    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, 1, c->scan.block_sums, sblocks,
                  &c->scal->cells);
-    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, t.flag, n, c->scan.block_sums,
+    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, 1, t.flag, n, c->scan.block_sums,
                  t.cell_of, t.rep_of);
     // SPLIT: the cells count their target groups as they link
     const int gsize = c->p.mode == NB_MODE_SPLIT ? split_group_size(c) : 0;
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
     chain_launch(c->stream, true, mono ? tree_link<true> : tree_link<false>, blocks_for(n, kThreads),
-                 kThreads, 0, key, t.lcp8, n, b.pos, b.mass, t, c->scal, mono ? t.prefix : nullptr,
+                 kThreads, 0, 1, key, t.lcp8, n, b.pos, b.mass, t, c->scal, mono ? t.prefix : nullptr,
                  c->batch, mono ? split_accept_scale(c) : 0.f, gsize, fill);
-    chain_launch(c->stream, true, tree_trivial_root, 1, 1, 0, b.pos, b.mass, n, t, c->scal, gsize);
+    chain_launch(c->stream, true, tree_trivial_root, 1, 1, 0, 1, b.pos, b.mass, n, t, c->scal, gsize);
 }
 
 void launch_features(nb_ctx* c, const BodyBuffers& b, bool chained) {
     const int cap = (int)(c->n > 1 ? c->n - 1 : 1);
     c->launches += 1;
-    chain_launch(c->stream, chained, learned_features, blocks_for(cap, kThreads), kThreads, 0, c->scal,
+    chain_launch(c->stream, chained, learned_features, blocks_for(cap, kThreads), kThreads, 0, 1, c->scal,
                  b.pos, b.mass, c->tree, c->batch);
 }
 
@@ -1332,14 +1332,14 @@ void launch_moments(nb_ctx* c, const BodyBuffers& b, bool split) {
     const unsigned blocks = blocks_for(cap, kThreads);
     if (second) {
         c->launches += 1;
-        chain_launch(c->stream, true, tree_moments<true, true>, blocks, kThreads, 0, c->scal, b.pos,
+        chain_launch(c->stream, true, tree_moments<true, true>, blocks, kThreads, 0, 1, c->scal, b.pos,
                      b.mass, c->tree, c->batch, accept_scale, mark_of(c, 5));
     } else if (split) {
         // monopoles: the prefix sums ran before the tree, and the linking
         // pass wrote every cell's record from them
     } else {
         c->launches += 1;
-        chain_launch(c->stream, true, tree_moments<false, false>, blocks, kThreads, 0, c->scal, b.pos,
+        chain_launch(c->stream, true, tree_moments<false, false>, blocks, kThreads, 0, 1, c->scal, b.pos,
                      b.mass, c->tree, c->batch, 0.f, mark_of(c, 5));
     }
 }

@@ -72,11 +72,11 @@ int alloc_all(nb_ctx* c) {
         NB_CUDA(c, dalloc(&c->sort.val[k], n));
     }
     c->sort.tiles = (int)((n + nb::kSortTile - 1) / nb::kSortTile);
-    NB_CUDA(c, dalloc(&c->sort.counts, (size_t)256 * c->sort.tiles));
-    NB_CUDA(c, dalloc(&c->sort.totals, 256));
-    NB_CUDA(c, dalloc(&c->sort.hist, 8 * 256));
-    NB_CUDA(c, dalloc(&c->sort.status, (size_t)8 * 256 * c->sort.tiles));
-    NB_CUDA(c, dalloc(&c->sort.tile_counter, 8));
+    if (c->n > nb::cluster_sort_size()) {  // onesweep passes
+        NB_CUDA(c, dalloc(&c->sort.hist, 8 * 256));
+        NB_CUDA(c, dalloc(&c->sort.status, (size_t)8 * 256 * c->sort.tiles));
+        NB_CUDA(c, dalloc(&c->sort.tile_counter, 8));
+    }
     NB_CUDA(c, dalloc(&c->sort.ties_small, n / 2 + 1));
     NB_CUDA(c, dalloc(&c->sort.ties_big, n / 33 + 1));
     c->scan.blocks = (int)((n + 2047) / 2048);
@@ -130,7 +130,8 @@ int alloc_all(nb_ctx* c) {
     }
     NB_CUDA(c, dalloc(&c->scal, 1));
     NB_CUDA(c, cudaMemset(c->scal, 0, sizeof(nb::DeviceScalars)));
-    c->bbox_blocks = 2 * c->sm_count;
+    // (the last block folds one partial per block: no more blocks than fill)
+    c->bbox_blocks = (int)std::min<size_t>(2 * c->sm_count, (n + 1023) / 1024);
     NB_CUDA(c, dalloc(&c->bbox_partials, (size_t)4 * c->bbox_blocks));
     NB_CUDA(c, dalloc(&c->acc, n));
     NB_CUDA(c, dalloc(&c->stage_pos, n));
@@ -147,8 +148,6 @@ void free_all(nb_ctx* c) {
         cudaFree(c->sort.key[k]);
         cudaFree(c->sort.val[k]);
     }
-    cudaFree(c->sort.counts);
-    cudaFree(c->sort.totals);
     cudaFree(c->sort.hist);
     cudaFree(c->sort.status);
     cudaFree(c->sort.tile_counter);

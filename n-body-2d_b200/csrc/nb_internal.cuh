@@ -149,8 +149,6 @@ struct Tree {
 struct SortBuffers {
     uint64_t* key[2] = {nullptr, nullptr};
     uint32_t* val[2] = {nullptr, nullptr};
-    uint32_t* counts = nullptr;   // [256][tiles]
-    uint32_t* totals = nullptr;   // [256]
     uint32_t* hist = nullptr;     // [8][256] digit histograms -> exclusive bin offsets
     uint32_t* status = nullptr;   // [8][tiles][256] look-back status words
     unsigned* tile_counter = nullptr;  // [8]
@@ -281,48 +279,62 @@ __device__ __forceinline__ double m_over_r3_any(double m, double r2) {
 
 // Number of radix passes (top bytes of the key) a sort should take, from the
 // histogram of shared leading digits of neighbouring sorted codes: the fewest
-// passes that leave at most n / 32 neighbouring pairs tied; 8 without data.
+// passes that leave at most n / 32 neighbouring pairs tied (agreeing in those
+// bytes but not equal); 8 without data.  One warp, all lanes get the answer.
 __device__ __forceinline__ int choose_sort_passes(const unsigned* hist, int64_t n) {
-    unsigned long long total = 0;
-    for (int d = 0; d <= 32; ++d) total += hist[d];
-    if (total == 0) return 8;
-    for (int p = 1; p < 8; ++p) {
-        unsigned long long tied = 0;  // pairs that agree in p bytes but are not equal
-        for (int d = 4 * p; d < 32; ++d) tied += hist[d];
-        if (tied * 32 <= (unsigned long long)n) return p;
+    const int lane = threadIdx.x & 31;
+    const unsigned h = hist[lane], equal = hist[32];
+    if (!__any_sync(0xffffffffu, h != 0 || equal != 0)) return 8;
+    unsigned long long from = h;  // pairs that share `lane` digits or more, below 32
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_down_sync(0xffffffffu, from, o);
+        if (lane + o < 32) from += t;
     }
-    return 8;
+    const bool few = (lane & 3) == 0 && lane >= 4 && from * 32 <= (unsigned long long)n;
+    const unsigned ok = __ballot_sync(0xffffffffu, few);
+    return ok ? (__ffs(ok) - 1) / 4 : 8;
 }
 
 // ---- the step's kernel chain ----------------------------------------------
 // A step is a chain of some 30 kernels, most of them a few microseconds long
 // below a million bodies, so the gaps between them count.  Its kernels are
 // launched with programmatic stream serialization: each begins with
-// chain_begin(), which lets the next kernel's blocks be launched as soon as all
-// blocks of this one run, and then waits until the kernel before has
-// completed and its writes are visible.  Nothing is read or written before
-// that wait, so the order of memory accesses is that of plain launches.
+// chain_begin(), which waits until the kernel before has completed and its
+// writes are visible, and then lets the next kernel's blocks be launched as
+// soon as all blocks of this one have come that far.  Nothing is read or
+// written before that wait, so the order of memory accesses is that of plain
+// launches.
 __device__ __forceinline__ void chain_begin() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // chained = false: an ordinary launch (the first kernel of a step, or one that
-// follows a copy, an event or another stream).
+// follows a copy, an event or another stream).  cluster: blocks per cluster.
 template <typename... Ps, typename... As>
-inline void chain_launch(cudaStream_t st, bool chained, void (*kernel)(Ps...), dim3 grid,
-                         dim3 block, size_t smem, As... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t chain_launch(cudaStream_t st, bool chained, void (*kernel)(Ps...), dim3 grid,
+                                dim3 block, size_t smem, int cluster, As... args) {
+    cudaLaunchAttribute attr[2] = {};
+    unsigned attrs = 0;
+    if (chained) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[attrs].id = cudaLaunchAttributeClusterDimension;
+        attr[attrs].val.clusterDim.x = (unsigned)cluster;
+        attr[attrs].val.clusterDim.y = attr[attrs].val.clusterDim.z = 1;
+        ++attrs;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = chained ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<Ps>(args)...);
+    cfg.attrs = attr;
+    cfg.numAttrs = attrs;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Ps>(args)...);
 }
 
 // Phase times: the first kernel of phase k writes marks[k] (mark_start), the
@@ -396,13 +408,21 @@ void launch_scatter(nb_ctx* c, const BodyBuffers& b, double2* out_pos, double2* 
                     const double2* acc, double2* out_acc);
 void launch_identity(nb_ctx* c, int32_t* orig);
 
+// Up to kClusterSortMax bodies are sorted by one cluster of blocks that holds
+// all keys in shared memory; cluster_sort_size() is the most that this device
+// sorts so (0 where it cannot run such a cluster).
+constexpr int64_t kClusterSortMax = 32768;
+int64_t cluster_sort_size();
+
 // The bounding-box, Morton and radix-sort stage on caller-provided buffers
 // (no context): key/val ping-pong scratch of n entries each, counts of
-// 256 x ceil(n / kSortTile), totals of 256, partials of 4 x bbox_blocks.  The
-// last pass writes the sorted codes and permutation to key_out / val_out.
-void launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* const key[2],
-                            uint32_t* const val[2], uint64_t* key_out, uint32_t* val_out,
-                            uint32_t* counts, uint32_t* totals, double* partials, int bbox_blocks,
-                            DeviceScalars* scal, cudaStream_t st);
+// [count_tiles(n)][256], partials of 4 x bbox_blocks.  The sorted codes and
+// permutation go to key_out and val_out.
+constexpr int kCountTile = 2048;
+inline int64_t count_tiles(int64_t n) { return (n + kCountTile - 1) / kCountTile; }
+cudaError_t launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* const key[2],
+                                   uint32_t* const val[2], uint64_t* key_out, uint32_t* val_out,
+                                   uint16_t* counts, double* partials, int bbox_blocks,
+                                   DeviceScalars* scal, cudaStream_t st);
 
 }  // namespace nb

@@ -24,7 +24,7 @@
 namespace {
 
 constexpr int64_t kMaxBodies = NB_STATIC_SORT_MAX_BODIES;
-constexpr int kMaxTiles = (int)((kMaxBodies + nb::kSortTile - 1) / nb::kSortTile);
+constexpr int kMaxTiles = (int)((kMaxBodies + nb::kCountTile - 1) / nb::kCountTile);
 constexpr int kBoxBlocks = 256;
 
 // Scratch layout (all offsets multiples of 256 bytes).
@@ -35,15 +35,13 @@ constexpr size_t kOffKey1 = kOffKey0 + kKeyBytes;
 constexpr size_t kOffVal0 = kOffKey1 + kKeyBytes;
 constexpr size_t kOffVal1 = kOffVal0 + kValBytes;
 constexpr size_t kOffCounts = kOffVal1 + kValBytes;
-constexpr size_t kOffTotals = kOffCounts + sizeof(uint32_t) * 256 * kMaxTiles;
-constexpr size_t kOffPartials = kOffTotals + sizeof(uint32_t) * 256;
+constexpr size_t kOffPartials = kOffCounts + sizeof(uint16_t) * 256 * kMaxTiles;
 constexpr size_t kOffScalars = kOffPartials + sizeof(double) * 4 * kBoxBlocks;
 constexpr size_t kScratchBytes = kOffScalars + ((sizeof(nb::DeviceScalars) + 255) / 256) * 256;
 static_assert(kScratchBytes - kOffCounts < 100 * 1024 && kScratchBytes < 6400 * 1000,
-              "the documented size of the scratch array (6.4 MB, ~100 KB beyond the keys) is stale");
+              "the documented size of the scratch array (6.4 MB, up to 100 KB beyond the keys) is stale");
 static_assert(kOffKey1 % 256 == 0 && kOffVal0 % 256 == 0 && kOffVal1 % 256 == 0 &&
-                  kOffCounts % 256 == 0 && kOffTotals % 256 == 0 && kOffPartials % 256 == 0 &&
-                  kOffScalars % 256 == 0,
+                  kOffCounts % 256 == 0 && kOffPartials % 256 == 0 && kOffScalars % 256 == 0,
               "scratch regions must stay 256-byte aligned");
 
 static __device__ __align__(256) unsigned char g_sort_scratch[kScratchBytes];
@@ -81,12 +79,13 @@ extern "C" int nb_morton_sort_static(const double* pos_xy, uint64_t n, uint64_t*
     // reduction's block counter must start at zero.
     if (cudaMemsetAsync(&scal->bbox_ticket, 0, sizeof(unsigned), st) != cudaSuccess)
         return NB_ERR_CUDA;
-    nb::launch_morton_sort_raw(reinterpret_cast<const double2*>(pos_xy), (int64_t)n, key, val,
-                               codes, reinterpret_cast<uint32_t*>(order),
-                               reinterpret_cast<uint32_t*>(base + kOffCounts),
-                               reinterpret_cast<uint32_t*>(base + kOffTotals),
-                               reinterpret_cast<double*>(base + kOffPartials), kBoxBlocks, scal, st);
-    if (cudaGetLastError() != cudaSuccess) return NB_ERR_CUDA;
+    if (nb::launch_morton_sort_raw(reinterpret_cast<const double2*>(pos_xy), (int64_t)n,
+                                   key, val, codes,
+                                   reinterpret_cast<uint32_t*>(order),
+                                   reinterpret_cast<uint16_t*>(base + kOffCounts),
+                                   reinterpret_cast<double*>(base + kOffPartials), kBoxBlocks, scal,
+                                   st) != cudaSuccess)
+        return NB_ERR_CUDA;
     if (box && cudaMemcpyAsync(box, scal->box, 4 * sizeof(double), cudaMemcpyDeviceToDevice, st) !=
                    cudaSuccess)
         return NB_ERR_CUDA;
