@@ -50,7 +50,6 @@ __device__ __forceinline__ void start_sort(DeviceScalars* s, int passes, int new
     s->lcp_hist[32] = 0;
     s->tie_count[0] = 0;
     s->tie_count[1] = 0;
-    s->nstart = 0;
     s->group_ticket = 0;
     if (new_step) {
         s->cell_terms = 0;

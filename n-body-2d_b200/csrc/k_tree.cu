@@ -553,18 +553,6 @@ tree_link(const uint64_t* __restrict__ key, const uint8_t* __restrict__ lcp8, in
     t.nint[id] = nint;
     t.ready[id] = 0;
     if (kMono) cell_from_prefix(prefix, t, s, bt, pos, id, make_int2(first, last), c, accept_scale);
-    // cells whose children are all leaves start the bottom-up climb: listed
-    // with one atomic per warp
-    const unsigned active = __activemask();
-    const unsigned starts = __ballot_sync(active, nint == 0);
-    if (nint == 0) {
-        const int leader = __ffs(starts) - 1;
-        const int lane = threadIdx.x & 31;
-        int base = 0;
-        if (lane == leader) base = atomicAdd(&s->nstart, __popc(starts));
-        base = __shfl_sync(starts, base, leader);
-        t.start_list[base + __popc(starts & ((1u << lane) - 1u))] = id;
-    }
     if (first == 0 && last == n - 1) {
         s->root = id;
         t.parent[id] = -1;
@@ -601,15 +589,6 @@ __global__ void tree_trivial_root(const double2* __restrict__ pos, const double*
     if (n > 1) bucket_moments(pos, mass, 0, n - 1, t.bucket_mass, t.bucket_com);
 }
 
-// Moments of one cell from its children, in quadrant order, with the
-// reference's arithmetic (CU:329-343): M += m; R = fma(m, com, R); com = R / M.
-// kSplit packs the FP32 records the group traversal reads.  kSecond (the
-// quadrupole walk) also accumulates second moments
-// about the COM by the parallel-axis rule, S = sum_c [S_c + m_c d_c d_c^T]
-// with d_c = com_c - com, in FP64.  Leaves have S = 0 (a multi-body leaf
-// spans less than width / 2^30, so its own S is negligible).
-// Children are read with L2-coherent loads: other threads of this launch
-// wrote them, published by the arrival counter's release/acquire.
 // b_max^2 of a cell: squared distance from its COM to the farthest corner of
 // its square.  The square is the cell's Morton prefix decoded in the box the
 // codes were made in (the single box, or the cell's universe); forest cells
@@ -667,78 +646,73 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <bool kSplit, bool kSecond>
-__device__ __forceinline__ void cell_moments(int id, const DeviceScalars* __restrict__ s,
-                                             const double2* __restrict__ pos,
-                                             const double* __restrict__ mass, const Tree& t,
-                                             const Batch& bt, float accept_scale) {
-    const int4 ch = t.child[id];
-    const int refs[4] = {ch.x, ch.y, ch.z, ch.w};
-    double cm[4], cmx[4], cmy[4];
-    double M = 0.0, Rx = 0.0, Ry = 0.0;
+// Mass, COM and (kSecond) second moments of a cell.
+struct Moments {
+    double m, x, y, sxx, sxy, syy;
+};
+
+// Moments of one cell from its children's masses and COMs c, in quadrant order
+// with the reference's arithmetic (CU:329-343): M += m; R = fma(m, com, R);
+// com = R / M (a missing child has mass 0 and changes nothing).  kSecond (the
+// quadrupole walk) also accumulates second moments about the COM by the
+// parallel-axis rule, S = sum_c [S_c + m_c d_c d_c^T] with d_c = com_c - com, in
+// FP64; second(q) is child q's {Sxx, Sxy, Syy}.  Leaves have S = 0 (a
+// multi-body leaf spans less than width / 2^30, so its own S is negligible).
+template <bool kSecond, typename Second>
+__device__ __forceinline__ Moments combine_children(const double3 (&c)[4], Second second) {
+    double M = c[0].x, Rx = c[0].x * c[0].y, Ry = c[0].x * c[0].z;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int r = refs[q];
-        cm[q] = 0.0;
-        cmx[q] = 0.0;
-        cmy[q] = 0.0;
-        if (r == INT_MIN) continue;
-        double2 cc;
-        if (r >= 0) {
-            cm[q] = __ldcg(t.mass + r);
-            cc = __ldcg(t.com + r);
-        } else {
-            const int b = ~r;
-            if (t.leaf_last[b] == b) {
-                cm[q] = mass[b];
-                cc = pos[b];
-            } else {
-                cm[q] = t.bucket_mass[b];
-                cc = t.bucket_com[b];
-            }
-        }
-        cmx[q] = cc.x;
-        cmy[q] = cc.y;
-        M += cm[q];
-        Rx = fma(cm[q], cc.x, Rx);
-        Ry = fma(cm[q], cc.y, Ry);
+    for (int q = 1; q < 4; ++q) {
+        M += c[q].x;
+        Rx = fma(c[q].x, c[q].y, Rx);
+        Ry = fma(c[q].x, c[q].z, Ry);
     }
-    const double2 com = make_double2(Rx / M, Ry / M);
-    __stcg(t.mass + id, M);
-    __stcg(t.com + id, com);
-    if (kSplit && !kSecond) {
-        const int first = t.range[id].x;
-        const double2 fc = frame_center(s, bt, first);
-        t.cell4[id] = make_float4((float)(com.x - fc.x), (float)(com.y - fc.y), (float)M,
-                                  accept_size2(s, bt, pos, first, t.level[id], com, accept_scale));
-    }
-    if (kSplit && kSecond) {
-        double sxx = 0.0, sxy = 0.0, syy = 0.0;
+    Moments o{M, Rx / M, Ry / M, 0.0, 0.0, 0.0};
+    if (kSecond) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int r = refs[q];
-            if (r == INT_MIN) continue;
-            if (r >= 0) {
-                const double2* sc = reinterpret_cast<const double2*>(t.s64 + r);
-                const double2 s01 = __ldcg(sc), s2 = __ldcg(sc + 1);
-                sxx += s01.x;
-                sxy += s01.y;
-                syy += s2.x;
-            }
-            const double dx = cmx[q] - com.x, dy = cmy[q] - com.y;
-            sxx += cm[q] * dx * dx;
-            sxy += cm[q] * dx * dy;
-            syy += cm[q] * dy * dy;
+            const double3 v = second(q);
+            o.sxx += v.x;
+            o.sxy += v.y;
+            o.syy += v.z;
+            const double dx = c[q].y - o.x, dy = c[q].z - o.y;
+            o.sxx += c[q].x * dx * dx;
+            o.sxy += c[q].x * dx * dy;
+            o.syy += c[q].x * dy * dy;
         }
+    }
+    return o;
+}
+
+__device__ __forceinline__ double3 bucket_leaf(const Tree& t, int b) {
+    const double2 p = t.bucket_com[b];
+    return make_double3(t.bucket_mass[b], p.x, p.y);
+}
+
+// A cell's moments as its parent and the walks read them; the second moments
+// themselves only where a parent will read them from memory (`up`).
+template <bool kSplit, bool kSecond>
+__device__ __forceinline__ void store_moments(int id, const Moments& o, bool up,
+                                              const DeviceScalars* __restrict__ s,
+                                              const double2* __restrict__ pos, const Tree& t,
+                                              const Batch& bt, float accept_scale) {
+    const double2 com = make_double2(o.x, o.y);
+    __stcg(t.mass + id, o.m);
+    __stcg(t.com + id, com);
+    if (kSecond && up) {
         double2* so = reinterpret_cast<double2*>(t.s64 + id);
-        __stcg(so, make_double2(sxx, sxy));
-        __stcg(so + 1, make_double2(syy, 0.0));
+        __stcg(so, make_double2(o.sxx, o.sxy));
+        __stcg(so + 1, make_double2(o.syy, 0.0));
+    }
+    if (kSplit) {
         const int first = t.range[id].x;
         const double2 fc = frame_center(s, bt, first);
-        t.cell4[id] = make_float4((float)(com.x - fc.x), (float)(com.y - fc.y), (float)M,
+        t.cell4[id] = make_float4((float)(com.x - fc.x), (float)(com.y - fc.y), (float)o.m,
                                   accept_size2(s, bt, pos, first, t.level[id], com, accept_scale));
         // the walk's record carries 7.5 S, the factor of its (d.S.d) r^-7 term
-        t.cellq[id] = make_float4((float)(7.5 * sxx), (float)(7.5 * sxy), (float)(7.5 * syy), 0.f);
+        if (kSecond)
+            t.cellq[id] =
+                make_float4((float)(7.5 * o.sxx), (float)(7.5 * o.sxy), (float)(7.5 * o.syy), 0.f);
     }
 }
 
@@ -753,36 +727,183 @@ __device__ __forceinline__ int arrive_acq_rel(int* counter) {
     return old;
 }
 
-// Bottom-up pass: threads start at cells without internal children and
-// climb; the last child to arrive at a parent (atomic counter) computes it.
+// Bottom-up pass, one block per kMomentBodies bodies.  Cells are numbered in
+// body order, so the cells whose first separator lies in the block's bodies
+// are one range of ids, and those whose bodies all do (some 99%) form whole
+// subtrees, which the block computes in shared memory.  Cells that reach beyond
+// the block are left to a climb over global memory: the last child to arrive
+// at a parent goes on with it, some 2 us a step, where a publication and three
+// dependent loads follow one another.  With that climb for all cells the pass
+// took 37 us at 1,001 bodies, 51 at 16,384, 99 at 1,048,576 (quadrupoles 173);
+// now 14, 27, 66 and 130.  A round is a chain of FP64 latencies (0.5 us), so
+// larger blocks of bodies gain while the rounds grow with the depth only (512
+// bodies: 22, 26, 78 and 151 us).
+constexpr int kMomentBodies = 1024;
+constexpr int kMomentThreads = 256;
+constexpr int kOutside = -1;
+
+// Node j of a block: its cell j, or with kMomentBodies more the leaf that starts
+// at its body j; the last node is the missing child.
+constexpr int kMomentNodes = 2 * kMomentBodies + 1;
+
+template <bool kSecond>
+struct MomentSmem {
+    double m[kMomentNodes], x[kMomentNodes], y[kMomentNodes];
+    double s[kSecond ? 3 : 1][kSecond ? kMomentBodies : 1];  // second moments of the cells
+    short4 child[kMomentBodies];    // nodes
+    int parent[kMomentBodies];      // in the block's numbering
+    int nint[kMomentBodies];        // kOutside: the cell reaches beyond the block
+    int arrived[kMomentBodies];
+    short ready[2][kMomentBodies];  // cells whose children are done, this round's and the next
+    short tops[kMomentBodies];      // roots of the block's subtrees
+    int nready[2], ntops;
+};
+
 template <bool kSplit, bool kSecond>
-__global__ void tree_moments(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
-                             const double* __restrict__ mass, Tree t, Batch bt,
-                             float accept_scale,
-         unsigned long long* mark) {
+__global__ void __launch_bounds__(kMomentThreads, 2)
+tree_moments(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
+             const double* __restrict__ mass, int n, Tree t, Batch bt, float accept_scale,
+             unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    MomentSmem<kSecond>& S = *reinterpret_cast<MomentSmem<kSecond>*>(smem_raw);
     const int cells = s->cells;
-    if (k >= s->nstart) return;
-    int id = t.start_list[k];
-    // A path to the root crosses at most 30 cells; the bound only guards
-    // against a malformed tree.
-    for (int hop = 0;; ++hop) {
-        if (hop > kMaxLevel + 1) {
-            atomicOr(&s->error, kErrTree);
-            return;
+    const int b0 = blockIdx.x * kMomentBodies, b1 = min(n, b0 + kMomentBodies);  // bodies [b0, b1)
+    const int id0 = t.cell_of[b0];
+    const int count = (b1 < n ? t.cell_of[b1] : cells) - id0;  // fewer than the bodies
+    for (int k = threadIdx.x; k < b1 - b0; k += kMomentThreads) {
+        const int b = b0 + k;
+        const double2 p = pos[b];
+        double3 v = make_double3(mass[b], p.x, p.y);
+        // (leaf_last and the buckets mean something at leaf starts only, and
+        // only these are read)
+        if (t.leaf_last[b] != b) v = bucket_leaf(t, b);
+        S.m[kMomentBodies + k] = v.x;
+        S.x[kMomentBodies + k] = v.y;
+        S.y[kMomentBodies + k] = v.z;
+    }
+    if (threadIdx.x == 0) {
+        S.nready[0] = S.nready[1] = S.ntops = 0;
+        S.m[kMomentNodes - 1] = S.x[kMomentNodes - 1] = S.y[kMomentNodes - 1] = 0.0;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < count; k += kMomentThreads) {
+        const int2 r = t.range[id0 + k];
+        const int nint = t.nint[id0 + k];
+        const int4 ch = t.child[id0 + k];
+        const bool own = r.x >= b0 && r.y < b1;
+        auto node = [&](int ref) {
+            return (short)(ref == INT_MIN ? kMomentNodes - 1
+                           : ref >= 0     ? ref - id0
+                                          : kMomentBodies + ~ref - b0);
+        };
+        if (own) S.child[k] = make_short4(node(ch.x), node(ch.y), node(ch.z), node(ch.w));
+        S.nint[k] = own ? nint : kOutside;
+        S.arrived[k] = 0;
+        S.parent[k] = t.parent[id0 + k] - id0;
+        if (nint == 0) {
+            if (own) S.ready[0][atomicAdd(&S.nready[0], 1)] = (short)k;
+            else S.tops[atomicAdd(&S.ntops, 1)] = (short)k;
         }
-        cell_moments<kSplit, kSecond>(id, s, pos, mass, t, bt, accept_scale);
-        const int par = t.parent[id];
-        if (par < 0) return;
-        if (par >= cells) {
-            atomicOr(&s->error, kErrTree);
-            return;
+    }
+    __syncthreads();
+    auto own_cell = [&](int k) { return k >= 0 && k < count && S.nint[k] != kOutside; };
+    // one of the block's own cells
+    auto own_moments = [&](int k) {
+        const short4 ch = S.child[k];
+        const int node[4] = {ch.x, ch.y, ch.z, ch.w};
+        double3 c[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) c[q] = make_double3(S.m[node[q]], S.x[node[q]], S.y[node[q]]);
+        const Moments o = combine_children<kSecond>(c, [&](int q) {
+            const bool cell = kSecond && node[q] < kMomentBodies;
+            return cell ? make_double3(S.s[0][node[q]], S.s[1][node[q]], S.s[2][node[q]])
+                        : make_double3(0.0, 0.0, 0.0);
+        });
+        S.m[k] = o.m;
+        S.x[k] = o.x;
+        S.y[k] = o.y;
+        if (kSecond) {
+            S.s[0][k] = o.sxx;
+            S.s[1][k] = o.sxy;
+            S.s[2][k] = o.syy;
         }
-        const int arrived = arrive_acq_rel(t.ready + par);
-        if (arrived != t.nint[par] - 1) return;
-        id = par;
+    };
+    // a cell whose children's moments are in global memory
+    auto any_moments = [&](int id, int4 ch) {
+        const int refs[4] = {ch.x, ch.y, ch.z, ch.w};
+        double3 c[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = refs[q];
+            c[q] = make_double3(0.0, 0.0, 0.0);
+            if (r == INT_MIN) continue;
+            if (r >= 0) {
+                const double2 p = __ldcg(t.com + r);
+                c[q] = make_double3(__ldcg(t.mass + r), p.x, p.y);
+            } else {
+                const double2 p = pos[~r];
+                c[q] = make_double3(mass[~r], p.x, p.y);
+                if (t.leaf_last[~r] != ~r) c[q] = bucket_leaf(t, ~r);
+            }
+        }
+        const Moments o = combine_children<kSecond>(c, [&](int q) {
+            if (refs[q] < 0) return make_double3(0.0, 0.0, 0.0);
+            const double2* sc = reinterpret_cast<const double2*>(t.s64 + refs[q]);
+            const double2 s01 = __ldcg(sc), s2 = __ldcg(sc + 1);
+            return make_double3(s01.x, s01.y, s2.x);
+        });
+        store_moments<kSplit, kSecond>(id, o, true, s, pos, t, bt, accept_scale);
+    };
+    // Rounds: the cells that are ready are computed by consecutive threads (a
+    // thread that climbed alone would leave its warp's other lanes idle), and
+    // the last child to be done makes its parent ready for the next round.
+    // Global memory is left out of the rounds, which follow one another.
+    for (int r = 0;; ++r) {
+        const int todo = S.nready[r & 1];
+        if (todo == 0) break;
+        for (int j = threadIdx.x; j < todo; j += kMomentThreads) {
+            const int k = S.ready[r & 1][j];
+            own_moments(k);
+            const int p = S.parent[k];
+            if (!own_cell(p)) {
+                S.tops[atomicAdd(&S.ntops, 1)] = (short)k;
+            } else if (atomicAdd(&S.arrived[p], 1) == S.nint[p] - 1) {
+                S.ready[(r & 1) ^ 1][atomicAdd(&S.nready[(r & 1) ^ 1], 1)] = (short)p;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) S.nready[r & 1] = 0;
+        __syncthreads();
+    }
+    for (int k = threadIdx.x; k < count; k += kMomentThreads)
+        if (S.nint[k] != kOutside)
+            store_moments<kSplit, kSecond>(
+                id0 + k,
+                Moments{S.m[k], S.x[k], S.y[k], kSecond ? S.s[0][k] : 0.0, kSecond ? S.s[1][k] : 0.0,
+                        kSecond ? S.s[2][k] : 0.0},
+                !own_cell(S.parent[k]), s, pos, t, bt, accept_scale);
+    __syncthreads();
+    // Beyond the block: the cells that reach out of it and have no internal
+    // children, and the parents of the block's subtrees.  A path to the root
+    // crosses at most 30 cells; the bound only guards against a malformed tree.
+    const int ntops = S.ntops;
+    for (int j = threadIdx.x; j < ntops; j += kMomentThreads) {
+        const int k = S.tops[j];
+        if (S.nint[k] == kOutside) any_moments(id0 + k, t.child[id0 + k]);
+        int par = S.parent[k] + id0;
+        for (int hop = 0; par >= 0; ++hop) {
+            if (par >= cells || hop > kMaxLevel + 1) {
+                atomicOr(&s->error, kErrTree);
+                break;
+            }
+            const int needed = t.nint[par], up = t.parent[par];
+            const int4 ch = t.child[par];
+            if (arrive_acq_rel(t.ready + par) != needed - 1) break;
+            any_moments(par, ch);
+            par = up;
+        }
     }
 }
 
@@ -1322,26 +1443,21 @@ void launch_features(nb_ctx* c, const BodyBuffers& b, bool chained) {
                  b.pos, b.mass, c->tree, c->batch);
 }
 
+template <bool kSplit, bool kSecond>
+static void launch_climb(nb_ctx* c, const BodyBuffers& b, float accept_scale) {
+    auto* kernel = tree_moments<kSplit, kSecond>;
+    const size_t smem = sizeof(MomentSmem<kSecond>);
+    c->launches += 1;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    chain_launch(c->stream, true, kernel, blocks_for(c->n, kMomentBodies), kMomentThreads, smem, 1,
+                 c->scal, b.pos, b.mass, (int)c->n, c->tree, c->batch, accept_scale, mark_of(c, 5));
+}
+
+// SPLIT monopoles need none: the prefix sums ran before the tree, and the
+// linking pass wrote every cell's record from them.
 void launch_moments(nb_ctx* c, const BodyBuffers& b, bool split) {
-    // Cells never exceed n - 1; threads beyond the live count exit at once.
-    const int cap = (int)(c->n > 1 ? c->n - 1 : 1);
-    const bool second = split && (c->p.flags & NB_FLAG_QUADRUPOLE);
-    const double ratio = c->p.bmax_ratio;
-    const float accept_scale =
-        split && ratio > 0.0 ? (float)(c->p.theta * c->p.theta / (ratio * ratio)) : 0.f;
-    const unsigned blocks = blocks_for(cap, kThreads);
-    if (second) {
-        c->launches += 1;
-        chain_launch(c->stream, true, tree_moments<true, true>, blocks, kThreads, 0, 1, c->scal, b.pos,
-                     b.mass, c->tree, c->batch, accept_scale, mark_of(c, 5));
-    } else if (split) {
-        // monopoles: the prefix sums ran before the tree, and the linking
-        // pass wrote every cell's record from them
-    } else {
-        c->launches += 1;
-        chain_launch(c->stream, true, tree_moments<false, false>, blocks, kThreads, 0, 1, c->scal, b.pos,
-                     b.mass, c->tree, c->batch, 0.f, mark_of(c, 5));
-    }
+    if (!split) launch_climb<false, false>(c, b, 0.f);
+    else if (c->p.flags & NB_FLAG_QUADRUPOLE) launch_climb<true, true>(c, b, split_accept_scale(c));
 }
 
 }  // namespace nb

@@ -90,7 +90,6 @@ int alloc_all(nb_ctx* c) {
     NB_CUDA(c, dalloc(&t.mass, n));
     NB_CUDA(c, dalloc(&t.com, n));
     NB_CUDA(c, dalloc(&t.range, n));
-    NB_CUDA(c, dalloc(&t.start_list, n));
     if (c->p.mode == NB_MODE_ALLPAIRS)
         NB_CUDA(c, dalloc(&c->ap_partial, n * (size_t)nb::allpairs_chunks((int64_t)n, c->sm_count)));
     if (c->p.mode == NB_MODE_SPLIT) {
@@ -161,7 +160,7 @@ void free_all(nb_ctx* c) {
                          t.bnd,       t.range,       t.s64,         t.cell4,      t.cellq,      t.s32,
                          t.body4,     t.gcount,      t.gbase,       t.groups,     t.rep_of,
                          t.t32,       t.cellh,       t.band,        t.band_count,
-                         t.start_list, t.prefix, t.prefix_tiles, t.lcp8, t.ansv_first,
+                         t.prefix, t.prefix_tiles, t.lcp8, t.ansv_first,
                          t.ansv_last};
     for (void* q : tree_ptrs) cudaFree(q);
     cudaFree(c->scal);

@@ -45,7 +45,7 @@ struct DeviceScalars {
     unsigned long long body_terms;
     int32_t stack_hw;         // FP64 walk: deepest stack (entries) of the last force pass
     int32_t stack_pad_;
-    int32_t nstart;           // cells whose children are all leaves (climb starts)
+    int32_t pad2_;
     unsigned upload_bad;      // nb_upload's checks: bit 0 non-finite, bit 1 mass <= 0
     // Radix sort over the top sort_passes bytes of the keys only (1..8), chosen
     // per step from the previous tree's histogram of shared leading digits of
@@ -118,7 +118,6 @@ struct Tree {
     uint4* cellh = nullptr;
     int32_t* band = nullptr;       // per group: band cells, kBandPerBody x first body onwards
     int32_t* band_count = nullptr; // per group: band cells found
-    int32_t* start_list = nullptr; // cells without internal children, in any order
     // SPLIT monopole moments: exclusive prefix sums over the sorted bodies of
     // {m, m (x - frame centre), m (y - frame centre), 0}, n + 1 entries, and
     // the per-tile totals of the scan that builds them
