@@ -9,11 +9,10 @@
 //   of leading 2-bit digits their codes share.  Every boundary with d_i < 30
 //   separates two children of the cell "bodies sharing d_i digits with body
 //   i", whose level is d_i.  That cell is created once, by its first child
-//   boundary (the one whose left neighbour run starts the cell), found with
-//   an O(1) test after one galloping search.  Cells are numbered by an
-//   exclusive scan over those boundaries, which lays every subtree out as a
-//   contiguous id range.  A third pass links children (<= 4 per cell) and
-//   parents.
+//   boundary.  Cells are numbered in the order of those boundaries, which lays
+//   every subtree out as a contiguous id range: each tile of boundaries ranks
+//   its own, the last tile to be done adds up the tiles.  A last pass links
+//   children (<= 4 per cell) and parents.
 //
 // The reference tree is uncompressed: a cell with one non-empty child is
 // followed by a chain of single-child cells down to the next split, all with
@@ -86,7 +85,7 @@ __device__ int gallop_right(const uint64_t* __restrict__ key, int i, int hi, int
 // thermometer word (bit v set for every v above its level) and a 32 x 32 bit
 // transpose across the warp (five butterfly shuffles) hands lane v bit v of
 // every lane, which is that mask.
-constexpr int kAnsvItems = kAnsvTile / kThreads;  // rows per warp
+constexpr int kAnsvItems = kAnsvTile / kThreads;  // rows per warp (256 threads per tile)
 constexpr int kAnsvRows = kAnsvTile / 32;           // 64 rows
 constexpr int kNoLevel = kMaxLevel + 1;             // past the last body: never below a level
 static_assert(kAnsvItems == 8 && kAnsvLevels == 32, "one lane per level, 8 rows per warp");
@@ -118,14 +117,31 @@ __device__ __forceinline__ unsigned thermometer(int c) {
     return c >= 31 ? 0u : (0xFFFFFFFFu << (c + 1));
 }
 
-// Tables are level-major: tab[v * tiles + t].
-__global__ void __launch_bounds__(kThreads)
-tree_lcp(const uint64_t* __restrict__ key, int n, int tiles, uint8_t* __restrict__ lcp8,
-         int32_t* __restrict__ tile_first, int32_t* __restrict__ tile_last,
-         unsigned* __restrict__ lcp_hist,
+// Per level v and tile t the first and last boundary with a level below v.
+// Level-major for the scan over the tiles; tile-major when tree_ansv reads the
+// other tiles' entries itself.
+struct TileTable {
+    int32_t *first, *last;
+    int level_stride, tile_stride;
+    __device__ __forceinline__ int at(int v, int t) const { return v * level_stride + t * tile_stride; }
+};
+// Up to this many tiles, tree_ansv goes through the other tiles' entries (a few
+// loads per thread) instead of a scan kernel before it.
+constexpr int kFewTiles = 64;
+
+// kBlock threads per tile: 1,024 while every SM has at most one tile (a warp's
+// rows follow one another), else 256.
+constexpr int kWideThreads = 1024;
+constexpr int kWideTiles = 148;
+
+template <int kBlock>
+__global__ void __launch_bounds__(kBlock)
+tree_lcp(const uint64_t* __restrict__ key, int n, uint8_t* __restrict__ lcp8,
+         TileTable tab, unsigned* __restrict__ lcp_hist,
          unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
+    constexpr int kItems = kAnsvTile / kBlock;
     __shared__ unsigned hist[33];
     __shared__ int sfirst[kAnsvLevels], slast[kAnsvLevels];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -135,13 +151,13 @@ tree_lcp(const uint64_t* __restrict__ key, int n, int tiles, uint8_t* __restrict
         slast[threadIdx.x] = -1;
     }
     __syncthreads();
-    const int base = blockIdx.x * kAnsvTile + warp * (32 * kAnsvItems);
+    const int base = blockIdx.x * kAnsvTile + warp * (32 * kItems);
     // lane v (1..30): first and last boundary of the warp's rows with level < v;
     // lane v (1..31) and lane 0 (for 32): how many have a level < v
     int myfirst = INT_MAX, mylast = -1;
     unsigned mycnt = 0, nbound = 0;
 #pragma unroll 1
-    for (int r = 0; r < kAnsvItems; ++r) {
+    for (int r = 0; r < kItems; ++r) {
         const int row0 = base + 32 * r;
         const int i = row0 + lane;
         int c = 64;  // not a boundary
@@ -170,8 +186,8 @@ tree_lcp(const uint64_t* __restrict__ key, int n, int tiles, uint8_t* __restrict
     }
     __syncthreads();
     if (threadIdx.x < kAnsvLevels) {
-        tile_first[threadIdx.x * tiles + blockIdx.x] = sfirst[threadIdx.x];
-        tile_last[threadIdx.x * tiles + blockIdx.x] = slast[threadIdx.x];
+        tab.first[tab.at(threadIdx.x, blockIdx.x)] = sfirst[threadIdx.x];
+        tab.last[tab.at(threadIdx.x, blockIdx.x)] = slast[threadIdx.x];
     }
     // the next step's sort reads how many neighbouring codes share d digits
     if (threadIdx.x < 33 && hist[threadIdx.x]) atomicAdd(lcp_hist + threadIdx.x, hist[threadIdx.x]);
@@ -229,107 +245,7 @@ tree_ansv_tiles(int tiles, int32_t* __restrict__ tile_first, int32_t* __restrict
     }
 }
 
-// Per boundary i below kMaxLevel: flag = 1 iff i is its cell's first
-// separator (no equal level between it and the cell's start), which numbers
-// the cells; bnd[i] = {first body of the cell, last body of the cell,
-// previous separator of the cell or -1, next separator or -1}, the first two
-// written for flagged boundaries only.  The cell's first body follows the
-// nearest smaller level on the left, its last body is the nearest smaller on
-// the right (or n - 1); a separator's neighbours are the nearest levels <= c_i
-// when those equal c_i.
-__global__ void __launch_bounds__(kThreads)
-tree_ansv(const uint8_t* __restrict__ lcp8, int n, int tiles,
-          const int32_t* __restrict__ tile_first, const int32_t* __restrict__ tile_last,
-          int32_t* __restrict__ flag, int4* __restrict__ bnd) {
-    chain_begin();
-    // masks[r][v]: row r's ballot of "level < v" (v = 1..30; 0 elsewhere).
-    // rlast[r][v]: after the scan, the last boundary with a level below v in
-    // rows 8p..r of r's part p (-1 if none), rfirst[r][v] the first in rows
-    // r..8p+7 (kAnsvTile if none); tile-local positions
-    __shared__ unsigned masks[kAnsvRows][32];
-    __shared__ int16_t rlast[kAnsvRows][kAnsvLevels];
-    __shared__ int16_t rfirst[kAnsvRows][kAnsvLevels];
-    __shared__ int16_t before[kThreads / 32][kAnsvLevels];  // last in the parts before p
-    __shared__ int16_t after[kThreads / 32][kAnsvLevels];   // first in the parts after p
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tile = blockIdx.x, tbase = tile * kAnsvTile;
-#pragma unroll 1
-    for (int r = 0; r < kAnsvItems; ++r) {
-        const int row = warp * kAnsvItems + r;
-        const int i = tbase + 32 * row + lane;
-        const int cap = i < n ? lcp8[i] : kNoLevel;
-        // lane v: the row's mask of levels below v (lanes 0 and 31 unused: 0)
-        unsigned mine = warp_transpose_bits(thermometer(cap));
-        if (lane == 0 || lane > kMaxLevel) mine = 0u;
-        masks[row][lane] = mine;
-        rfirst[row][lane] = (int16_t)(mine ? 32 * row + __ffs(mine) - 1 : kAnsvTile);
-        rlast[row][lane] = (int16_t)(mine ? 32 * row + 31 - __clz(mine) : -1);
-    }
-    __syncwarp();
-    {   // scan the warp's own 8 rows, lane = level
-        int run = -1;
-        for (int r = 0; r < kAnsvItems; ++r) {
-            const int row = warp * kAnsvItems + r;
-            run = max(run, (int)rlast[row][lane]);
-            rlast[row][lane] = (int16_t)run;
-        }
-        int runf = kAnsvTile;
-        for (int r = kAnsvItems - 1; r >= 0; --r) {
-            const int row = warp * kAnsvItems + r;
-            runf = min(runf, (int)rfirst[row][lane]);
-            rfirst[row][lane] = (int16_t)runf;
-        }
-    }
-    __syncthreads();
-    {
-        int b = -1, a = kAnsvTile;
-        for (int p = 0; p < kThreads / 32; ++p) {
-            if (p < warp) b = max(b, (int)rlast[p * kAnsvItems + kAnsvItems - 1][lane]);
-            if (p > warp) a = min(a, (int)rfirst[p * kAnsvItems][lane]);
-        }
-        before[warp][lane] = (int16_t)b;
-        after[warp][lane] = (int16_t)a;
-    }
-    __syncthreads();
-    const unsigned lt = lanemask_lt(), gt = ~lt & ~(1u << lane);
-#pragma unroll 1
-    for (int r = 0; r < kAnsvItems; ++r) {
-        const int row = warp * kAnsvItems + r;
-        const int i = tbase + 32 * row + lane;
-        if (i >= n) continue;
-        const int v = lcp8[i];
-        if (i == n - 1 || v >= kMaxLevel) {
-            flag[i] = 0;
-            continue;
-        }
-        // nearest boundary on the left / right with a level below u
-        auto left = [&](int u) {
-            const unsigned m = masks[row][u] & lt;
-            if (m) return tbase + 32 * row + 31 - __clz(m);
-            int j = r > 0 ? (int)rlast[row - 1][u] : -1;
-            if (j < 0) j = before[warp][u];
-            if (j >= 0) return tbase + j;
-            return tile > 0 ? tile_last[u * tiles + tile - 1] : -1;
-        };
-        auto right = [&](int u) {
-            const unsigned m = masks[row][u] & gt;
-            if (m) return tbase + 32 * row + __ffs(m) - 1;
-            int j = r < kAnsvItems - 1 ? (int)rfirst[row + 1][u] : kAnsvTile;
-            if (j >= kAnsvTile) j = after[warp][u];
-            if (j < kAnsvTile) return tbase + j;
-            const int g = tile + 1 < tiles ? tile_first[u * tiles + tile + 1] : INT_MAX;
-            return g == INT_MAX ? n - 1 : g;
-        };
-        const int l_lt = left(v), l_le = left(v + 1);
-        const int r_lt = right(v), r_le = right(v + 1);
-        const bool first_sep = l_le == l_lt;
-        flag[i] = first_sep ? 1 : 0;
-        bnd[i] = make_int4(first_sep ? l_lt + 1 : -1, first_sep ? r_lt : -1,
-                           first_sep ? -1 : l_le, r_le == r_lt ? -1 : r_le);
-    }
-}
-
-// ---- exclusive scan of flag[] -> cell_of[], total -> scal->cells ----------
+// ---- numbering the cells ---------------------------------------------------
 __device__ __forceinline__ int warp_inclusive(int v) {
     const int lane = threadIdx.x & 31;
     for (int o = 1; o < 32; o <<= 1) {
@@ -358,80 +274,194 @@ __device__ int block_exclusive(int v, int* wsum, int* total) {
     return r;
 }
 
-// Items of a tile are read in coalesced rows: warp w takes the 32 *
-// kScanItems items [w 32 kScanItems, (w + 1) 32 kScanItems) of the tile,
-// lane l the items 32 k + l of them.
-__global__ void __launch_bounds__(kThreads)
-scan_reduce(const int32_t* __restrict__ in, int n, int32_t* __restrict__ block_sums,
-         unsigned long long* mark) {
-    chain_begin();
-    mark_start(mark);
-    __shared__ int wsum[kThreads / 32];
-    __shared__ int total;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int base = blockIdx.x * kScanTile + warp * 32 * kScanItems + lane;
-    int v = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const int i = base + 32 * k;
-        if (i < n) v += in[i];
-    }
-    block_exclusive(v, wsum, &total);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-// One block of kSumsThreads: the block sums of 4M entries (2,048) take two
-// rounds instead of eight.
-constexpr int kSumsThreads = 1024;
-__global__ void __launch_bounds__(kSumsThreads)
-scan_block_sums(int32_t* __restrict__ block_sums, int blocks, int32_t* __restrict__ total_out) {
-    chain_begin();
-    __shared__ int wsum[kSumsThreads / 32];
-    __shared__ int total;
-    int carry = 0;
-    for (int b = 0; b < blocks; b += kSumsThreads) {
-        const int t = b + threadIdx.x;
-        const int v = t < blocks ? block_sums[t] : 0;
-        const int ex = block_exclusive<kSumsThreads>(v, wsum, &total);
-        if (t < blocks) block_sums[t] = carry + ex;
-        carry += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *total_out = carry;
-}
-
-// Each row of 32 items is scanned with shuffles; the rows' totals carry
-// within the warp, and the warps' totals (one barrier) within the tile.
-__global__ void __launch_bounds__(kThreads)
-scan_apply(const int32_t* __restrict__ in, int n, const int32_t* __restrict__ block_sums,
-           int32_t* __restrict__ out, int32_t* __restrict__ index_of) {
-    chain_begin();
-    __shared__ int wsum[kThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int base = blockIdx.x * kScanTile + warp * 32 * kScanItems + lane;
-    int v[kScanItems], ex[kScanItems];
-    int carry = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const int i = base + 32 * k;
-        v[k] = i < n ? in[i] : 0;
-        const int inc = warp_inclusive(v[k]);
-        ex[k] = carry + inc - v[k];
-        carry += __shfl_sync(kFull, inc, 31);
-    }
-    if (lane == 0) wsum[warp] = carry;
+// Whether this block is the grid's last to come here; the writes of all blocks
+// before are then visible to it.  The ticket is left at zero.
+__device__ bool last_block(unsigned* ticket, unsigned blocks) {
+    __shared__ bool last;
     __syncthreads();
-    int off = block_sums[blockIdx.x];
-    for (int w = 0; w < warp; ++w) off += wsum[w];
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const int i = base + 32 * k;
-        if (i < n) {
-            const int run = off + ex[k];
-            out[i] = run;
-            // with 0/1 inputs, index_of lists the flagged positions in order
-            if (index_of && v[k]) index_of[run] = i;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == blocks - 1;
+        if (last) {
+            __threadfence();
+            *ticket = 0;
         }
+    }
+    __syncthreads();
+    return last;
+}
+
+// One block: out[k] = sum of in[0..k), returns the total.
+template <int kBlock>
+__device__ int scan_tiles(const int32_t* in, int count, int32_t* out) {
+    __shared__ int wsum[kBlock / 32];
+    __shared__ int total;
+    const int per = (count + kBlock - 1) / kBlock;
+    const int k0 = min(count, (int)threadIdx.x * per), k1 = min(count, k0 + per);
+    int sum = 0;
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) sum += __ldcg(in + k);
+    int run = block_exclusive<kBlock>(sum, wsum, &total);
+    for (int k = k0; k < k1; ++k) {
+        const int v = __ldcg(in + k);
+        out[k] = run;
+        run += v;
+    }
+    return total;
+}
+
+// Cells are numbered by their first separators: the cells of the tiles before,
+// then the rank in the tile.
+__device__ __forceinline__ int cell_id(const Tree& t, int boundary) {
+    return t.tile_cells[boundary / kAnsvTile] + t.cell_rank[boundary];
+}
+
+// A boundary i below kMaxLevel creates a cell iff it is the cell's first
+// separator (no equal level between it and the cell's start), which numbers
+// the cells: cell_rank[i] = such boundaries before i in its tile, rep[] lists a
+// tile's, and the grid's last block adds up the tiles (three scan kernels and a
+// number per boundary before: tree and groups 254 -> 209 us at 4M, 51 -> 38 at
+// 300,007 bodies, 36 -> 22 at 16,384).  bnd[i] = {first body of the cell, last body of the cell,
+// previous separator of the cell or -1, next separator or -1}, the first two
+// written for flagged boundaries only.  The cell's first body follows the
+// nearest smaller level on the left, its last body is the nearest smaller on
+// the right (or n - 1); a separator's neighbours are the nearest levels <= c_i
+// when those equal c_i.
+template <int kBlock>
+__global__ void __launch_bounds__(kBlock)
+tree_ansv(Tree t, int n, int tiles, TileTable tab, DeviceScalars* __restrict__ s) {
+    chain_begin();
+    constexpr int kItems = kAnsvTile / kBlock, kWarps = kBlock / 32;
+    // masks[r][v]: row r's ballot of "level < v" (v = 1..30; 0 elsewhere).
+    // rlast[r][v]: after the scan, the last boundary with a level below v in
+    // rows of r's part p up to r (-1 if none), rfirst[r][v] the first in rows
+    // from r on (kAnsvTile if none); tile-local positions
+    __shared__ unsigned masks[kAnsvRows][32];
+    __shared__ int16_t rlast[kAnsvRows][kAnsvLevels];
+    __shared__ int16_t rfirst[kAnsvRows][kAnsvLevels];
+    __shared__ int16_t before[kWarps][kAnsvLevels];  // last in the parts before p
+    __shared__ int16_t after[kWarps][kAnsvLevels];   // first in the parts after p
+    __shared__ unsigned creates[kAnsvRows];  // the row's first separators
+    __shared__ int far_last[kWarps][32], far_first[kWarps][32];
+    const uint8_t* __restrict__ lcp8 = t.lcp8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tile = blockIdx.x, tbase = tile * kAnsvTile;
+    // few tiles: the last boundary below level `lane` in the tiles before, the
+    // first in the tiles after, over a part of the tiles per warp
+    const bool few = tiles <= kFewTiles;
+    if (few) {
+        int l = -1, f = INT_MAX;
+#pragma unroll 4
+        for (int q = warp; q < tiles; q += kWarps) {
+            if (q < tile) l = max(l, tab.last[tab.at(lane, q)]);
+            if (q > tile) f = min(f, tab.first[tab.at(lane, q)]);
+        }
+        far_last[warp][lane] = l;
+        far_first[warp][lane] = f;
+    }
+#pragma unroll 1
+    for (int r = 0; r < kItems; ++r) {
+        const int row = warp * kItems + r;
+        const int i = tbase + 32 * row + lane;
+        const int cap = i < n ? lcp8[i] : kNoLevel;
+        // lane v: the row's mask of levels below v (lanes 0 and 31 unused: 0)
+        unsigned mine = warp_transpose_bits(thermometer(cap));
+        if (lane == 0 || lane > kMaxLevel) mine = 0u;
+        masks[row][lane] = mine;
+        rfirst[row][lane] = (int16_t)(mine ? 32 * row + __ffs(mine) - 1 : kAnsvTile);
+        rlast[row][lane] = (int16_t)(mine ? 32 * row + 31 - __clz(mine) : -1);
+    }
+    __syncwarp();
+    {   // scan the warp's own 8 rows, lane = level
+        int run = -1;
+        for (int r = 0; r < kItems; ++r) {
+            const int row = warp * kItems + r;
+            run = max(run, (int)rlast[row][lane]);
+            rlast[row][lane] = (int16_t)run;
+        }
+        int runf = kAnsvTile;
+        for (int r = kItems - 1; r >= 0; --r) {
+            const int row = warp * kItems + r;
+            runf = min(runf, (int)rfirst[row][lane]);
+            rfirst[row][lane] = (int16_t)runf;
+        }
+    }
+    __syncthreads();
+    {
+        int b = -1, a = kAnsvTile;
+        for (int p = 0; p < kWarps; ++p) {
+            if (p < warp) b = max(b, (int)rlast[p * kItems + kItems - 1][lane]);
+            if (p > warp) a = min(a, (int)rfirst[p * kItems][lane]);
+        }
+        before[warp][lane] = (int16_t)b;
+        after[warp][lane] = (int16_t)a;
+    }
+    if (few && warp == 0) {
+        int l = -1, f = INT_MAX;
+        for (int p = 0; p < kWarps; ++p) {
+            l = max(l, far_last[p][lane]);
+            f = min(f, far_first[p][lane]);
+        }
+        far_last[0][lane] = l;
+        far_first[0][lane] = f;
+    }
+    __syncthreads();
+    const unsigned lt = lanemask_lt(), gt = ~lt & ~(1u << lane);
+#pragma unroll 1
+    for (int r = 0; r < kItems; ++r) {
+        const int row = warp * kItems + r;
+        const int i = tbase + 32 * row + lane;
+        const int v = i < n - 1 ? lcp8[i] : kNoLevel;
+        bool first_sep = false;
+        if (v < kMaxLevel) {
+            // nearest boundary on the left / right with a level below u
+            auto left = [&](int u) {
+                const unsigned m = masks[row][u] & lt;
+                if (m) return tbase + 32 * row + 31 - __clz(m);
+                int j = r > 0 ? (int)rlast[row - 1][u] : -1;
+                if (j < 0) j = before[warp][u];
+                if (j >= 0) return tbase + j;
+                if (few) return far_last[0][u];
+                return tile > 0 ? tab.last[tab.at(u, tile - 1)] : -1;
+            };
+            auto right = [&](int u) {
+                const unsigned m = masks[row][u] & gt;
+                if (m) return tbase + 32 * row + __ffs(m) - 1;
+                int j = r < kItems - 1 ? (int)rfirst[row + 1][u] : kAnsvTile;
+                if (j >= kAnsvTile) j = after[warp][u];
+                if (j < kAnsvTile) return tbase + j;
+                const int g = few                ? far_first[0][u]
+                              : tile + 1 < tiles ? tab.first[tab.at(u, tile + 1)]
+                                                 : INT_MAX;
+                return g == INT_MAX ? n - 1 : g;
+            };
+            const int l_lt = left(v), l_le = left(v + 1);
+            const int r_lt = right(v), r_le = right(v + 1);
+            first_sep = l_le == l_lt;
+            t.bnd[i] = make_int4(first_sep ? l_lt + 1 : -1, first_sep ? r_lt : -1,
+                                 first_sep ? -1 : l_le, r_le == r_lt ? -1 : r_le);
+        }
+        const unsigned c = __ballot_sync(kFull, first_sep);
+        if (lane == 0) creates[row] = c;
+    }
+    __syncthreads();
+    int run = 0;  // of the warps before
+    for (int q = lane; q < warp * kItems; q += 32) run += __popc(creates[q]);
+    run = __reduce_add_sync(kFull, run);
+    for (int r = 0; r < kItems; ++r) {
+        const int row = warp * kItems + r;
+        const int i = tbase + 32 * row + lane;
+        const unsigned c = creates[row];
+        const int rank = run + __popc(c & lt);
+        if (i < n) t.cell_rank[i] = (uint16_t)rank;
+        if ((c >> lane) & 1u) t.rep[tbase + rank] = (uint16_t)(i - tbase);
+        run += __popc(c);
+    }
+    if (threadIdx.x == kBlock - 1) t.tile_count[tile] = run;
+    if (threadIdx.x == 0 && t.tile_groups) t.tile_groups[tile] = 0;  // the linking pass counts
+    if (last_block(&s->tile_ticket, gridDim.x)) {
+        const int total = scan_tiles<kBlock>(t.tile_count, tiles, t.tile_cells);
+        if (threadIdx.x == 0) s->cells = total;
     }
 }
 
@@ -483,49 +513,52 @@ __device__ void cell_from_prefix(const double4* __restrict__ prefix, const Tree&
 
 // The SPLIT target groups of one cell (defined with tree_groups_write below).
 template <bool kWrite>
-__device__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const int* cb,
+__device__ __forceinline__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const int* cb,
                            const bool* leaf, int gsize, int fill, const Batch& bt,
                            const uint64_t* __restrict__ key, int2* __restrict__ out);
 
-// Five blocks per SM (48 registers): more dependent load chains in flight
-// than the 56-register build's four (tree phase 0.196 -> 0.192 ms at 4M).
-// kMono (SPLIT monopoles): the prefix sums are ready, and each cell also
-// writes its monopole record, which saves a pass over the cells.  gsize > 0
-// (SPLIT): each cell also counts its target groups into gcount.
+// A tree without internal cells: one body, or all bodies in one level-30 leaf.
+__device__ void trivial_root(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
+                             const Tree& t, DeviceScalars* __restrict__ s) {
+    s->root = ~0;
+    t.leaf_last[0] = n - 1;
+    t.leaf_plevel[0] = -1;
+    if (n > 1) bucket_moments(pos, mass, 0, n - 1, t.bucket_mass, t.bucket_com);
+}
+
+// Cell id, created by boundary i; returns its target groups (gsize > 0).
 template <bool kMono>
-__global__ void __launch_bounds__(kThreads, 5)
-tree_link(const uint64_t* __restrict__ key, const uint8_t* __restrict__ lcp8, int n,
-          const double2* __restrict__ pos, const double* __restrict__ mass, Tree t,
-          DeviceScalars* __restrict__ s, const double4* __restrict__ prefix, Batch bt,
-          float accept_scale, int gsize, int fill) {
-    chain_begin();
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    const int cells = s->cells;
-    if (id >= cells) {
-        if (gsize > 0 && id < n) t.gcount[id] = 0;  // the group scan runs over n entries
-        return;
-    }
-    const int i = t.rep_of[id];
+__device__ __forceinline__ int link_cell(int i, int id, const uint64_t* __restrict__ key, int n,
+                                         const double2* __restrict__ pos,
+                                         const double* __restrict__ mass, const Tree& t,
+                                         DeviceScalars* __restrict__ s,
+                                         const double4* __restrict__ prefix, const Batch& bt,
+                                         float accept_scale, int gsize, int fill) {
+    const uint8_t* __restrict__ lcp8 = t.lcp8;
     const int4 bi = t.bnd[i];
     const int c = lcp8[i];
     const int first = bi.x, last = bi.y;
     // the cell's separators: i, then the chain of next separators
     int sep[3] = {i, n - 1, n - 1};
     int ns = 1;
-    for (int j = bi.w; j >= 0; j = t.bnd[j].w) {
-        if (ns == 3) {  // a fifth child: the codes are inconsistent
-            atomicOr(&s->error, kErrTree);
-            break;
+    int next = bi.w;
+#pragma unroll
+    for (int q = 1; q < 3; ++q)
+        if (next >= 0) {
+            sep[q] = next;
+            ++ns;
+            next = t.bnd[next].w;
         }
-        sep[ns++] = j;
-    }
+    if (next >= 0) atomicOr(&s->error, kErrTree);  // a fifth child: inconsistent codes
     int* child = reinterpret_cast<int*>(t.child + id);
     int nint = 0;
     int ca[4], cb[4];
     bool leaf[4];
-    for (int q = 0; q <= ns; ++q) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q > ns) continue;
         const int a = q == 0 ? first : sep[q - 1] + 1;
-        const int b = q == ns ? last : sep[q];
+        const int b = q == ns ? last : sep[min(q, 2)];
         ca[q] = a;
         cb[q] = b;
         leaf[q] = true;
@@ -544,9 +577,12 @@ tree_link(const uint64_t* __restrict__ key, const uint8_t* __restrict__ lcp8, in
             ++nint;  // a cell: it enters itself below
         }
     }
-    if (gsize > 0)
-        t.gcount[id] = cell_groups<false>(make_int2(first, last), first == 0 && last == n - 1,
+    int groups = 0;
+    if (gsize > 0) {
+        groups = cell_groups<false>(make_int2(first, last), first == 0 && last == n - 1,
                                           ns + 1, ca, cb, leaf, gsize, fill, bt, key, nullptr);
+        t.gcount[id] = groups;
+    }
     for (int q = ns + 1; q < 4; ++q) child[q] = INT_MIN;
     t.range[id] = make_int2(first, last);
     t.level[id] = c;
@@ -556,7 +592,7 @@ tree_link(const uint64_t* __restrict__ key, const uint8_t* __restrict__ lcp8, in
     if (first == 0 && last == n - 1) {
         s->root = id;
         t.parent[id] = -1;
-        return;
+        return groups;
     }
     const int cl = first > 0 ? lcp8[first - 1] : -1;
     const int cr = last < n - 1 ? lcp8[last] : -1;
@@ -570,23 +606,43 @@ tree_link(const uint64_t* __restrict__ key, const uint8_t* __restrict__ lcp8, in
     const int slot = from_left ? rank + 1 : rank;
     if (slot > 3) {  // more than four children: the codes are inconsistent
         atomicOr(&s->error, kErrTree);
-        return;
+        return groups;
     }
-    const int pid = t.cell_of[k];
+    const int pid = cell_id(t, k);
     reinterpret_cast<int*>(t.child + pid)[slot] = id;
     t.parent[id] = pid;
+    return groups;
 }
 
-// A tree without internal cells: one body, or all bodies in one level-30 leaf.
-__global__ void tree_trivial_root(const double2* __restrict__ pos, const double* __restrict__ mass,
-                                  int n, Tree t, DeviceScalars* __restrict__ s, int gsize) {
+// Five blocks per SM (48 registers): more dependent load chains in flight
+// than the 56-register build's four (tree phase 0.196 -> 0.192 ms at 4M).
+// kMono (SPLIT monopoles): the prefix sums are ready, and each cell also
+// writes its monopole record, which saves a pass over the cells.  gsize > 0
+// (SPLIT): each cell also counts its target groups into gcount.
+constexpr int kLinkBlocks = kAnsvTile / kThreads;
+
+template <bool kMono>
+__global__ void __launch_bounds__(kThreads, 5)
+tree_link(const uint64_t* __restrict__ key, int n, const double2* __restrict__ pos,
+          const double* __restrict__ mass, Tree t, DeviceScalars* __restrict__ s,
+          const double4* __restrict__ prefix, Batch bt, float accept_scale, int gsize, int fill) {
     chain_begin();
-    if (s->cells != 0) return;
-    if (gsize > 0) t.gcount[0] = (n + gsize - 1) / gsize;  // groups of the root leaf
-    s->root = ~0;
-    t.leaf_last[0] = n - 1;
-    t.leaf_plevel[0] = -1;
-    if (n > 1) bucket_moments(pos, mass, 0, n - 1, t.bucket_mass, t.bucket_com);
+    const int tile = blockIdx.x / kLinkBlocks;
+    const int cells = s->cells;
+    if (cells == 0) {  // one body, or all bodies in one level-30 leaf
+        if (blockIdx.x == 0 && threadIdx.x == 0) trivial_root(pos, mass, n, t, s);
+        return;
+    }
+    // the tile's cell j; kLinkBlocks blocks share a tile
+    const int j = (blockIdx.x % kLinkBlocks) * kThreads + threadIdx.x;
+    int groups = 0;
+    if (j < t.tile_count[tile])
+        groups = link_cell<kMono>(tile * kAnsvTile + t.rep[tile * kAnsvTile + j],
+                                  t.tile_cells[tile] + j, key, n, pos, mass, t, s, prefix, bt,
+                                  accept_scale, gsize, fill);
+    if (gsize == 0) return;
+    const int sum = __reduce_add_sync(kFull, groups);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(t.tile_groups + tile, sum);
 }
 
 // b_max^2 of a cell: squared distance from its COM to the farthest corner of
@@ -770,8 +826,8 @@ tree_moments(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
     MomentSmem<kSecond>& S = *reinterpret_cast<MomentSmem<kSecond>*>(smem_raw);
     const int cells = s->cells;
     const int b0 = blockIdx.x * kMomentBodies, b1 = min(n, b0 + kMomentBodies);  // bodies [b0, b1)
-    const int id0 = t.cell_of[b0];
-    const int count = (b1 < n ? t.cell_of[b1] : cells) - id0;  // fewer than the bodies
+    const int id0 = cell_id(t, b0);
+    const int count = (b1 < n ? cell_id(t, b1) : cells) - id0;  // fewer than the bodies
     for (int k = threadIdx.x; k < b1 - b0; k += kMomentThreads) {
         const int b = b0 + k;
         const double2 p = pos[b];
@@ -944,28 +1000,12 @@ __device__ double4 block_sum_d4(double4 v, double4* red) {
     return tot;  // valid in thread 0
 }
 
-// Bodies of a tile are read in coalesced rows: warp w takes the kWarpItems
-// bodies [w kWarpItems, (w + 1) kWarpItems) of the tile, lane l the bodies
-// 32 k + l of them.
+// Bodies of a tile are read in coalesced rows: each warp takes consecutive rows
+// of 32.
 constexpr int kWarpItems = 32 * kScanItems;
-
-// Phase 1: per tile of kScanTile bodies, the total.
-__global__ void __launch_bounds__(kThreads)
-prefix_reduce(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
-              const DeviceScalars* __restrict__ s, Batch bt, double4* __restrict__ tiles,
-         unsigned long long* mark) {
-    chain_begin();
-    mark_start(mark);
-    __shared__ double4 red[kThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int base = blockIdx.x * kScanTile + warp * kWarpItems + lane;
-    double4 v = make_double4(0.0, 0.0, 0.0, 0.0);
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + 32 * k < n) v = d4_add(v, body_term(pos, mass, s, bt, base + 32 * k));
-    const double4 tot = block_sum_d4(v, red);
-    if (threadIdx.x == 0) tiles[blockIdx.x] = tot;
-}
+// Up to this many tiles a block of the second phase scans the totals itself
+// (one warp, 8 per lane) instead of a kernel between the phases.
+constexpr int kFewSums = 32 * kScanItems;
 
 // Inclusive scan across the warp of the three components body_term fills.
 __device__ __forceinline__ double4 warp_inclusive_d4(double4 v) {
@@ -1000,13 +1040,14 @@ __device__ double4 block_exclusive_d4(double4 v, double4* part, double4& total) 
     return ex;
 }
 
-// Phase 2: exclusive scan of the tile totals (one block, chunks of
-// kThreads * kScanItems tiles in order); tiles[ntiles] = the grand total.
-__global__ void __launch_bounds__(kThreads) prefix_tiles_scan(double4* __restrict__ tiles, int ntiles) {
+// Many tiles: exclusive scan of the totals (one block, chunks of kThreads *
+// kScanItems tiles in order); tiles[ntiles] = the grand total.
+__global__ void __launch_bounds__(kThreads)
+prefix_tiles_scan(double4* __restrict__ tiles, int ntiles) {
     chain_begin();
     __shared__ double4 part[kThreads];
     double4 carry = make_double4(0.0, 0.0, 0.0, 0.0);
-    for (int c0 = 0; c0 < ntiles; c0 += kScanTile) {
+    for (int c0 = 0; c0 < ntiles; c0 += kThreads * kScanItems) {
         const int base = c0 + threadIdx.x * kScanItems;
         double4 v[kScanItems];
         double4 run = make_double4(0.0, 0.0, 0.0, 0.0);
@@ -1025,46 +1066,91 @@ __global__ void __launch_bounds__(kThreads) prefix_tiles_scan(double4* __restric
     if (threadIdx.x == 0) tiles[ntiles] = carry;
 }
 
-// Phase 3: prefix[i] = sum over bodies before i; prefix[n] = the total.
-// Each row of 32 bodies is scanned with shuffles; the rows' totals carry
-// within the warp, and the warps' totals (one barrier) within the tile.
+// Phase 1: per tile of kScanTile bodies, the total.
 __global__ void __launch_bounds__(kThreads)
+prefix_reduce(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
+              const DeviceScalars* __restrict__ s, Batch bt, double4* __restrict__ tiles,
+              unsigned long long* mark) {
+    chain_begin();
+    mark_start(mark);
+    __shared__ double4 red[kThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int base = blockIdx.x * kScanTile + warp * kWarpItems + lane;
+    double4 v = make_double4(0.0, 0.0, 0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k)
+        if (base + 32 * k < n) v = d4_add(v, body_term(pos, mass, s, bt, base + 32 * k));
+    const double4 tot = block_sum_d4(v, red);
+    if (threadIdx.x == 0) tiles[blockIdx.x] = tot;
+}
+
+// Phase 2: prefix[i] = sum over bodies before i; prefix[n] = the total.
+// Each row of 32 bodies is scanned with shuffles; the rows' totals carry
+// within the warp, and the warps' totals (one barrier) within the tile.  Few
+// tiles (kFew): the block scans the tiles' totals itself.
+// A warp of its own does that beside the rows' scans.
+template <bool kFew>
+__global__ void __launch_bounds__(kThreads + (kFew ? 32 : 0))
 prefix_apply(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
              const DeviceScalars* __restrict__ s, Batch bt, const double4* __restrict__ tiles,
              int ntiles, double4* __restrict__ prefix) {
     chain_begin();
-    __shared__ double4 wtot[kThreads / 32];
+    __shared__ double4 wtot[kThreads / 32], tile_off;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int base = blockIdx.x * kScanTile + warp * kWarpItems + lane;
     const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
     double4 ex[kScanItems];   // exclusive prefix within the row, then within the warp
     double4 carry = zero;     // total of the rows before
+    if (!kFew || warp < kThreads / 32) {
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const int i = base + 32 * k;
-        const double4 v = i < n ? body_term(pos, mass, s, bt, i) : zero;
-        const double4 inc = warp_inclusive_d4(v);
-        double4 e;
-        e.x = __shfl_up_sync(kFull, inc.x, 1);
-        e.y = __shfl_up_sync(kFull, inc.y, 1);
-        e.z = __shfl_up_sync(kFull, inc.z, 1);
-        e.w = 0.0;
-        if (lane == 0) e = zero;
-        ex[k] = d4_add(carry, e);
-        const double4 row = make_double4(__shfl_sync(kFull, inc.x, 31), __shfl_sync(kFull, inc.y, 31),
-                                         __shfl_sync(kFull, inc.z, 31), 0.0);
-        carry = d4_add(carry, row);
+        for (int k = 0; k < kScanItems; ++k) {
+            const int i = base + 32 * k;
+            const double4 v = i < n ? body_term(pos, mass, s, bt, i) : zero;
+            const double4 inc = warp_inclusive_d4(v);
+            double4 e;
+            e.x = __shfl_up_sync(kFull, inc.x, 1);
+            e.y = __shfl_up_sync(kFull, inc.y, 1);
+            e.z = __shfl_up_sync(kFull, inc.z, 1);
+            e.w = 0.0;
+            if (lane == 0) e = zero;
+            ex[k] = d4_add(carry, e);
+            const double4 row = make_double4(__shfl_sync(kFull, inc.x, 31), __shfl_sync(kFull, inc.y, 31),
+                                             __shfl_sync(kFull, inc.z, 31), 0.0);
+            carry = d4_add(carry, row);
+        }
+        if (lane == 0) wtot[warp] = carry;
+    } else {
+        // the scan kernel's sums, association included: lane l adds up tiles
+        // 8 l .. 8 l + 7, the lanes are scanned, the tile's own lane goes on
+        double4 v[kScanItems], run = zero;
+        for (int k = 0; k < kScanItems; ++k) {
+            const int q = lane * kScanItems + k;
+            v[k] = q < ntiles ? tiles[q] : zero;
+            run = d4_add(run, v[k]);
+        }
+        const double4 inc = warp_inclusive_d4(run);
+        double4 acc;
+        acc.x = __shfl_up_sync(kFull, inc.x, 1);
+        acc.y = __shfl_up_sync(kFull, inc.y, 1);
+        acc.z = __shfl_up_sync(kFull, inc.z, 1);
+        acc.w = 0.0;
+        if (lane == 0) acc = zero;
+        if (lane == (int)blockIdx.x / kScanItems) {
+            for (int k = 0; k < (int)blockIdx.x % kScanItems; ++k) acc = d4_add(acc, v[k]);
+            tile_off = acc;
+        }
+        if (lane == 31 && blockIdx.x == ntiles - 1) prefix[n] = inc;
     }
-    if (lane == 0) wtot[warp] = carry;
     __syncthreads();
-    double4 off = tiles[blockIdx.x];
+    if (kFew && warp == kThreads / 32) return;
+    double4 off = kFew ? tile_off : tiles[blockIdx.x];
     for (int w = 0; w < warp; ++w) off = d4_add(off, wtot[w]);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         const int i = base + 32 * k;
         if (i < n) prefix[i] = d4_add(off, ex[k]);
     }
-    if (blockIdx.x == ntiles - 1 && threadIdx.x == 0) prefix[n] = tiles[ntiles];
+    if (!kFew && blockIdx.x == ntiles - 1 && threadIdx.x == 0) prefix[n] = tiles[ntiles];
 }
 
 __device__ void cell_from_prefix(const double4* __restrict__ prefix, const Tree& t,
@@ -1211,7 +1297,7 @@ learned_features(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
 // child that would overflow the group is split instead: the group takes
 // exactly gsize bodies and the child's rest starts the next group.  Multi-body
 // leaves larger than a group are cut into chunks of gsize.  kWrite = false
-// counts the groups of each cell, kWrite = true writes them at gbase[cell].
+// counts the groups of each cell, kWrite = true writes them.
 //
 // Children in key order are quadrants 0..3; 0,1 and 2,3 are the two halves of
 // the cell, while a run that takes quadrants from both halves has the whole
@@ -1224,7 +1310,7 @@ learned_features(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
 // ([ca, cb], leaf marks the leaf children); returns their number and, with
 // kWrite, writes them from out on.
 template <bool kWrite>
-__device__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const int* cb,
+__device__ __forceinline__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const int* cb,
                            const bool* leaf, int gsize, int fill, const Batch& bt,
                            const uint64_t* __restrict__ key, int2* __restrict__ out) {
     int emitted = 0;
@@ -1240,13 +1326,16 @@ __device__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const i
         return emitted;
     }
     bool large = false;  // some child emits its own groups
-    for (int q = 0; q < nc; ++q)
-        large |= cb[q] - ca[q] + 1 > gsize || (bt.nuni && bt.uid[ca[q]] != bt.uid[cb[q]]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        large |= q < nc && (cb[q] - ca[q] + 1 > gsize || (bt.nuni && bt.uid[ca[q]] != bt.uid[cb[q]]));
     // the children differ in digit `level` of their codes; its high bit is
     // the half (read only when a large child makes it matter)
     const int level = large ? min(lcp_digits(key[rg.x], key[rg.y]), 31) : 0;
     int run_a = -1, run_b = -1, run_half = 0;
-    for (int q = 0; q < nc; ++q) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= nc) continue;
         const int a = ca[q], b = cb[q];
         const int cnt = b - a + 1;
         if (cnt > gsize || (bt.nuni && bt.uid[a] != bt.uid[b])) {  // the child emits
@@ -1284,44 +1373,88 @@ __device__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const i
     return emitted;
 }
 
-// Writes every cell's groups at gbase[cell] (the linking pass counted them).
-__global__ void tree_groups_write(int n, int gsize, int fill, Tree t,
-                                  const DeviceScalars* __restrict__ s, Batch bt,
-                                  const uint64_t* __restrict__ key) {
+// Writes the groups, which the linking pass counted, one block per tile: the
+// tile's counts are scanned (each warp 8 rows of 32 cells), and the few cells
+// that have groups (1.5% at 4M) are listed and written one thread each.
+__global__ void __launch_bounds__(kThreads)
+tree_groups_write(int n, int gsize, int fill, Tree t, DeviceScalars* __restrict__ s, Batch bt,
+                  const uint64_t* __restrict__ key, unsigned long long* mark) {
     chain_begin();
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    const int cells = s->cells;
-    if (id >= n) return;
-    if (id >= cells) {
-        if (cells == 0 && id == 0) {  // no cell: the root leaf holds all bodies
-            const int ng = (n + gsize - 1) / gsize;
-            for (int k = 0; k < ng; ++k)
-                t.groups[k] = make_int2(k * gsize, min(n, (k + 1) * gsize) - 1);
-        }
+    mark_start(mark);
+    const int tile = blockIdx.x;
+    if (s->cells == 0) {  // no cell: the root leaf holds all bodies
+        const int ng = (n + gsize - 1) / gsize;
+        for (int k = tile * kThreads + threadIdx.x; k < ng; k += gridDim.x * kThreads)
+            t.groups[k] = make_int2(k * gsize, min(n, (k + 1) * gsize) - 1);
+        if (tile == 0 && threadIdx.x == 0) s->groups = ng;
         return;
     }
-    const int2 rg = t.range[id];
-    const int4 ch = t.child[id];
-    const int refs[4] = {ch.x, ch.y, ch.z, ch.w};
-    int ca[4], cb[4], nc = 0;
-    bool leaf[4];
+    __shared__ int wsum[kThreads / 32], wbefore[kThreads / 32];
+    __shared__ int2 some[kAnsvTile];  // {cell, first group}
+    __shared__ int nsome;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int count = t.tile_count[tile], id0 = t.tile_cells[tile];
+    if (threadIdx.x == 0) nsome = 0;
+    // the groups of the tiles before (at most 8 loads per thread at 4M; a scan
+    // by the linking pass's last block cost its other blocks more in fences)
+    int off = 0;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < tile; q += kThreads) off += t.tile_groups[q];
+    int v[kAnsvItems], ex[kAnsvItems], carry = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int r = refs[q];
-        if (r == INT_MIN) break;
-        leaf[q] = r < 0;
-        if (r >= 0) {
-            const int2 cr = t.range[r];
-            ca[q] = cr.x;
-            cb[q] = cr.y;
-        } else {
-            ca[q] = ~r;
-            cb[q] = t.leaf_last[ca[q]];
-        }
-        nc = q + 1;
+    for (int k = 0; k < kAnsvItems; ++k) {
+        const int j = (warp * kAnsvItems + k) * 32 + lane;
+        v[k] = j < count ? t.gcount[id0 + j] : 0;
     }
-    cell_groups<true>(rg, id == s->root, nc, ca, cb, leaf, gsize, fill, bt, key,
-                      t.groups + t.gbase[id]);
+#pragma unroll
+    for (int k = 0; k < kAnsvItems; ++k) {
+        const int inc = warp_inclusive(v[k]);
+        ex[k] = carry + inc - v[k];
+        carry += __shfl_sync(kFull, inc, 31);
+    }
+    off = __reduce_add_sync(kFull, off);
+    if (lane == 0) {
+        wsum[warp] = carry;
+        wbefore[warp] = off;
+    }
+    __syncthreads();
+    off = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+        off += wbefore[w];
+        if (w < warp) off += wsum[w];
+    }
+    if (tile == gridDim.x - 1 && threadIdx.x == kThreads - 1) s->groups = off + carry;
+#pragma unroll
+    for (int k = 0; k < kAnsvItems; ++k)
+        if (v[k])
+            some[atomicAdd(&nsome, 1)] =
+                make_int2(id0 + (warp * kAnsvItems + k) * 32 + lane, off + ex[k]);
+    __syncthreads();
+    for (int q = threadIdx.x; q < nsome; q += kThreads) {
+        const int id = some[q].x;
+        const int2 rg = t.range[id];
+        const int4 ch = t.child[id];
+        const int refs[4] = {ch.x, ch.y, ch.z, ch.w};
+        int ca[4], cb[4], nc = 0;
+        bool leaf[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int r = refs[c];
+            if (r == INT_MIN) break;
+            leaf[c] = r < 0;
+            if (r >= 0) {
+                const int2 cr = t.range[r];
+                ca[c] = cr.x;
+                cb[c] = cr.y;
+            } else {
+                ca[c] = ~r;
+                cb[c] = t.leaf_last[ca[c]];
+            }
+            nc = c + 1;
+        }
+        cell_groups<true>(rg, id == s->root, nc, ca, cb, leaf, gsize, fill, bt, key,
+                          t.groups + some[q].y);
+    }
 }
 
 // Root reference of each universe: the cell whose body range is exactly the
@@ -1340,7 +1473,7 @@ __global__ void batch_roots(const uint64_t* __restrict__ key, Tree t, Batch bt) 
         bt.root[u] = ~a;
         return;
     }
-    bt.root[u] = t.cell_of[gallop_right(key, a, b, c + 1)];
+    bt.root[u] = cell_id(t, gallop_right(key, a, b, c + 1));
 }
 
 inline unsigned blocks_for(int64_t n, int threads) {
@@ -1356,25 +1489,15 @@ void launch_batch_roots(nb_ctx* c) {
                  c->sort.key[0], c->tree, c->batch);
 }
 
-// chained: the kernel before is the linking pass, on the same stream
-void launch_groups(nb_ctx* c, bool chained) {
-    const int n = (int)c->n;
-    const int sblocks = (int)blocks_for(n, kScanTile);
-    c->launches += 4;
-    const int gsize = split_group_size(c);
+void launch_groups(nb_ctx* c) {
+    c->launches += 1;
     // plain SPLIT fills groups to gsize bodies across sibling cells (fuller
     // warps, measured 2.6% off the walk at 4M with slightly lower errors); the
     // learned correction keeps groups of whole cells, whose residuals it fits.
-    // The linking pass counted every cell's groups; scan, then write them.
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
-    chain_launch(c->stream, chained, scan_reduce, sblocks, kThreads, 0, 1, c->tree.gcount, n,
-                 c->scan.block_sums, mark_of(c, 6));
-    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, 1, c->scan.block_sums, sblocks,
-                 &c->scal->groups);
-    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, 1, c->tree.gcount, n,
-                 c->scan.block_sums, c->tree.gbase, nullptr);
-    chain_launch(c->stream, true, tree_groups_write, blocks_for(n, kThreads), kThreads, 0, 1, n, gsize,
-                 fill, c->tree, c->scal, c->batch, c->sort.key[0]);
+    chain_launch(c->stream, true, tree_groups_write, blocks_for(c->n, kAnsvTile), kThreads, 0, 1,
+                 (int)c->n, split_group_size(c), fill, c->tree, c->scal, c->batch, c->sort.key[0],
+                 mark_of(c, 6));
 }
 
 // SPLIT without quadrupoles takes its monopoles from prefix sums over the
@@ -1393,47 +1516,43 @@ static float split_accept_scale(const nb_ctx* c) {
 
 void launch_prefix_sums(nb_ctx* c, const BodyBuffers& b) {
     if (!mono_prefix(c)) return;
-    const int n = (int)c->n;
-    {  // the prefix sums need only the sorted bodies
-        const int ptiles = (int)blocks_for(n, kScanTile);
-        c->launches += 3;
-        chain_launch(c->stream, true, prefix_reduce, ptiles, kThreads, 0, 1, b.pos, b.mass, n, c->scal,
-                     c->batch, c->tree.prefix_tiles, mark_of(c, 3));
+    const int n = (int)c->n, ptiles = (int)blocks_for(n, kScanTile);
+    const bool few = ptiles <= kFewSums;
+    c->launches += few ? 2 : 3;
+    chain_launch(c->stream, true, prefix_reduce, ptiles, kThreads, 0, 1, b.pos, b.mass, n, c->scal,
+                 c->batch, c->tree.prefix_tiles, mark_of(c, 3));
+    if (!few)
         chain_launch(c->stream, true, prefix_tiles_scan, 1, kThreads, 0, 1, c->tree.prefix_tiles,
                      ptiles);
-        chain_launch(c->stream, true, prefix_apply, ptiles, kThreads, 0, 1, b.pos, b.mass, n, c->scal,
-                     c->batch, c->tree.prefix_tiles, ptiles, c->tree.prefix);
-    }
+    chain_launch(c->stream, true, few ? prefix_apply<true> : prefix_apply<false>, ptiles,
+                 kThreads + (few ? 32 : 0), 0, 1, b.pos, b.mass, n, c->scal, c->batch, c->tree.prefix_tiles, ptiles,
+                 c->tree.prefix);
 }
 
-void launch_tree(nb_ctx* c, const BodyBuffers& b, bool prefix_done) {
+void launch_tree(nb_ctx* c, const BodyBuffers& b) {
     const int n = (int)c->n;
     const bool mono = mono_prefix(c);
-    if (mono && !prefix_done) launch_prefix_sums(c, b);
     const uint64_t* key = c->sort.key[0];
     Tree& t = c->tree;
     const int tiles = (int)blocks_for(n, kAnsvTile);
-    c->launches += 8;
-    chain_launch(c->stream, true, tree_lcp, tiles, kThreads, 0, 1, key, n, tiles, t.lcp8, t.ansv_first,
-                 t.ansv_last, c->scal->lcp_hist, mark_of(c, 4));
-    chain_launch(c->stream, true, tree_ansv_tiles, kAnsvLevels, kTileScanThreads, 0, 1, tiles,
-                 t.ansv_first, t.ansv_last);
-    chain_launch(c->stream, true, tree_ansv, tiles, kThreads, 0, 1, t.lcp8, n, tiles, t.ansv_first,
-                 t.ansv_last, t.flag, t.bnd);
-    const int sblocks = (int)blocks_for(n, kScanTile);
-    chain_launch(c->stream, true, scan_reduce, sblocks, kThreads, 0, 1, t.flag, n, c->scan.block_sums,
-                 nullptr);
-    chain_launch(c->stream, true, scan_block_sums, 1, kSumsThreads, 0, 1, c->scan.block_sums, sblocks,
-                 &c->scal->cells);
-    chain_launch(c->stream, true, scan_apply, sblocks, kThreads, 0, 1, t.flag, n, c->scan.block_sums,
-                 t.cell_of, t.rep_of);
+    const bool few = tiles <= kFewTiles;
+    c->launches += few ? 3 : 4;
+    const TileTable tab{t.ansv_first, t.ansv_last, few ? 1 : tiles, few ? kAnsvLevels : 1};
+    const bool wide = tiles <= kWideTiles;
+    chain_launch(c->stream, true, wide ? tree_lcp<kWideThreads> : tree_lcp<kThreads>, tiles,
+                 wide ? kWideThreads : kThreads, 0, 1, key, n, t.lcp8, tab, c->scal->lcp_hist,
+                 mark_of(c, 4));
+    if (!few)
+        chain_launch(c->stream, true, tree_ansv_tiles, kAnsvLevels, kTileScanThreads, 0, 1, tiles,
+                     t.ansv_first, t.ansv_last);
+    chain_launch(c->stream, true, wide ? tree_ansv<kWideThreads> : tree_ansv<kThreads>, tiles,
+                 wide ? kWideThreads : kThreads, 0, 1, t, n, tiles, tab, c->scal);
     // SPLIT: the cells count their target groups as they link
     const int gsize = c->p.mode == NB_MODE_SPLIT ? split_group_size(c) : 0;
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
-    chain_launch(c->stream, true, mono ? tree_link<true> : tree_link<false>, blocks_for(n, kThreads),
-                 kThreads, 0, 1, key, t.lcp8, n, b.pos, b.mass, t, c->scal, mono ? t.prefix : nullptr,
+    chain_launch(c->stream, true, mono ? tree_link<true> : tree_link<false>, tiles * kLinkBlocks,
+                 kThreads, 0, 1, key, n, b.pos, b.mass, t, c->scal, mono ? t.prefix : nullptr,
                  c->batch, mono ? split_accept_scale(c) : 0.f, gsize, fill);
-    chain_launch(c->stream, true, tree_trivial_root, 1, 1, 0, 1, b.pos, b.mass, n, t, c->scal, gsize);
 }
 
 void launch_features(nb_ctx* c, const BodyBuffers& b, bool chained) {

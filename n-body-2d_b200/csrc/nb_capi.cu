@@ -79,8 +79,6 @@ int alloc_all(nb_ctx* c) {
     }
     NB_CUDA(c, dalloc(&c->sort.ties_small, n / 2 + 1));
     NB_CUDA(c, dalloc(&c->sort.ties_big, n / 33 + 1));
-    c->scan.blocks = (int)((n + 2047) / 2048);
-    NB_CUDA(c, dalloc(&c->scan.block_sums, (size_t)c->scan.blocks));
     nb::Tree& t = c->tree;
     NB_CUDA(c, dalloc(&t.level, n));
     NB_CUDA(c, dalloc(&t.child, n));
@@ -99,7 +97,6 @@ int alloc_all(nb_ctx* c) {
         NB_CUDA(c, dalloc(&t.s32, n));
         NB_CUDA(c, dalloc(&t.body4, n));
         NB_CUDA(c, dalloc(&t.gcount, n));
-        NB_CUDA(c, dalloc(&t.gbase, n));
         NB_CUDA(c, dalloc(&t.groups, n));
         NB_CUDA(c, dalloc(&t.prefix, n + 1));
         NB_CUDA(c, dalloc(&t.prefix_tiles, (n + 2047) / 2048 + 1));
@@ -117,13 +114,15 @@ int alloc_all(nb_ctx* c) {
     NB_CUDA(c, dalloc(&t.leaf_plevel, n));
     NB_CUDA(c, dalloc(&t.bucket_mass, n));
     NB_CUDA(c, dalloc(&t.bucket_com, n));
-    NB_CUDA(c, dalloc(&t.flag, n));
-    NB_CUDA(c, dalloc(&t.cell_of, n));
-    NB_CUDA(c, dalloc(&t.rep_of, n));
+    NB_CUDA(c, dalloc(&t.cell_rank, n));
+    NB_CUDA(c, dalloc(&t.rep, n));
     NB_CUDA(c, dalloc(&t.bnd, n));
     NB_CUDA(c, dalloc(&t.lcp8, n));
     {
         const size_t tiles = (n + nb::kAnsvTile - 1) / nb::kAnsvTile;
+        NB_CUDA(c, dalloc(&t.tile_count, tiles));
+        NB_CUDA(c, dalloc(&t.tile_cells, tiles));
+        if (c->p.mode == NB_MODE_SPLIT) NB_CUDA(c, dalloc(&t.tile_groups, tiles));
         NB_CUDA(c, dalloc(&t.ansv_first, tiles * nb::kAnsvLevels));
         NB_CUDA(c, dalloc(&t.ansv_last, tiles * nb::kAnsvLevels));
     }
@@ -152,13 +151,13 @@ void free_all(nb_ctx* c) {
     cudaFree(c->sort.tile_counter);
     cudaFree(c->sort.ties_small);
     cudaFree(c->sort.ties_big);
-    cudaFree(c->scan.block_sums);
     nb::Tree& t = c->tree;
     void* tree_ptrs[] = {t.level,       t.child,      t.parent,
                          t.nint,      t.ready,       t.mass,        t.com,        t.leaf_last,
-                         t.leaf_plevel, t.bucket_mass, t.bucket_com, t.flag,      t.cell_of,
+                         t.leaf_plevel, t.bucket_mass, t.bucket_com, t.cell_rank, t.tile_count, t.tile_cells,
+                         t.tile_groups,
                          t.bnd,       t.range,       t.s64,         t.cell4,      t.cellq,      t.s32,
-                         t.body4,     t.gcount,      t.gbase,       t.groups,     t.rep_of,
+                         t.body4,     t.gcount,      t.groups,     t.rep,
                          t.t32,       t.cellh,       t.band,        t.band_count,
                          t.prefix, t.prefix_tiles, t.lcp8, t.ansv_first,
                          t.ansv_last};
@@ -252,34 +251,25 @@ void enqueue_step(nb_ctx* c, int parity, bool integrate, bool store_acc, bool ti
     const bool split = c->p.mode == NB_MODE_SPLIT;
     nb::launch_gather(c, A, B, split ? c->tree.body4 : nullptr);
     nb::launch_prefix_sums(c, B);  // SPLIT monopoles only
-    nb::launch_tree(c, B, true);
+    nb::launch_tree(c, B);
     nb::launch_batch_roots(c);
-    // the target groups need only the tree: with quadrupoles, whose moments
-    // climb the tree, they are built on the side stream meanwhile (two branches
-    // of the captured graph)
-    const bool fork = split && (c->p.flags & NB_FLAG_QUADRUPOLE);
-    auto on_side = [&](cudaEvent_t forked, cudaEvent_t joined, auto&& launch) {
-        cudaEventRecord(forked, c->stream);
-        cudaStreamWaitEvent(c->side_stream, forked, 0);
-        cudaStream_t main_stream = c->stream;
-        c->stream = c->side_stream;
-        launch();
-        c->stream = main_stream;
-        cudaEventRecord(joined, c->side_stream);
-    };
-    if (fork) on_side(c->fork_ev, c->join_ev, [&] { nb::launch_groups(c, false); });
-    else if (split) nb::launch_groups(c, true);
+    if (split) nb::launch_groups(c);
     nb::launch_moments(c, B, split);
-    if (fork) cudaStreamWaitEvent(c->stream, c->join_ev, 0);
     if (split && (c->p.flags & NB_FLAG_LEARNED)) {
         // the features need only the monopoles, and only the correction reads
         // them: they are built on the side stream while the walk runs
-        on_side(c->feat_fork_ev, c->feat_join_ev, [&] { nb::launch_features(c, B, false); });
+        cudaEventRecord(c->feat_fork_ev, c->stream);
+        cudaStreamWaitEvent(c->side_stream, c->feat_fork_ev, 0);
+        cudaStream_t main_stream = c->stream;
+        c->stream = c->side_stream;
+        nb::launch_features(c, B, false);
+        c->stream = main_stream;
+        cudaEventRecord(c->feat_join_ev, c->side_stream);
         nb::launch_force_split(c, B, integrate, store_acc, false);  // FP32 accelerations + band lists
         cudaStreamWaitEvent(c->stream, c->feat_join_ev, 0);
         nb::launch_mlp_correct(c, B, integrate, store_acc);  // learned term, kick, drift
     } else if (split) {
-        nb::launch_force_split(c, B, integrate, store_acc, !fork);  // kick and drift fused
+        nb::launch_force_split(c, B, integrate, store_acc, true);  // kick and drift fused
     } else {
         nb::launch_force_fp64(c, B, integrate, store_acc);
         if (integrate) nb::launch_drift(c, B);
@@ -291,7 +281,7 @@ void enqueue_step(nb_ctx* c, int parity, bool integrate, bool store_acc, bool ti
 unsigned active_phases(const nb_ctx* c) {
     if (c->p.mode == NB_MODE_ALLPAIRS) return 1u << 7;
     if (c->p.mode == NB_MODE_FP64) return 1u | 2u | 4u | 16u | 32u | 128u | 256u;
-    // with quadrupoles the groups are built while the moments run, as part of them
+    // (with quadrupoles the groups come before the moments, as part of the tree)
     unsigned a = 1u | 2u | 4u | 16u | 128u;
     a |= (c->p.flags & NB_FLAG_QUADRUPOLE) ? 32u : 8u | 64u;
     if (c->p.flags & NB_FLAG_LEARNED) a |= 256u;
@@ -429,8 +419,6 @@ int create_context(const nb_params* p, uint64_t n, const double* mass, const dou
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->feat_fork_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->feat_join_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->staged, cudaEventDisableTiming) != cudaSuccess ||
@@ -485,8 +473,6 @@ int nb_destroy(nb_ctx* c) {
     if (c->staged) cudaEventDestroy(c->staged);
     if (c->copied) cudaEventDestroy(c->copied);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
-    if (c->fork_ev) cudaEventDestroy(c->fork_ev);
-    if (c->join_ev) cudaEventDestroy(c->join_ev);
     if (c->feat_fork_ev) cudaEventDestroy(c->feat_fork_ev);
     if (c->feat_join_ev) cudaEventDestroy(c->feat_join_ev);
     if (c->side_stream) cudaStreamDestroy(c->side_stream);
@@ -997,10 +983,11 @@ int nb_mlp_samples(nb_ctx* c, uint64_t ntargets, uint64_t seed, uint64_t capacit
     nb::launch_morton(c, A.pos);
     nb::launch_sort(c);
     nb::launch_gather(c, A, B, c->tree.body4);
+    nb::launch_prefix_sums(c, B);
     nb::launch_tree(c, B);
     nb::launch_moments(c, B, true);
+    nb::launch_groups(c);
     nb::launch_features(c, B, true);
-    nb::launch_groups(c, true);
     NB_CUDA(c, cudaGetLastError());
     c->parity ^= 1;
     // target groups: a seeded uniform choice (splitmix64), reduced modulo the

@@ -45,7 +45,7 @@ struct DeviceScalars {
     unsigned long long body_terms;
     int32_t stack_hw;         // FP64 walk: deepest stack (entries) of the last force pass
     int32_t stack_pad_;
-    int32_t pad2_;
+    unsigned tile_ticket;     // last-block-done counter of the tree kernels
     unsigned upload_bad;      // nb_upload's checks: bit 0 non-finite, bit 1 mass <= 0
     // Radix sort over the top sort_passes bytes of the keys only (1..8), chosen
     // per step from the previous tree's histogram of shared leading digits of
@@ -126,7 +126,6 @@ struct Tree {
     // SPLIT target groups: <= split_group_size() Morton-consecutive bodies in one
     // parent cell (merged sibling cells/leaves), stored as body ranges
     int32_t* gcount = nullptr;   // groups each cell emits
-    int32_t* gbase = nullptr;    // exclusive scan of gcount
     int2* groups = nullptr;      // {first, last} body of each group
     // per-body side tables, only meaningful at leaf starts
     int32_t* leaf_last = nullptr;   // last body of the leaf starting here
@@ -135,9 +134,11 @@ struct Tree {
     double2* bucket_com = nullptr;
     // build scratch (per boundary i between bodies i and i+1)
     uint8_t* lcp8 = nullptr;        // level of boundary i: shared leading digits, capped at 30
-    int32_t* flag = nullptr;
-    int32_t* cell_of = nullptr;     // exclusive scan of flag
-    int32_t* rep_of = nullptr;      // cell id -> the boundary that creates it
+    uint16_t* cell_rank = nullptr;  // cells created by the boundaries before, in the tile
+    uint16_t* rep = nullptr;        // per tile: the boundaries (in it) that create its cells
+    int32_t* tile_count = nullptr;  // per tile: cells created in it
+    int32_t* tile_cells = nullptr;  //   and in the tiles before
+    int32_t* tile_groups = nullptr; // SPLIT, per tile: groups of its cells
     int4* bnd = nullptr;            // per boundary: {first body, last body} of the cell it
                                     // creates (flagged boundaries only), {previous, next}
                                     // separator of its cell or -1
@@ -156,11 +157,6 @@ struct SortBuffers {
     int tiles = 0;
 };
 
-struct ScanBuffers {
-    int32_t* block_sums = nullptr;
-    int blocks = 0;
-};
-
 }  // namespace nb
 
 struct nb_ctx {
@@ -171,8 +167,7 @@ struct nb_ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaStream_t copy_stream = nullptr;  // nb_download_async: device-to-host copies
-    cudaStream_t side_stream = nullptr;  // the target groups, built while the moments run
-    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+    cudaStream_t side_stream = nullptr;  // the learned features, built while the walk runs
     cudaEvent_t feat_fork_ev = nullptr, feat_join_ev = nullptr;  // learned features beside the walk
     cudaEvent_t staged = nullptr;        // the download's scatter into the staging buffers is done
     cudaEvent_t copied = nullptr;        // the staging buffers have been copied out (free again)
@@ -181,7 +176,6 @@ struct nb_ctx {
     int parity = 0;                 // which BodyBuffers holds the state
     nb::BodyBuffers buf[2];
     nb::SortBuffers sort;
-    nb::ScanBuffers scan;
     nb::Tree tree;
     nb::DeviceScalars* scal = nullptr;   // device
     double* bbox_partials = nullptr;     // [blocks][4]
@@ -363,10 +357,10 @@ void launch_batch_roots(nb_ctx* c);   // per-universe root cells after the tree 
 void launch_sort(nb_ctx* c);
 unsigned sort_timeout_probe(cudaStream_t st);                                   // result in key[0]/val[0]
 void launch_gather(nb_ctx* c, const BodyBuffers& src, const BodyBuffers& dst, float4* body4);
-// SPLIT monopoles: the prefix sums over the sorted bodies (nothing in other
-// modes); launch_tree runs them itself unless prefix_done.
+// SPLIT monopoles (nothing in other modes): the prefix sums over the sorted
+// bodies, which launch_tree reads.
 void launch_prefix_sums(nb_ctx* c, const BodyBuffers& b);
-void launch_tree(nb_ctx* c, const BodyBuffers& b, bool prefix_done = false);
+void launch_tree(nb_ctx* c, const BodyBuffers& b);
 void launch_moments(nb_ctx* c, const BodyBuffers& b, bool split);
 // learned mode: second and third moments and the BF16 feature records
 void launch_features(nb_ctx* c, const BodyBuffers& b, bool chained);
@@ -388,7 +382,7 @@ size_t mlp_train_image_bytes();
 int mlp_grad_tc_device(const float* params, const float* X, const float* Yt, const int64_t* idx,
                        int64_t n, float* grad, float* loss, void* image, unsigned* err,
                        int sm_count, cudaStream_t st);
-void launch_groups(nb_ctx* c, bool chained);
+void launch_groups(nb_ctx* c);
 void launch_force_split(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc, bool chained);
 void launch_force_fp64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc);
 void launch_drift(nb_ctx* c, const BodyBuffers& b);
