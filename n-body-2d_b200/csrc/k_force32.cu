@@ -185,44 +185,54 @@ __device__ __forceinline__ void fold_block(WarpLists& L, float2* ax, float2* ay)
     }
 }
 
-// Sum the first npairs pairs of the cell list.
-template <bool kQuad, bool kZeroSoft, int kBPL>
-__device__ __forceinline__ void sum_cells(WarpLists& L, int npairs, const float2* nx,
-                                          const float2* ny, const float2 e2, float2* ax,
-                                          float2* ay, bool fold) {
-    if (npairs == 16) {
+// Which entries a lane takes: pairs slot, slot + slots, ...  Groups of 17 or
+// more bodies have a lane for each body (slots = 1); smaller groups give each
+// body 2 or 4 lanes, whose sums are added at the end.
+struct Slots {
+    int slot, slots;
+};
+
+// The first npairs pairs of the cell list (kCells) or the body list against
+// the lane's first kN bodies.
+template <bool kCells, bool kQuad, bool kZeroSoft, int kN>
+__device__ __forceinline__ void sum_pairs(const WarpLists& L, int npairs, Slots sl, const float2* nx,
+                                          const float2* ny, const float2 e2, float2* ax, float2* ay) {
+    auto pair = [&](int k) {
+        if (kCells && kQuad)
+            quad_pair<kZeroSoft, kN>(L.cxy[k], L.cm[k], L.qa[k], L.qb[k], nx, ny, e2, ax, ay);
+        else if (kCells)
+            mono_pair<kZeroSoft, kN>(L.cxy[k], L.cm[k], nx, ny, e2, ax, ay);
+        else
+            mono_pair<kZeroSoft, kN>(L.bxy[k], L.bm[k], nx, ny, e2, ax, ay);
+    };
+    if (kN > 1) {
+        if (npairs == 16) {
 #pragma unroll 4
-        for (int k = 0; k < 16; ++k) {
-            if (kQuad)
-                quad_pair<kZeroSoft, kBPL>(L.cxy[k], L.cm[k], L.qa[k], L.qb[k], nx, ny, e2, ax,
-                                           ay);
-            else
-                mono_pair<kZeroSoft, kBPL>(L.cxy[k], L.cm[k], nx, ny, e2, ax, ay);
+            for (int k = 0; k < 16; ++k) pair(k);
+        } else {
+            for (int k = 0; k < npairs; ++k) pair(k);
+        }
+    } else if (npairs == 16) {
+        for (int k = sl.slot; k < 16; k += 4 * sl.slots) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) pair(k + q * sl.slots);
         }
     } else {
-        for (int k = 0; k < npairs; ++k) {
-            if (kQuad)
-                quad_pair<kZeroSoft, kBPL>(L.cxy[k], L.cm[k], L.qa[k], L.qb[k], nx, ny, e2, ax,
-                                           ay);
-            else
-                mono_pair<kZeroSoft, kBPL>(L.cxy[k], L.cm[k], nx, ny, e2, ax, ay);
-        }
+        for (int k = sl.slot; k < npairs; k += sl.slots) pair(k);
     }
-    if (fold) fold_block<kBPL>(L, ax, ay);
 }
 
-template <bool kZeroSoft, int kBPL>
-__device__ __forceinline__ void sum_bodies(WarpLists& L, int npairs, const float2* nx,
-                                           const float2* ny, const float2 e2, float2* ax,
-                                           float2* ay, bool fold) {
-    if (npairs == 16) {
-#pragma unroll 4
-        for (int k = 0; k < 16; ++k)
-            mono_pair<kZeroSoft, kBPL>(L.bxy[k], L.bm[k], nx, ny, e2, ax, ay);
-    } else {
-        for (int k = 0; k < npairs; ++k)
-            mono_pair<kZeroSoft, kBPL>(L.bxy[k], L.bm[k], nx, ny, e2, ax, ay);
-    }
+// kBPL bodies per lane, or one where the group has no more bodies than lanes:
+// a quarter of the groups of up to 64 bodies have 32 or fewer, and the pair
+// terms of empty places were a sixth of all.
+template <bool kCells, bool kQuad, bool kZeroSoft, int kBPL>
+__device__ __forceinline__ void sum_list(WarpLists& L, int npairs, bool one, Slots sl,
+                                         const float2* nx, const float2* ny, const float2 e2,
+                                         float2* ax, float2* ay, bool fold) {
+    if (kBPL == 1 || one)
+        sum_pairs<kCells, kQuad, kZeroSoft, 1>(L, npairs, sl, nx, ny, e2, ax, ay);
+    else
+        sum_pairs<kCells, kQuad, kZeroSoft, kBPL>(L, npairs, sl, nx, ny, e2, ax, ay);
     if (fold) fold_block<kBPL>(L, ax, ay);
 }
 
@@ -230,7 +240,8 @@ __device__ __forceinline__ void sum_bodies(WarpLists& L, int npairs, const float
 // g0 + l, g0 + 32 + l, ...) and accumulate the FP32 accelerations.
 template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft>
 __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root, int n, int g0,
-                                           int g1, const float* px, const float* py,
+                                           int g1, bool one, Slots sl, const float* px,
+                                           const float* py,
                                            const bool* act_body, float eps2, float theta2,
                                            int leaf_size, float* ax, float* ay,
                                            unsigned long long& ncell, unsigned long long& npair,
@@ -333,8 +344,8 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
         ccount += __popc(acc_mask);
         __syncwarp();
         if (ccount >= 32) {
-            sum_cells<kQuad, kZeroSoft, kBPL>(L, 16, nx, ny, e2, ax2, ay2,
-                                              ++flushes % kFoldFlushes == 0);
+            sum_list<true, kQuad, kZeroSoft, kBPL>(L, 16, one, sl, nx, ny, e2, ax2, ay2,
+                                                   ++flushes % kFoldFlushes == 0);
             ncell += 32;
             __syncwarp();
             // pairs 16.. move down; source and destination never overlap
@@ -388,8 +399,8 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
             bcount += added;
             __syncwarp();
             if (bcount >= 32) {
-                sum_bodies<kZeroSoft, kBPL>(L, 16, nx, ny, e2, ax2, ay2,
-                                            ++flushes % kFoldFlushes == 0);
+                sum_list<false, false, kZeroSoft, kBPL>(L, 16, one, sl, nx, ny, e2, ax2, ay2,
+                                                        ++flushes % kFoldFlushes == 0);
                 npair += 32;
                 __syncwarp();
                 if (lane < (bcount - 31) / 2) {
@@ -410,8 +421,8 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
         if (bcount & 1) put_entry(L.bxy, L.bm, bcount, kPadCoord, kPadCoord, 0.f);
     }
     __syncwarp();
-    sum_cells<kQuad, kZeroSoft, kBPL>(L, (ccount + 1) >> 1, nx, ny, e2, ax2, ay2, false);
-    sum_bodies<kZeroSoft, kBPL>(L, (bcount + 1) >> 1, nx, ny, e2, ax2, ay2, true);
+    sum_list<true, kQuad, kZeroSoft, kBPL>(L, (ccount + 1) >> 1, one, sl, nx, ny, e2, ax2, ay2, false);
+    sum_list<false, false, kZeroSoft, kBPL>(L, (bcount + 1) >> 1, one, sl, nx, ny, e2, ax2, ay2, true);
     ncell += ccount;
     npair += bcount;
 #pragma unroll
@@ -420,13 +431,23 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
         ax[b] = tx.x + tx.y;
         ay[b] = ty.x + ty.y;
     }
+    // the lanes that share a body
+    for (int o = 32 / sl.slots; o < 32; o <<= 1) {
+        ax[0] += __shfl_xor_sync(kFull, ax[0], o);
+        ay[0] += __shfl_xor_sync(kFull, ay[0], o);
+    }
     __syncwarp();
 }
 
 // Persistent: each warp takes groups from a global ticket until none is left,
 // which balances groups of very different cost.
+// Blocks per SM that the walk needs to hide its loads (registers are held to
+// what they leave: 64 and 72).
+template <bool kQuad, int kBPL>
+constexpr int kMinBlocks = kBPL == 4 ? 4 : kQuad && kBPL == 2 ? 7 : 8;
+
 template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocks<kQuad, kBPL>)
 force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __restrict__ acc_out,
             float2* __restrict__ acc32, int n, Tree t, DeviceScalars* __restrict__ s, Batch bt,
             float eps2, float theta2, int leaf_size, double G_dt, double dt, int kick,
@@ -449,22 +470,25 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
         const int root = bt.nuni ? bt.root[bt.uid[g0]] : s->root;
         const double2 fc = frame_center(s, bt, g0);
         const double cx = fc.x, cy = fc.y;
+        const int count = g1 - g0 + 1;
+        const int width = count > 16 ? 32 : count > 8 ? 16 : 8;  // lanes for the first bodies
+        const Slots sl{lane / width, 32 / width};
+        const int place = lane & (width - 1);
         int me[kBPL];
         bool on[kBPL];
         float px[kBPL], py[kBPL], ax[kBPL], ay[kBPL];
-        double2 P[kBPL];
 #pragma unroll
         for (int b = 0; b < kBPL; ++b) {
-            on[b] = g0 + 32 * b + lane <= g1;
-            me[b] = min(g0 + 32 * b + lane, g1);
-            P[b] = pos[me[b]];
-            px[b] = (float)(P[b].x - cx);
-            py[b] = (float)(P[b].y - cy);
+            on[b] = 32 * b + place < count;
+            me[b] = min(g0 + 32 * b + place, g1);
+            const double2 p = pos[me[b]];
+            px[b] = (float)(p.x - cx);
+            py[b] = (float)(p.y - cy);
         }
         unsigned long long ncell, npair;
         int nband = 0;
         int* band = kLearned ? t.band + (int64_t)kBandPerBody * g0 : nullptr;
-        walk_group<kQuad, kBPL, kLearned, kZeroSoft>(L, t, root, n, g0, g1, px, py, on, eps2, theta2,
+        walk_group<kQuad, kBPL, kLearned, kZeroSoft>(L, t, root, n, g0, g1, count <= 32, sl, px, py, on, eps2, theta2,
                                           leaf_size, ax, ay, ncell, npair, &s->error, band, nband,
                                           kBandPerBody * (g1 - g0 + 1), band2);
         if (kLearned) {
@@ -472,11 +496,11 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
             if (lane == 0) t.band_count[g] = nband;
 #pragma unroll
             for (int b = 0; b < kBPL; ++b)
-                if (on[b]) acc32[me[b]] = make_float2(ax[b], ay[b]);
+                if (on[b] && sl.slot == 0) acc32[me[b]] = make_float2(ax[b], ay[b]);
         }
 #pragma unroll
         for (int b = 0; b < kBPL; ++b) {
-            if (kLearned || !on[b]) continue;
+            if (kLearned || !on[b] || sl.slot > 0) continue;
             const int i = me[b];
             if (acc_out) acc_out[i] = make_double2((double)ax[b], (double)ay[b]);
             if (kick) {
@@ -484,7 +508,7 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
                 v.x += (double)ax[b] * G_dt;
                 v.y += (double)ay[b] * G_dt;
                 vel[i] = v;
-                double2 p = P[b];
+                double2 p = pos[i];  // (read again: not held over the walk)
                 p.x += v.x * dt;
                 p.y += v.y * dt;
                 pos[i] = p;
