@@ -185,9 +185,10 @@ __device__ __forceinline__ void fold_block(WarpLists& L, float2* ax, float2* ay)
     }
 }
 
-// Which entries a lane takes: pairs slot, slot + slots, ...  Groups of 17 or
-// more bodies have a lane for each body (slots = 1); smaller groups give each
-// body 2 or 4 lanes, whose sums are added at the end.
+// Which entries a lane takes: pairs slot, slot + slots, ...  A lane for each
+// body takes them all (slots = 1); where a block shares a group (kShare), a
+// group of 16 or 8 bodies gives each 2 or 4 lanes, whose sums are added at the
+// end.
 struct Slots {
     int slot, slots;
 };
@@ -238,7 +239,14 @@ __device__ __forceinline__ void sum_list(WarpLists& L, int npairs, bool one, Slo
 
 // Walk the tree for one group [g0, g1] of <= 32 kBPL bodies (lane l owns
 // g0 + l, g0 + 32 + l, ...) and accumulate the FP32 accelerations.
-template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft>
+// kShare: the block's warps walk for the same group.  Each opens the top of the
+// tree until its stack holds kShareAt nodes, from which warp `part` then keeps
+// every kWarpsPerBlock-th; what is accepted or summed directly before that counts
+// in the first warp only.
+constexpr int kShareAt = 24;
+static_assert(kShareAt <= 32 && kWarpsPerBlock == 4, "a warp's part of the stack fits its lanes");
+
+template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft, bool kShare>
 __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root, int n, int g0,
                                            int g1, bool one, Slots sl, const float* px,
                                            const float* py,
@@ -246,7 +254,7 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
                                            int leaf_size, float* ax, float* ay,
                                            unsigned long long& ncell, unsigned long long& npair,
                                            unsigned* err, int* band, int& nband, int band_cap,
-                                           float band2) {
+                                           float band2, int part) {
     const int lane = threadIdx.x & 31;
     float bx0 = INFINITY, bx1 = -INFINITY, by0 = INFINITY, by1 = -INFINITY;
 #pragma unroll
@@ -280,6 +288,7 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
     for (int b = 0; b < kBPL; ++b) L.tot[2 * b][lane] = L.tot[2 * b + 1][lane] = make_float2(0.f, 0.f);
     int ccount = 0, bcount = 0, size = 1;
     int flushes = 0;  // warp-uniform: every lane takes part in every flush
+    bool shared_top = kShare;
     if (lane == 0) L.stack[0] = root;
     __syncwarp();
 
@@ -320,6 +329,10 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
                 bfirst = b;
                 bcnt = max(0, min(t.leaf_last[b], n - 1) - b + 1);
             }
+        }
+        if (kShare && shared_top && part > 0 && act != 3) {
+            act = 0;
+            bcnt = 0;
         }
         // accepted cells
         const unsigned acc_mask = __ballot_sync(kFull, act == 1);
@@ -377,6 +390,16 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
             if (nch > 3) dst[3] = ch.w;
         }
         size += pushed;
+        // (until then a round takes the whole stack, so size < 4 kShareAt)
+        if (kShare && shared_top && size >= kShareAt) {
+            shared_top = false;
+            __syncwarp();
+            const int mine = (size - part + kWarpsPerBlock - 1) / kWarpsPerBlock;
+            const int r0 = lane < mine ? L.stack[part + kWarpsPerBlock * lane] : 0;
+            __syncwarp();
+            if (lane < mine) L.stack[lane] = r0;
+            size = mine;
+        }
         // bodies of directly summed cells and leaves, expanded 32 at a time
         int btot;
         const int boff = warp_exclusive_sum(bcnt, btot);
@@ -446,7 +469,7 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
 template <bool kQuad, int kBPL>
 constexpr int kMinBlocks = kBPL == 4 ? 4 : kQuad && kBPL == 2 ? 7 : 8;
 
-template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft>
+template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft, bool kShare>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocks<kQuad, kBPL>)
 force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __restrict__ acc_out,
             float2* __restrict__ acc32, int n, Tree t, DeviceScalars* __restrict__ s, Batch bt,
@@ -456,13 +479,22 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
     mark_start(mark);
     __shared__ WarpLists lists[kWarpsPerBlock];
     const int lane = threadIdx.x & 31;
+    __shared__ int block_group;
+    const int part = kShare ? threadIdx.x >> 5 : 0;
     WarpLists& L = lists[threadIdx.x >> 5];
     const int ngroups = s->groups;
     unsigned long long cells_total = 0, pairs_total = 0;
     while (true) {
         int g = 0;
-        if (lane == 0) g = (int)atomicAdd(&s->group_ticket, 1u);
-        g = __shfl_sync(kFull, g, 0);
+        if (kShare) {
+            __syncthreads();  // the sums of the last group have been read
+            if (threadIdx.x == 0) block_group = (int)atomicAdd(&s->group_ticket, 1u);
+            __syncthreads();
+            g = block_group;
+        } else {
+            if (lane == 0) g = (int)atomicAdd(&s->group_ticket, 1u);
+            g = __shfl_sync(kFull, g, 0);
+        }
         if (g >= ngroups) break;
         const int2 gr = t.groups[g];
         const int g0 = gr.x, g1 = min(gr.y, n - 1);
@@ -471,8 +503,8 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
         const double2 fc = frame_center(s, bt, g0);
         const double cx = fc.x, cy = fc.y;
         const int count = g1 - g0 + 1;
-        const int width = count > 16 ? 32 : count > 8 ? 16 : 8;  // lanes for the first bodies
-        const Slots sl{lane / width, 32 / width};
+        const int width = !kShare || count > 16 ? 32 : count > 8 ? 16 : 8;
+        const Slots sl = kShare ? Slots{lane / width, 32 / width} : Slots{0, 1};
         const int place = lane & (width - 1);
         int me[kBPL];
         bool on[kBPL];
@@ -488,9 +520,20 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
         unsigned long long ncell, npair;
         int nband = 0;
         int* band = kLearned ? t.band + (int64_t)kBandPerBody * g0 : nullptr;
-        walk_group<kQuad, kBPL, kLearned, kZeroSoft>(L, t, root, n, g0, g1, count <= 32, sl, px, py, on, eps2, theta2,
+        walk_group<kQuad, kBPL, kLearned, kZeroSoft, kShare>(L, t, root, n, g0, g1, count <= 32, sl, px, py, on, eps2, theta2,
                                           leaf_size, ax, ay, ncell, npair, &s->error, band, nband,
-                                          kBandPerBody * (g1 - g0 + 1), band2);
+                                          kBandPerBody * (g1 - g0 + 1), band2, part);
+        if (kShare) {  // the warps' sums, in order
+#pragma unroll
+            for (int b = 0; b < kBPL; ++b) L.tot[b][lane] = make_float2(ax[b], ay[b]);
+            __syncthreads();
+#pragma unroll
+            for (int b = 0; b < kBPL; ++b)
+                for (int w = 1; w < kWarpsPerBlock; ++w) {
+                    ax[b] += lists[w].tot[b][lane].x;
+                    ay[b] += lists[w].tot[b][lane].y;
+                }
+        }
         if (kLearned) {
             // the correction kernel adds the learned term, then kicks and drifts
             if (lane == 0) t.band_count[g] = nband;
@@ -500,7 +543,7 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
         }
 #pragma unroll
         for (int b = 0; b < kBPL; ++b) {
-            if (kLearned || !on[b] || sl.slot > 0) continue;
+            if (kLearned || !on[b] || sl.slot > 0 || part > 0) continue;
             const int i = me[b];
             if (acc_out) acc_out[i] = make_double2((double)ax[b], (double)ay[b]);
             if (kick) {
@@ -517,7 +560,7 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
         // every body of the group summed every entry and skipped itself once
         const unsigned long long bodies = (unsigned long long)(g1 - g0 + 1);
         cells_total += ncell * bodies;
-        pairs_total += npair * bodies - bodies;
+        pairs_total += npair * bodies - (part > 0 ? 0 : bodies);
     }
     if (lane == 0) {
         atomicAdd(&s->cell_terms, cells_total);
@@ -526,16 +569,16 @@ force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __res
     }
 }
 
-template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft>
+template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft, bool kShare>
 void launch_split_soft(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc, bool chained,
                        float eps2) {
     int& grid = c->split_blocks[(kQuad ? 1 : 0) + (kLearned ? 2 : 0) + (kBPL == 1 ? 4 : 0) +
                                 (kBPL == 4 ? 16 : 0) +
-                                (kZeroSoft ? 8 : 0)];
+                                (kZeroSoft ? 8 : 0) + (kShare ? 32 : 0)];
     if (grid == 0) {
         int blocks = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &blocks, force_split<kQuad, kBPL, kLearned, kZeroSoft>, kWarpsPerBlock * 32, 0) !=
+                &blocks, force_split<kQuad, kBPL, kLearned, kZeroSoft, kShare>, kWarpsPerBlock * 32, 0) !=
                     cudaSuccess ||
             blocks < 1)
             blocks = 4;
@@ -543,12 +586,19 @@ void launch_split_soft(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_ac
     }
     const float theta2 = (float)(c->p.theta * c->p.theta);
     const int leaf = c->p.leaf_size > 0 ? c->p.leaf_size : kDefaultLeaf;
-    chain_launch(c->stream, chained, force_split<kQuad, kBPL, kLearned, kZeroSoft>, grid,
+    chain_launch(c->stream, chained, force_split<kQuad, kBPL, kLearned, kZeroSoft, kShare>, grid,
                  32 * kWarpsPerBlock, 0, 1, b.pos, b.vel, store_acc ? c->acc : nullptr, c->acc32,
                  (int)c->n, c->tree, c->scal, c->batch, eps2, theta2, leaf, c->p.G * c->p.timestep,
                  c->p.timestep, kick ? 1 : 0, band_theta(c) * band_theta(c), mark_of(c, 7),
                  kLearned ? nullptr : mark_of(c, kPhases));
 }
+
+// The block's four warps walk for one group while all groups fit the GPU at
+// once (23 bodies to a group of up to 32: 4,300 of 4,736 resident warps at the
+// limit); a group's walk is a chain of some 25 dependent rounds.  Force, us,
+// one warp and four: 1,001 bodies 36 and 24, 4,096 45 and 39, 16,384 56 and 47
+// (quadrupoles 82 and 69), 32,768 57 and 62.
+constexpr int64_t kShareMax = 24576;
 
 // eps2 = 0 takes the variant whose terms skip coincident FP32 points
 template <bool kQuad, int kBPL, bool kLearned>
@@ -556,10 +606,14 @@ void launch_split_kernel(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_
                          bool chained) {
     // eps2 below the smallest normal float is treated like eps2 = 0
     const float eps2 = (float)c->p.epsilon_squared;
+    constexpr bool kCanShare = kBPL == 1 && !kLearned;
+    const bool share = kCanShare && c->n <= kShareMax;
     if (eps2 >= FLT_MIN)
-        launch_split_soft<kQuad, kBPL, kLearned, false>(c, b, kick, store_acc, chained, eps2);
+        share ? launch_split_soft<kQuad, kBPL, kLearned, false, kCanShare>(c, b, kick, store_acc, chained, eps2)
+              : launch_split_soft<kQuad, kBPL, kLearned, false, false>(c, b, kick, store_acc, chained, eps2);
     else
-        launch_split_soft<kQuad, kBPL, kLearned, true>(c, b, kick, store_acc, chained, eps2);
+        share ? launch_split_soft<kQuad, kBPL, kLearned, true, kCanShare>(c, b, kick, store_acc, chained, eps2)
+              : launch_split_soft<kQuad, kBPL, kLearned, true, false>(c, b, kick, store_acc, chained, eps2);
 }
 
 }  // namespace
