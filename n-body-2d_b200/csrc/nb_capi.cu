@@ -198,6 +198,7 @@ int alloc_batch(nb_ctx* c, uint32_t nuni, const uint64_t* counts) {
     NB_CUDA(c, dalloc(&b.boxbits, 4 * (size_t)nuni));
     NB_CUDA(c, dalloc(&b.center, nuni));
     NB_CUDA(c, dalloc(&b.w2, nuni));
+    NB_CUDA(c, dalloc(&b.inv_w, nuni));
     NB_CUDA(c, dalloc(&b.lo, nuni));
     NB_CUDA(c, dalloc(&b.root, nuni));
     NB_CUDA(c, cudaMemcpy(doff, off.data(), sizeof(int32_t) * (nuni + 1), cudaMemcpyHostToDevice));
@@ -214,6 +215,7 @@ void free_batch(nb_ctx* c) {
     cudaFree(b.boxbits);
     cudaFree(b.center);
     cudaFree(b.w2);
+    cudaFree(b.inv_w);
     cudaFree(b.lo);
     cudaFree(b.root);
     b = nb::Batch();

@@ -78,6 +78,7 @@ struct Batch {
     unsigned long long* boxbits = nullptr;  // [nuni][4] order-preserving min/max of x, y
     double2* center = nullptr;           // [nuni] squared-box centre
     double* w2 = nullptr;                // [nuni] squared root width
+    double* inv_w = nullptr;             // [nuni] 1 / root width
     double2* lo = nullptr;               // [nuni] squared-box lower corner
     int32_t* root = nullptr;             // [nuni] root ref (cell, or ~first body of a leaf)
 };
