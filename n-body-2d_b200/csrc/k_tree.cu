@@ -957,6 +957,7 @@ tree_moments(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
             const int needed = t.nint[par], up = t.parent[par];
             const int4 ch = t.child[par];
             if (arrive_acq_rel(t.ready + par) != needed - 1) break;
+            t.ready[par] = 0;  // all have arrived: the learned features count again
             any_moments(par, ch);
             par = up;
         }
