@@ -1233,13 +1233,38 @@ __device__ __forceinline__ void add_shifted(float m, float dx, float dy, const f
     S[2] += cs.z + m * dy * dy;
 }
 
+// A block deals its cells to its threads by size, so that the lanes of a warp
+// sum over about as many bodies each (in id order 9 of 32 lanes were active).
 __global__ void __launch_bounds__(kThreads)
 learned_features(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
                  const double* __restrict__ mass, Tree t, Batch bt) {
     chain_begin();
-    int id = blockIdx.x * blockDim.x + threadIdx.x;
+    const int id0 = blockIdx.x * blockDim.x;
     const int cells = s->cells;
-    if (id >= cells || !direct_cell(t, id)) return;
+    if (id0 >= cells) return;
+    __shared__ int bin[kDirectCell + 1];  // sizes of more than 32 bodies, 32, 31, ..., 1
+    __shared__ short deal[kThreads];
+    for (int k = threadIdx.x; k <= kDirectCell; k += kThreads) bin[k] = 0;
+    __syncthreads();
+    int id = id0 + threadIdx.x;
+    const bool mine = id < cells && direct_cell(t, id);
+    int rank = 0, b = 0;
+    if (mine) {
+        const int2 r = t.range[id];
+        b = kDirectCell - min(r.y - r.x, kDirectCell);
+        rank = atomicAdd(&bin[b], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {  // where each size starts (size 1 has no cells)
+        const int inc = warp_inclusive(bin[threadIdx.x]);
+        bin[threadIdx.x] = inc - bin[threadIdx.x];
+        if (threadIdx.x == 31) bin[kDirectCell] = inc;
+    }
+    __syncthreads();
+    if (mine) deal[bin[b] + rank] = (short)threadIdx.x;
+    __syncthreads();
+    if ((int)threadIdx.x >= bin[kDirectCell]) return;
+    id = id0 + deal[threadIdx.x];
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     {
         const double2 com = t.com[id];
