@@ -128,6 +128,7 @@ int alloc_all(nb_ctx* c) {
     }
     NB_CUDA(c, dalloc(&c->scal, 1));
     NB_CUDA(c, cudaMemset(c->scal, 0, sizeof(nb::DeviceScalars)));
+    NB_CUDA(c, cudaMallocHost(&c->host_error, sizeof(unsigned)));
     // (the last block folds one partial per block: no more blocks than fill)
     c->bbox_blocks = (int)std::min<size_t>(2 * c->sm_count, (n + 1023) / 1024);
     NB_CUDA(c, dalloc(&c->bbox_partials, (size_t)4 * c->bbox_blocks));
@@ -163,6 +164,7 @@ void free_all(nb_ctx* c) {
                          t.ansv_last};
     for (void* q : tree_ptrs) cudaFree(q);
     cudaFree(c->scal);
+    cudaFreeHost(c->host_error);
     cudaFree(c->bbox_partials);
     cudaFree(c->acc);
     cudaFree(c->dbg_terms);
@@ -305,11 +307,14 @@ int capture_graph(nb_ctx* c, int parity) {
     return NB_OK;
 }
 
+// Waits for the stream and reports the device's error flags.  The flags come
+// into pinned memory behind whatever the stream still has to do, so that one
+// wait covers both.
 int read_device_error(nb_ctx* c) {
-    unsigned flags = 0;
-    NB_CUDA(c, cudaMemcpyAsync(&flags, &c->scal->error, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                               c->stream));
+    NB_CUDA(c, cudaMemcpyAsync(c->host_error, &c->scal->error, sizeof(unsigned),
+                               cudaMemcpyDeviceToHost, c->stream));
     NB_CUDA(c, cudaStreamSynchronize(c->stream));
+    const unsigned flags = *c->host_error;
     if (!flags) return NB_OK;
     NB_CUDA(c, cudaMemsetAsync(&c->scal->error, 0, sizeof(unsigned), c->stream));
     if (flags & nb::kErrTimeout) return fail(c, NB_ERR_TIMEOUT, "a bounded device wait gave up");
@@ -604,13 +609,13 @@ int nb_step(nb_ctx* c, uint32_t nsteps) {
 int nb_sync(nb_ctx* c) {
     if (!c) return NB_ERR_INVALID;
     DeviceGuard guard(c->device);
-    NB_CUDA(c, cudaStreamSynchronize(c->stream));
+    const int rc = read_device_error(c);  // waits for the steps
     NB_CUDA(c, cudaStreamSynchronize(c->copy_stream));
     float ms = 0.f;
     if (c->batch_steps && cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess)
         c->ms_last = ms / c->batch_steps;
     c->batch_steps = 0;
-    return read_device_error(c);
+    return rc;
 }
 
 int nb_debug_wait_timeout(int32_t device) {
@@ -670,7 +675,6 @@ int nb_download(nb_ctx* c, double* pos_xy, double* vel_xy) {
         NB_CUDA(c, cudaMemcpyAsync(pos_xy, c->stage_pos, bytes, cudaMemcpyDeviceToHost, c->stream));
     if (vel_xy)
         NB_CUDA(c, cudaMemcpyAsync(vel_xy, c->stage_vel, bytes, cudaMemcpyDeviceToHost, c->stream));
-    NB_CUDA(c, cudaStreamSynchronize(c->stream));
     return read_device_error(c);
 }
 
@@ -687,7 +691,6 @@ int nb_accelerations(nb_ctx* c, double* acc_xy) {
     NB_CUDA(c, cudaGetLastError());
     NB_CUDA(c, cudaMemcpyAsync(acc_xy, c->stage_pos, (size_t)c->n * sizeof(double2),
                                cudaMemcpyDeviceToHost, c->stream));
-    NB_CUDA(c, cudaStreamSynchronize(c->stream));
     return read_device_error(c);
 }
 
@@ -707,7 +710,6 @@ int nb_debug_morton(nb_ctx* c, uint64_t* codes, int32_t* order, double* box_out)
     if (box_out)
         NB_CUDA(c, cudaMemcpyAsync(box_out, c->scal->box, 4 * sizeof(double), cudaMemcpyDeviceToHost,
                                    c->stream));
-    NB_CUDA(c, cudaStreamSynchronize(c->stream));
     return read_device_error(c);
 }
 
@@ -888,7 +890,6 @@ int nb_render(nb_ctx* c, const nb_view* v, uint8_t* rgba_out) {
     NB_CUDA(c, cudaGetLastError());
     NB_CUDA(c, cudaMemcpyAsync(rgba_out, c->render_rgba, (size_t)pixels * 4, cudaMemcpyDeviceToHost,
                                c->stream));
-    NB_CUDA(c, cudaStreamSynchronize(c->stream));
     return read_device_error(c);
 }
 
