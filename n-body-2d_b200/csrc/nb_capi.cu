@@ -74,7 +74,7 @@ int alloc_all(nb_ctx* c) {
     c->sort.tiles = (int)((n + nb::kSortTile - 1) / nb::kSortTile);
     if (c->n > nb::cluster_sort_size()) {  // onesweep passes
         NB_CUDA(c, dalloc(&c->sort.hist, 8 * 256));
-        NB_CUDA(c, dalloc(&c->sort.status, (size_t)8 * 256 * c->sort.tiles));
+        NB_CUDA(c, dalloc(&c->sort.status, (size_t)8 * 256 * nb::sort_status_rows(c->sort.tiles)));
         NB_CUDA(c, dalloc(&c->sort.tile_counter, 8));
     }
     NB_CUDA(c, dalloc(&c->sort.ties_small, n / 2 + 1));

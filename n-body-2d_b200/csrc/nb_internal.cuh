@@ -17,6 +17,12 @@ constexpr int kStackDepth = 96;   // >= 1 + 3 * 30 pending cells of a DFS
 constexpr int kSortTileItems = 12; // keys per thread in a radix tile
 constexpr int kSortThreads = 256;
 constexpr int kSortTile = kSortTileItems * kSortThreads;  // 3072 keys
+constexpr int kSortGroup = 8;      // tiles whose counts the look-back takes together
+// rows of 256 look-back words per pass: each tile's counts, each group's, each
+// group's start
+inline __host__ __device__ int sort_status_rows(int tiles) {
+    return tiles + 2 * ((tiles + kSortGroup - 1) / kSortGroup);
+}
 constexpr int kAnsvTile = 2048;   // boundaries per tile of the tree build's level scans
 constexpr int kAnsvLevels = 32;   // table width per tile: levels 0..30 and one spare
 constexpr int kPhases = 9;        // morton, sort, gather, prefix, tree, moments, groups, force, drift
@@ -151,7 +157,7 @@ struct SortBuffers {
     uint64_t* key[2] = {nullptr, nullptr};
     uint32_t* val[2] = {nullptr, nullptr};
     uint32_t* hist = nullptr;     // [8][256] digit histograms -> exclusive bin offsets
-    uint32_t* status = nullptr;   // [8][tiles][256] look-back status words
+    uint32_t* status = nullptr;   // [8][sort_status_rows(tiles)][256] look-back status words
     unsigned* tile_counter = nullptr;  // [8]
     uint2* ties_small = nullptr;  // tie groups of 2..32 keys: {first, size}, n / 2 + 1
     uint2* ties_big = nullptr;    // tie groups of more than 32 keys, n / 33 + 1
