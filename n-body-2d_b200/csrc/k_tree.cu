@@ -511,11 +511,29 @@ __device__ void cell_from_prefix(const double4* __restrict__ prefix, const Tree&
                                  const double2* __restrict__ pos, int id, int2 r, int level,
                                  float accept_scale);
 
+// Groups of half the size or less, whose bodies lie one to a lane, are listed
+// after all others up to kSmallLastMax bodies (small > 0): the walk takes the
+// groups in order, and ends sooner when the cheap ones come last.  Above, the
+// end matters less than the places in the tree that neighbours share.  Force
+// phase, us, in key order and small ones last: collision 262,144 bodies 130 and
+// 126, 524,288 223 and 204, 1M 404 and 386, 2M 777 and 767, 4M 1,541 and 1,546,
+// 1M with quadrupoles 865 and 841, Plummer 300,000 171 and 161; listing them costs
+// 1.2 us.  Groups of up to 32 bodies cost alike, and learned contexts sample groups
+// by index: both keep the order of the keys.
+constexpr int64_t kSmallLastMax = 2097152;
+// Counts of groups: all above kSmallBits and small ones (at most 9 a cell) below,
+// where small ones are listed apart; else all.
+constexpr int kSmallBits = 15;
+static_assert(9 * kAnsvTile < 1 << kSmallBits &&
+                  kSmallLastMax / 64 + 9 * kAnsvTile < 1 << (31 - kSmallBits),
+              "a tile's counts fit a word");
+
 // The SPLIT target groups of one cell (defined with tree_groups_write below).
 template <bool kWrite>
 __device__ __forceinline__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const int* cb,
-                           const bool* leaf, int gsize, int fill, const Batch& bt,
-                           const uint64_t* __restrict__ key, int2* __restrict__ out);
+                           const bool* leaf, int gsize, int fill, int small, const Batch& bt,
+                           const uint64_t* __restrict__ key, int2* __restrict__ out,
+                           int2* __restrict__ out_small);
 
 // A tree without internal cells: one body, or all bodies in one level-30 leaf.
 __device__ void trivial_root(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
@@ -533,7 +551,7 @@ __device__ __forceinline__ int link_cell(int i, int id, const uint64_t* __restri
                                          const double* __restrict__ mass, const Tree& t,
                                          DeviceScalars* __restrict__ s,
                                          const double4* __restrict__ prefix, const Batch& bt,
-                                         float accept_scale, int gsize, int fill) {
+                                         float accept_scale, int gsize, int fill, int small) {
     const uint8_t* __restrict__ lcp8 = t.lcp8;
     const int4 bi = t.bnd[i];
     const int c = lcp8[i];
@@ -580,7 +598,8 @@ __device__ __forceinline__ int link_cell(int i, int id, const uint64_t* __restri
     int groups = 0;
     if (gsize > 0) {
         groups = cell_groups<false>(make_int2(first, last), first == 0 && last == n - 1,
-                                          ns + 1, ca, cb, leaf, gsize, fill, bt, key, nullptr);
+                                    ns + 1, ca, cb, leaf, gsize, fill, small, bt, key, nullptr,
+                                    nullptr);
         t.gcount[id] = groups;
     }
     for (int q = ns + 1; q < 4; ++q) child[q] = INT_MIN;
@@ -625,7 +644,8 @@ template <bool kMono>
 __global__ void __launch_bounds__(kThreads, 5)
 tree_link(const uint64_t* __restrict__ key, int n, const double2* __restrict__ pos,
           const double* __restrict__ mass, Tree t, DeviceScalars* __restrict__ s,
-          const double4* __restrict__ prefix, Batch bt, float accept_scale, int gsize, int fill) {
+          const double4* __restrict__ prefix, Batch bt, float accept_scale, int gsize, int fill,
+          int small) {
     chain_begin();
     const int tile = blockIdx.x / kLinkBlocks;
     const int cells = s->cells;
@@ -639,7 +659,7 @@ tree_link(const uint64_t* __restrict__ key, int n, const double2* __restrict__ p
     if (j < t.tile_count[tile])
         groups = link_cell<kMono>(tile * kAnsvTile + t.rep[tile * kAnsvTile + j],
                                   t.tile_cells[tile] + j, key, n, pos, mass, t, s, prefix, bt,
-                                  accept_scale, gsize, fill);
+                                  accept_scale, gsize, fill, small);
     if (gsize == 0) return;
     const int sum = __reduce_add_sync(kFull, groups);
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(t.tile_groups + tile, sum);
@@ -1333,16 +1353,18 @@ learned_features(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
 // bodies then walked the whole core on one warp (2.3 ms of a 65,536-body
 // step).  So with a large child present, runs also end at the half boundary.
 // The groups of one cell with body range rg and nc children in code order
-// ([ca, cb], leaf marks the leaf children); returns their number and, with
-// kWrite, writes them from out on.
+// ([ca, cb], leaf marks the leaf children); returns their counts and, with kWrite,
+// writes them from out on, those of up to `small` bodies from out_small on.
 template <bool kWrite>
 __device__ __forceinline__ int cell_groups(int2 rg, bool is_root, int nc, const int* ca, const int* cb,
-                           const bool* leaf, int gsize, int fill, const Batch& bt,
-                           const uint64_t* __restrict__ key, int2* __restrict__ out) {
+                           const bool* leaf, int gsize, int fill, int small, const Batch& bt,
+                           const uint64_t* __restrict__ key, int2* __restrict__ out,
+                           int2* __restrict__ out_small) {
     int emitted = 0;
     auto emit = [&](int a, int b) {
-        if (kWrite) out[emitted] = make_int2(a, b);
-        ++emitted;
+        const bool is_small = b - a < small;
+        if (kWrite) *(is_small ? out_small++ : out++) = make_int2(a, b);
+        emitted += small > 0 ? (1 << kSmallBits) + is_small : 1;
     };
     // batched universes: a forest cell above the universe roots may hold few
     // bodies but never becomes a group; it hands its children on instead
@@ -1402,9 +1424,14 @@ __device__ __forceinline__ int cell_groups(int2 rg, bool is_root, int nc, const 
 // Writes the groups, which the linking pass counted, one block per tile: the
 // tile's counts are scanned (each warp 8 rows of 32 cells), and the few cells
 // that have groups (1.5% at 4M) are listed and written one thread each.
-__global__ void __launch_bounds__(kThreads)
-tree_groups_write(int n, int gsize, int fill, Tree t, DeviceScalars* __restrict__ s, Batch bt,
-                  const uint64_t* __restrict__ key, unsigned long long* mark) {
+constexpr int kCellBits = 11;
+constexpr int kSmallMask = (1 << kSmallBits) - 1;
+static_assert(kAnsvTile <= 1 << kCellBits && kCellBits + kSmallBits < 31, "a list word's fields");
+
+template <bool kSmall>  // small groups are listed apart
+__global__ void __launch_bounds__(kThreads, kSmall ? 4 : 5)
+tree_groups_write(int n, int gsize, int fill, int small, Tree t, DeviceScalars* __restrict__ s,
+                  Batch bt, const uint64_t* __restrict__ key, unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
     const int tile = blockIdx.x;
@@ -1415,18 +1442,29 @@ tree_groups_write(int n, int gsize, int fill, Tree t, DeviceScalars* __restrict_
         if (tile == 0 && threadIdx.x == 0) s->groups = ng;
         return;
     }
-    __shared__ int wsum[kThreads / 32], wbefore[kThreads / 32];
-    __shared__ int2 some[kAnsvTile];  // {cell, first group}
+    __shared__ int2 wsum[kThreads / 32], wbefore[kThreads / 32];
+    __shared__ int wlarge[kThreads / 32];
+    // cells with groups: {cell and small groups before (kCellBits), others before}
+    __shared__ int2 some[kAnsvTile];
     __shared__ int nsome;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int count = t.tile_count[tile], id0 = t.tile_cells[tile];
     if (threadIdx.x == 0) nsome = 0;
-    // the groups of the tiles before (at most 8 loads per thread at 4M; a scan
-    // by the linking pass's last block cost its other blocks more in fences)
-    int off = 0;
+    // the groups of the tiles before, and all large ones (8 loads per thread at
+    // 4M; a scan by the linking pass's last block cost its other blocks more in
+    // fences)
+    int before = 0, before_small = 0, large = 0;
 #pragma unroll 4
-    for (int q = threadIdx.x; q < tile; q += kThreads) off += t.tile_groups[q];
-    int v[kAnsvItems], ex[kAnsvItems], carry = 0;
+    for (int q = threadIdx.x; q < (kSmall ? (int)gridDim.x : tile); q += kThreads) {
+        const int g = t.tile_groups[q];
+        const int sm = kSmall ? g & kSmallMask : 0, lg = kSmall ? (g >> kSmallBits) - sm : g;
+        large += lg;
+        before += q < tile ? lg : 0;
+        before_small += q < tile ? sm : 0;
+    }
+    // the tile's counts: large groups, small ones
+    int v[kAnsvItems];
+    int2 ex[kAnsvItems], carry = make_int2(0, 0);
 #pragma unroll
     for (int k = 0; k < kAnsvItems; ++k) {
         const int j = (warp * kAnsvItems + k) * 32 + lane;
@@ -1434,30 +1472,43 @@ tree_groups_write(int n, int gsize, int fill, Tree t, DeviceScalars* __restrict_
     }
 #pragma unroll
     for (int k = 0; k < kAnsvItems; ++k) {
-        const int inc = warp_inclusive(v[k]);
-        ex[k] = carry + inc - v[k];
-        carry += __shfl_sync(kFull, inc, 31);
+        const int sm = kSmall ? v[k] & kSmallMask : 0;
+        const int lg = kSmall ? (v[k] >> kSmallBits) - sm : v[k];
+        const int il = warp_inclusive(lg), is = kSmall ? warp_inclusive(sm) : 0;
+        ex[k] = make_int2(carry.x + il - lg, carry.y + is - sm);
+        carry.x += __shfl_sync(kFull, il, 31);
+        if (kSmall) carry.y += __shfl_sync(kFull, is, 31);
     }
-    off = __reduce_add_sync(kFull, off);
+    before = __reduce_add_sync(kFull, before);
+    if (kSmall) {
+        before_small = __reduce_add_sync(kFull, before_small);
+        large = __reduce_add_sync(kFull, large);
+    }
     if (lane == 0) {
         wsum[warp] = carry;
-        wbefore[warp] = off;
+        wbefore[warp] = make_int2(before, before_small);
+        wlarge[warp] = large;
     }
     __syncthreads();
-    off = 0;
+    int2 off = make_int2(0, 0), in_tile = make_int2(0, 0);  // (small ones follow all others)
+#pragma unroll
     for (int w = 0; w < kThreads / 32; ++w) {
-        off += wbefore[w];
-        if (w < warp) off += wsum[w];
+        off.x += wbefore[w].x;
+        off.y += wlarge[w] + wbefore[w].y;
+        in_tile.x += w < warp ? wsum[w].x : 0;
+        in_tile.y += w < warp ? wsum[w].y : 0;
     }
-    if (tile == gridDim.x - 1 && threadIdx.x == kThreads - 1) s->groups = off + carry;
+    if (tile == gridDim.x - 1 && threadIdx.x == kThreads - 1)
+        s->groups = kSmall ? off.y + in_tile.y + carry.y : off.x + in_tile.x + carry.x;
 #pragma unroll
     for (int k = 0; k < kAnsvItems; ++k)
         if (v[k])
             some[atomicAdd(&nsome, 1)] =
-                make_int2(id0 + (warp * kAnsvItems + k) * 32 + lane, off + ex[k]);
+                make_int2((warp * kAnsvItems + k) * 32 + lane | (in_tile.y + ex[k].y) << kCellBits,
+                          in_tile.x + ex[k].x);
     __syncthreads();
     for (int q = threadIdx.x; q < nsome; q += kThreads) {
-        const int id = some[q].x;
+        const int id = id0 + (some[q].x & (1 << kCellBits) - 1);
         const int2 rg = t.range[id];
         const int4 ch = t.child[id];
         const int refs[4] = {ch.x, ch.y, ch.z, ch.w};
@@ -1478,8 +1529,9 @@ tree_groups_write(int n, int gsize, int fill, Tree t, DeviceScalars* __restrict_
             }
             nc = c + 1;
         }
-        cell_groups<true>(rg, id == s->root, nc, ca, cb, leaf, gsize, fill, bt, key,
-                          t.groups + some[q].y);
+        cell_groups<true>(rg, id == s->root, nc, ca, cb, leaf, gsize, fill, kSmall ? small : 0, bt, key,
+                          t.groups + off.x + some[q].y,
+                          t.groups + off.y + (some[q].x >> kCellBits));
     }
 }
 
@@ -1515,14 +1567,21 @@ void launch_batch_roots(nb_ctx* c) {
                  c->sort.key[0], c->tree, c->batch);
 }
 
+static int small_group(const nb_ctx* c) {
+    const int gsize = split_group_size(c);
+    return c->n <= kSmallLastMax && gsize > 32 && !(c->p.flags & NB_FLAG_LEARNED) ? gsize / 2 : 0;
+}
+
 void launch_groups(nb_ctx* c) {
     c->launches += 1;
     // plain SPLIT fills groups to gsize bodies across sibling cells (fuller
     // warps, measured 2.6% off the walk at 4M with slightly lower errors); the
     // learned correction keeps groups of whole cells, whose residuals it fits.
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
-    chain_launch(c->stream, true, tree_groups_write, blocks_for(c->n, kAnsvTile), kThreads, 0, 1,
-                 (int)c->n, split_group_size(c), fill, c->tree, c->scal, c->batch, c->sort.key[0],
+    const int small = small_group(c);
+    chain_launch(c->stream, true, small > 0 ? tree_groups_write<true> : tree_groups_write<false>,
+                 blocks_for(c->n, kAnsvTile), kThreads, 0, 1, (int)c->n, split_group_size(c), fill,
+                 small, c->tree, c->scal, c->batch, c->sort.key[0],
                  mark_of(c, 6));
 }
 
@@ -1578,7 +1637,8 @@ void launch_tree(nb_ctx* c, const BodyBuffers& b) {
     const int fill = (c->p.flags & NB_FLAG_LEARNED) ? 0 : 1;
     chain_launch(c->stream, true, mono ? tree_link<true> : tree_link<false>, tiles * kLinkBlocks,
                  kThreads, 0, 1, key, n, b.pos, b.mass, t, c->scal, mono ? t.prefix : nullptr,
-                 c->batch, mono ? split_accept_scale(c) : 0.f, gsize, fill);
+                 c->batch, mono ? split_accept_scale(c) : 0.f, gsize, fill,
+                 gsize > 0 ? small_group(c) : 0);
 }
 
 void launch_features(nb_ctx* c, const BodyBuffers& b, bool chained) {
