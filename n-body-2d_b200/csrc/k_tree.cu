@@ -1111,7 +1111,8 @@ prefix_reduce(const double2* __restrict__ pos, const double* __restrict__ mass, 
 // tiles (kFew): the block scans the tiles' totals itself.
 // A warp of its own does that beside the rows' scans.
 template <bool kFew>
-__global__ void __launch_bounds__(kThreads + (kFew ? 32 : 0))
+// (four blocks per SM, 64 registers: 300k bodies 14.5 -> 12.0 us, 4M as with 80)
+__global__ void __launch_bounds__(kThreads + (kFew ? 32 : 0), kFew ? 1 : 4)
 prefix_apply(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
              const DeviceScalars* __restrict__ s, Batch bt, const double4* __restrict__ tiles,
              int ntiles, double4* __restrict__ prefix) {
