@@ -823,7 +823,7 @@ count_scatter(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
 // ---------------------------------------------------------------------------
 constexpr uint32_t kFlagAgg = 1u << 31;  // a published word; the rest is the value
 constexpr int kGroupBits = 20;           // a group's sum: counts below, tiles counted above
-static_assert(kSortGroup * kSortTile < (1 << kGroupBits) && kSortGroup < 1 << (32 - kGroupBits),
+static_assert(kSortGroup * kSortItemsMax * kSortThreads < (1 << kGroupBits) && kSortGroup < 1 << (32 - kGroupBits),
               "a group's counts fit its word");
 constexpr int kSpinLimit = 1 << 22;
 constexpr int kLook = 4;  // words in flight (8 and 16: 4M sort 289 -> 297, 304 us)
@@ -937,15 +937,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar) {
     return false;
 }
 
-// Four blocks per SM (at most 64 registers): tiles of 3072 keys keep enough
-// loads in flight per block, and the occupancy hides the look-back.  The
-// tile's keys and values arrive in shared memory by two bulk copies (the
-// copy engine moves the 36 KB while the block's threads are free), then each
-// thread ranks its 12 keys, and the tile leaves sorted by digit through the
+// Four blocks per SM (at most 64 registers); kItems keys per thread (see
+// sort_tile_items).  The tile's keys and values arrive in shared memory by two
+// bulk copies (the copy engine moves them, up to 36 KB, while the block's
+// threads are free), then each thread ranks its keys, and the tile leaves sorted by digit through the
 // same shared buffers with coalesced stores.  The scatter itself cannot be a
 // bulk copy: a digit's run starts at an arbitrary 8-byte offset of the output.
 // Passes below the step's first pass (shift < 64 - 8 sort_passes) return at
 // once; passes == nullptr runs every pass.
+template <int kItems>
 __global__ void __launch_bounds__(kSortThreads, 4)
 onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ val_in,
               uint64_t* __restrict__ key_out, uint32_t* __restrict__ val_out, int64_t n, int shift,
@@ -953,13 +953,15 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
               unsigned* __restrict__ tile_counter, unsigned* __restrict__ err,
               const int32_t* __restrict__ passes, int tiles) {
     chain_begin();
+    constexpr int kTile = kItems * kSortThreads;
+    constexpr int kMatch = 256 * kWarps;  // the match words, in the values' place
     if (passes && shift < 64 - 8 * *passes) return;
     __shared__ uint16_t whist[kWarps][256];
     __shared__ uint32_t tile_start[256];
     __shared__ uint32_t goff[256];
     __shared__ uint32_t warp_tot[kWarps];
-    __shared__ __align__(16) uint64_t skey[kSortTile];
-    __shared__ __align__(16) uint32_t sval[kSortTile];
+    __shared__ __align__(16) uint64_t skey[kTile];
+    __shared__ __align__(16) uint32_t sval[kTile > kMatch ? kTile : kMatch];
     __shared__ __align__(8) uint64_t bar;
     __shared__ int tile_sh;
 
@@ -967,8 +969,8 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
     if (tid == 0) {
         const int tile = (int)atomicAdd(tile_counter, 1u);
         tile_sh = tile;
-        const int64_t base = (int64_t)tile * kSortTile;
-        const int tile_n = (int)min((int64_t)kSortTile, n - base);
+        const int64_t base = (int64_t)tile * kTile;
+        const int tile_n = (int)min((int64_t)kTile, n - base);
         const int bulk = tile_n & ~3;  // whole 16-byte chunks of both arrays
         mbar_init(&bar);
         mbar_expect_tx(&bar, (unsigned)bulk * 12u);
@@ -981,8 +983,8 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
     for (int w = 0; w < kWarps; ++w) whist[w][tid] = 0;
     __syncthreads();
     const int tile = tile_sh;
-    const int64_t base = (int64_t)tile * kSortTile;
-    const int tile_n = (int)min((int64_t)kSortTile, n - base);
+    const int64_t base = (int64_t)tile * kTile;
+    const int tile_n = (int)min((int64_t)kTile, n - base);
     {
         const int bulk = tile_n & ~3;
         if (tid < tile_n - bulk) {  // the last tile's ragged end, at most 3 keys
@@ -996,13 +998,13 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
         }
     }
     __syncthreads();
-    const int seg = warp * (32 * kSortTileItems);
-    uint64_t k_reg[kSortTileItems];
-    uint32_t v_reg[kSortTileItems];
-    uint32_t r_reg[kSortTileItems];
+    const int seg = warp * (32 * kItems);
+    uint64_t k_reg[kItems];
+    uint32_t v_reg[kItems];
+    uint32_t r_reg[kItems];
     const unsigned below = lanemask_lt();
 #pragma unroll
-    for (int k = 0; k < kSortTileItems; ++k) {
+    for (int k = 0; k < kItems; ++k) {
         const int li = seg + k * 32 + lane;
         const bool valid = li < tile_n;
         k_reg[k] = valid ? skey[li] : 0ull;
@@ -1015,7 +1017,7 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
     for (int k = lane; k < 256; k += 32) match[k] = 0;
     __syncwarp();
 #pragma unroll
-    for (int k = 0; k < kSortTileItems; ++k)
+    for (int k = 0; k < kItems; ++k)
         r_reg[k] = row_rank(match, whist[warp], (uint32_t)(k_reg[k] >> shift) & 255u,
                             seg + k * 32 + lane < tile_n, below);
     __syncthreads();
@@ -1051,7 +1053,7 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
     // (after the look-back: 60 us at 300k, 111 at 1M, 304 at 4M).  The scan's
     // barriers stand between tile_start's writes and these reads.
 #pragma unroll
-    for (int k = 0; k < kSortTileItems; ++k) {
+    for (int k = 0; k < kItems; ++k) {
         const int li = seg + k * 32 + lane;
         if (li < tile_n) {
             const uint32_t d = (uint32_t)((k_reg[k] >> shift) & 0xFF);
@@ -1407,7 +1409,7 @@ void launch_morton(nb_ctx* c, const double2* pos) {
 // its look-back waits on a predecessor that never publishes, so the bounded
 // wait must give up and raise kErrTimeout.  Returns the error bits.
 unsigned sort_timeout_probe(cudaStream_t st) {
-    constexpr int n = 2 * kSortTile;
+    constexpr int n = 2 * kSortItemsMax * kSortThreads;
     uint64_t *key_in = nullptr, *key_out = nullptr;
     uint32_t *val_in = nullptr, *val_out = nullptr, *hist = nullptr, *status = nullptr;
     unsigned *counter = nullptr, *err = nullptr;
@@ -1428,7 +1430,7 @@ unsigned sort_timeout_probe(cudaStream_t st) {
         cudaMemsetAsync(err, 0, sizeof(unsigned), st);
         const unsigned one = 1u;  // the single block takes tile 1
         cudaMemcpyAsync(counter, &one, sizeof(unsigned), cudaMemcpyHostToDevice, st);
-        onesweep_pass<<<1, kSortThreads, 0, st>>>(key_in, val_in, key_out, val_out, n, 0, hist, status,
+        onesweep_pass<kSortItemsMax><<<1, kSortThreads, 0, st>>>(key_in, val_in, key_out, val_out, n, 0, hist, status,
                                                   counter, err, nullptr, 2);
         cudaMemcpyAsync(&flags, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) flags = ~0u;
@@ -1457,14 +1459,17 @@ void launch_sort(nb_ctx* c) {
         }
     } else {
         // the Morton pass has reset the histograms, tile counters and status words
-        const int tiles = c->sort.tiles;
+        const int tiles = c->sort.tiles, items = sort_tile_items(c->n, c->sm_count);
+        auto* pass_kernel = items == 4   ? onesweep_pass<4>
+                            : items == 8 ? onesweep_pass<8>
+                                         : onesweep_pass<kSortItemsMax>;
         c->launches += 1 + 8;
         chain_launch(c->stream, true, onesweep_histogram,
                      std::min<unsigned>(4 * c->sm_count, blocks_for(c->n, 32 * kHistRows * kWarps)),
                      kSortThreads, 0, 1, key[0], key[1], c->n, c->scal, c->sort.hist, mark_of(c, 1));
         for (int pass = 0; pass < 8; ++pass) {
             const int src = pass & 1, dst = src ^ 1;
-            chain_launch(c->stream, true, onesweep_pass, tiles, kSortThreads, 0, 1, key[src], val[src],
+            chain_launch(c->stream, true, pass_kernel, tiles, kSortThreads, 0, 1, key[src], val[src],
                          key[dst], val[dst], c->n, 8 * pass, c->sort.hist + 256 * pass,
                          c->sort.status + (size_t)pass * 256 * sort_status_rows(tiles),
                          c->sort.tile_counter + pass, &c->scal->error, &c->scal->sort_passes, tiles);

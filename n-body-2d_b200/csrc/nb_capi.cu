@@ -71,7 +71,8 @@ int alloc_all(nb_ctx* c) {
         NB_CUDA(c, dalloc(&c->sort.key[k], n));
         NB_CUDA(c, dalloc(&c->sort.val[k], n));
     }
-    c->sort.tiles = (int)((n + nb::kSortTile - 1) / nb::kSortTile);
+    const int tile_keys = nb::sort_tile_items(c->n, c->sm_count) * nb::kSortThreads;
+    c->sort.tiles = (int)((n + tile_keys - 1) / tile_keys);
     if (c->n > nb::cluster_sort_size()) {  // onesweep passes
         NB_CUDA(c, dalloc(&c->sort.hist, 8 * 256));
         NB_CUDA(c, dalloc(&c->sort.status, (size_t)8 * 256 * nb::sort_status_rows(c->sort.tiles)));

@@ -14,9 +14,17 @@ namespace nb {
 
 constexpr int kMaxLevel = 30;     // level-30 cells are leaves (BarnesHutCuda.cu:182)
 constexpr int kStackDepth = 96;   // >= 1 + 3 * 30 pending cells of a DFS
-constexpr int kSortTileItems = 12; // keys per thread in a radix tile
 constexpr int kSortThreads = 256;
-constexpr int kSortTile = kSortTileItems * kSortThreads;  // 3072 keys
+constexpr int kSortItemsMax = 12;
+// Keys per thread of a radix tile: 4 up to one tile of 1,024 keys per SM, 8 up to
+// one wave (four per SM) of tiles of 2,048, else 12.  A pass over few tiles takes
+// as long as one of them, whose steps are as long as its rows; over many, larger
+// tiles have fewer look-backs and longer runs to write.  Sort phase, us, with
+// 4 / 8 / 12: 32,769 bodies 30 / 35 / 40; 131,072 42 / 46 / 53; 300,007 53 / 50 / 57;
+// 524,288 73 / 61 / 67; 1M 114 / 94 / 103; 1.5M 146 / 137 / 118; 4M 340 / 292 / 290.
+inline int sort_tile_items(int64_t n, int sms) {
+    return n <= (int64_t)sms * 1024 ? 4 : n <= (int64_t)sms * 4 * 2048 ? 8 : kSortItemsMax;
+}
 constexpr int kSortGroup = 8;      // tiles whose counts the look-back takes together
 // rows of 256 look-back words per pass: each tile's counts, each group's, each
 // group's start

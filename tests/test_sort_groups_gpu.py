@@ -1,6 +1,6 @@
-"""Digit passes whose tiles (3,072 keys) take their places from groups of eight
-tiles: sizes one key around a tile's and a group's edge, with up to 43 groups,
-more than a look-back has in flight.  Codes and permutation are compared with
+"""Digit passes whose tiles take their places from groups of eight tiles: sizes
+around whole tiles and groups of 1,024, 2,048 or 3,072 keys to a tile, with more
+groups than a look-back has in flight.  Codes and permutation are compared with
 the oracle bit for bit."""
 import numpy as np
 import pytest
