@@ -4,8 +4,8 @@
 // a_i = sum_{j != i} m_j d_ij (|d_ij|^2 + eps2)^-3/2, the pair law of the
 // reference GPU backend (BarnesHutCuda.cu:427-431) without any tree.  Used to
 // state p50/p99 force errors at full size, where a CPU all-pairs sum is too
-// slow.  Sources are staged through shared memory in tiles; each thread owns
-// one target.
+// slow.  Sources are staged through shared memory in tiles, split over the blocks;
+// each thread owns kPer targets.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
