@@ -233,13 +233,18 @@ force_fp64(const double2* __restrict__ pos, const double* __restrict__ mass, dou
         double2 c = make_double2(0.0, 0.0);
         int4 ch = make_int4(INT_MIN, INT_MIN, INT_MIN, INT_MIN);
         if (mask && e.x >= 0) {
-            const int lv = e.x < cells ? t.level[e.x] : -1;
-            if (lv < 0 || lv >= kMaxLevel) {
-                atomicOr(&s->error, kErrTree);
-            } else {
+            int lv = -1;
+            // one round of loads, none waiting for the level (1,001 bodies 21.5 ->
+            // 18.7 us, 300k 384 -> 375, 1M 1,044 -> 1,037)
+            if (e.x < cells) {
+                lv = t.level[e.x];
                 m = t.mass[e.x];
                 c = t.com[e.x];
                 ch = t.child[e.x];
+            }
+            if (lv < 0 || lv >= kMaxLevel) {
+                atomicOr(&s->error, kErrTree);
+            } else {
                 w = wsq[lv];
                 // nearest and farthest side of the box
                 const double x0 = bx0 - c.x, x1 = c.x - bx1, y0 = by0 - c.y, y1 = c.y - by1;
@@ -256,7 +261,12 @@ force_fp64(const double2* __restrict__ pos, const double* __restrict__ mass, dou
             }
         } else if (mask) {
             first = ~e.x;
-            last = t.leaf_last[first];
+            last = -1;
+            if (first < n) {
+                last = t.leaf_last[first];
+                c = pos[first];  // of a single body, CU:424-433
+                m = mass[first];
+            }
             if (last < first || last >= n) {
                 atomicOr(&s->error, kErrTree);
             } else {
@@ -265,9 +275,7 @@ force_fp64(const double2* __restrict__ pos, const double* __restrict__ mass, dou
                 inside = b >= a ? (kFull >> (31 - (b - a))) << a : 0u;
                 accept = mask & ~inside;
                 inside &= mask;
-                if (first == last) {  // CU:424-433
-                    c = pos[first];
-                    m = mass[first];
+                if (first == last) {
                     single = true;
                     inside = 0;
                 } else {  // CU:434-442; the bodies inside: below
