@@ -559,7 +559,8 @@ void launch_force_fp64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_ac
     // bodies.  us at kG = 1 / 4 / 16 / 32: 1,001 bodies 26 / 32 / 45 / 63; 16,384
     // 122 / 55 / 73 / 96; 65,536 624 / 206 / 120 / 132; 262,144 2212 / 665 / 358 /
     // 303; 1,048,576 10599 / 2732 / 1351 / 1058 (one thread per body before: 303,
-    // 486, -, 1225, 3596).
+    // 486, -, 1225, 3596; with a node's loads issued together the chosen sizes now
+    // take 19, 49, 117, - and 1037).
     const int64_t per_warp = c->n / 4096;
     if (per_warp < 2) return launch_walk64<1, false>(c, b, kick, store_acc);
     if (per_warp < 4) return launch_walk64<2, false>(c, b, kick, store_acc);
