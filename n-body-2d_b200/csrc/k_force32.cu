@@ -407,6 +407,9 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
             if (lane < mine) L.stack[lane] = r0;
             size = mine;
         }
+        // the next round's lanes read what other lanes pushed; a round without
+        // bodies meets no other barrier on its way there
+        __syncwarp();
         // bodies of directly summed cells and leaves, expanded 32 at a time
         for (int base = 0; base < btot; base += 32) {
             const int item = base + lane;
