@@ -122,9 +122,9 @@ __device__ __forceinline__ void sum_sources(const double2* __restrict__ pos,
 // i is body i.
 template <bool kCpuLaw, int kPer>
 __global__ void __launch_bounds__(kThreads)
-allpairs_partial(const double2* __restrict__ pos, const double* __restrict__ mass, int64_t n,
-                 const int64_t* __restrict__ targets, int64_t k, int64_t chunk, double eps2,
-                 double2* __restrict__ partial) {
+allpairs_partial(const double2* pos, const double* mass, int64_t n,
+                 const int64_t* targets, int64_t k, int64_t chunk, double eps2,
+                 double2* partial) {
     nb::chain_begin();
     const int64_t first = blockIdx.x * (int64_t)(kThreads * kPer) + threadIdx.x;
     double2 p[kPer];
@@ -168,7 +168,7 @@ __global__ void allpairs_fold(const double2* __restrict__ partial, int chunks, i
 // NB_MODE_ALLPAIRS, stage 1 (AllPairs.cpp:31-35): b = a with x += v dt (or a
 // plain copy when only accelerations are wanted).
 __global__ void allpairs_drift(nb::BodyBuffers a, nb::BodyBuffers b, int64_t n, double dt,
-                               nb::DeviceScalars* __restrict__ s, unsigned long long* mark) {
+                               nb::DeviceScalars* s, unsigned long long* mark) {
     nb::chain_begin();
     nb::mark_start(mark);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -189,9 +189,9 @@ __global__ void allpairs_drift(nb::BodyBuffers a, nb::BodyBuffers b, int64_t n, 
 // Stage 2 (AllPairs.cpp:38-49): every body sums all others (allpairs_partial;
 // each pair is evaluated from both sides: twice the reference's pair
 // evaluations, no atomics), then the kick.
-__global__ void allpairs_kick(const double2* __restrict__ partial, int chunks, int64_t n,
-                              double2* __restrict__ vel, double2* __restrict__ acc_out,
-                              double G_dt, int kick, unsigned long long* __restrict__ body_terms,
+__global__ void allpairs_kick(const double2* partial, int chunks, int64_t n,
+                              double2* vel, double2* acc_out,
+                              double G_dt, int kick, unsigned long long* body_terms,
                               unsigned long long* end) {
     nb::chain_begin();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

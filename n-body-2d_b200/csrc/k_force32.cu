@@ -304,11 +304,10 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
         float4 c4 = make_float4(0.f, 0.f, 0.f, 0.f);
         float band_d2 = 0.f;
         if (lane < k) {
-            // the tree is read-only while the walk runs: non-coherent loads
             if (ref >= 0) {
-                c4 = __ldg(t.cell4 + ref);
-                const int2 rg = __ldg(t.range + ref);
-                ch = __ldg(t.child + ref);  // (with the test, not after it: 1,547 -> 1,542 us)
+                c4 = t.cell4[ref];
+                const int2 rg = t.range[ref];
+                ch = t.child[ref];  // (with the test, not after it: 1,547 -> 1,542 us)
                 const bool overlap = !(rg.y < g0 || rg.x > g1);
                 const float dx = fmaxf(fabsf(c4.x - gcx) - ghx, 0.f);
                 const float dy = fmaxf(fabsf(c4.y - gcy) - ghy, 0.f);
@@ -424,7 +423,7 @@ __device__ __forceinline__ void walk_group(WarpLists& L, const Tree& t, int root
             const int added = min(32, btot - base);
             __syncwarp();
             if (lane < added) {
-                const float4 b4 = __ldg(t.body4 + j);
+                const float4 b4 = t.body4[j];
                 put_entry(L.bxy, L.bm, bcount + lane, b4.x, b4.y, b4.z);
             }
             bcount += added;
@@ -479,8 +478,8 @@ constexpr int kMinBlocks = kBPL == 4 ? 4 : kQuad && kBPL == 2 ? 7 : 8;
 
 template <bool kQuad, int kBPL, bool kLearned, bool kZeroSoft, bool kShare>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocks<kQuad, kBPL>)
-force_split(double2* __restrict__ pos, double2* __restrict__ vel, double2* __restrict__ acc_out,
-            float2* __restrict__ acc32, int n, Tree t, DeviceScalars* __restrict__ s, Batch bt,
+force_split(double2* pos, double2* vel, double2* acc_out,
+            float2* acc32, int n, Tree t, DeviceScalars* s, Batch bt,
             float eps2, float theta2, int leaf_size, double G_dt, double dt, int kick,
             float band2, unsigned long long* mark, unsigned long long* end) {
     chain_begin();

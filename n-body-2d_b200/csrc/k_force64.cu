@@ -92,9 +92,9 @@ __device__ __forceinline__ void plummer(double dx, double dy, double m, double e
 // waiting at and above it) is a property of its path, so each node carries it.
 template <int kG, bool kTerms>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 7)
-force_fp64(const double2* __restrict__ pos, const double* __restrict__ mass, double2* __restrict__ vel,
-           double2* __restrict__ acc_out, int n, Tree t, DeviceScalars* __restrict__ s, double eps2,
-           double theta_sq, double G_dt, int kick, uint2* __restrict__ terms_out,
+force_fp64(const double2* pos, const double* mass, double2* vel,
+           double2* acc_out, int n, Tree t, DeviceScalars* s, double eps2,
+           double theta_sq, double G_dt, int kick, uint2* terms_out,
            unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
@@ -470,7 +470,7 @@ void launch_walk64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc) {
 }
 
 // Drift, CU:489-495.
-__global__ void drift_kernel(double2* __restrict__ pos, const double2* __restrict__ vel, int64_t n,
+__global__ void drift_kernel(double2* pos, const double2* vel, int64_t n,
                              double dt, unsigned long long* mark, unsigned long long* end) {
     chain_begin();
     mark_start(mark);

@@ -126,8 +126,8 @@ __device__ __forceinline__ void write_box(DeviceScalars* s, const RootBox& b) {
 }
 
 __global__ void __launch_bounds__(kBoxThreads)
-bbox_kernel(const double2* __restrict__ pos, int64_t n, double* __restrict__ partials,
-            DeviceScalars* __restrict__ s, int adaptive, int new_step, unsigned long long* mark) {
+bbox_kernel(const double2* pos, int64_t n, double* partials,
+            DeviceScalars* s, int adaptive, int new_step, unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
     double xmin = INFINITY, xmax = -INFINITY, ymin = INFINITY, ymax = -INFINITY;
@@ -136,7 +136,7 @@ bbox_kernel(const double2* __restrict__ pos, int64_t n, double* __restrict__ par
     for (; i + 3 * stride < n; i += 4 * stride) {
         double2 p[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) p[u] = __ldg(pos + i + u * stride);
+        for (int u = 0; u < 4; ++u) p[u] = pos[i + u * stride];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             xmin = fmin(xmin, p[u].x);
@@ -146,7 +146,7 @@ bbox_kernel(const double2* __restrict__ pos, int64_t n, double* __restrict__ par
         }
     }
     for (; i < n; i += stride) {
-        const double2 p = __ldg(pos + i);
+        const double2 p = pos[i];
         xmin = fmin(xmin, p.x);
         xmax = fmax(xmax, p.x);
         ymin = fmin(ymin, p.y);
@@ -232,19 +232,20 @@ __device__ __forceinline__ uint64_t morton_code(double2 p, double x0, double y0,
 // codes go to the buffer the first radix pass reads: pass k reads buffer
 // k & 1, and the first of the step's sort_passes passes is 8 - sort_passes,
 // so the last one always writes buffer 0.
-__global__ void morton_kernel(const double2* __restrict__ pos, int64_t n,
-                              const DeviceScalars* __restrict__ s, uint64_t* __restrict__ key0,
-                              uint64_t* __restrict__ key1, uint32_t* __restrict__ val0,
-                              uint32_t* __restrict__ val1, SortState z) {
+__global__ void morton_kernel(const double2* pos, int64_t n,
+                              const DeviceScalars* s, uint64_t* key0,
+                              uint64_t* key1, uint32_t* val0,
+                              uint32_t* val1, SortState z) {
     chain_begin();
-    reset_sort(z, s->sort_passes);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int passes = s->sort_passes;
+    const double2 p = i < n ? pos[i] : make_double2(0.0, 0.0);
+    const uint64_t code = morton_code(p, s->box[0], s->box[2], s->inv_wh[0], s->inv_wh[1]);
+    reset_sort(z, passes);
     if (i >= n) return;
-    const bool odd = s->sort_passes & 1;
-    uint64_t* __restrict__ key = odd ? key1 : key0;
-    uint32_t* __restrict__ val = odd ? val1 : val0;
-    key[i] = morton_code(__ldg(pos + i), s->box[0], s->box[2], s->inv_wh[0], s->inv_wh[1]);
-    val[i] = (uint32_t)i;
+    const bool odd = passes & 1;
+    (odd ? key1 : key0)[i] = code;
+    (odd ? val1 : val0)[i] = (uint32_t)i;
 }
 
 // ---------------------------------------------------------------------------
@@ -268,7 +269,7 @@ __device__ __forceinline__ double from_ordered(unsigned long long o) {
 constexpr int kBoxRows = 16;
 
 __global__ void __launch_bounds__(256)
-bbox_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b, unsigned long long* mark) {
+bbox_batch_kernel(const double2* pos, int64_t n, Batch b, unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
     const int lane = threadIdx.x & 31;
@@ -295,7 +296,7 @@ bbox_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b, unsigned 
         const int64_t i = base + 32 * r;
         const bool valid = i < n;
         const int u = valid ? b.uid[i] : -1;
-        const double2 p = valid ? __ldg(pos + i) : make_double2(0.0, 0.0);
+        const double2 p = valid ? pos[i] : make_double2(0.0, 0.0);
         const int u0 = __shfl_sync(kFull, u, 0);
         if (u0 < 0) break;  // past the last body
         if (u0 != current) {
@@ -316,7 +317,7 @@ bbox_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b, unsigned 
 
 // Squares every universe's box as the single-universe path does, and resets
 // the reduction slots for the next step.
-__global__ void bbox_batch_finish(Batch b, DeviceScalars* __restrict__ s, int64_t n,
+__global__ void bbox_batch_finish(Batch b, DeviceScalars* s, int64_t n,
                                   int new_step) {
     chain_begin();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
@@ -351,23 +352,27 @@ __global__ void bbox_batch_finish(Batch b, DeviceScalars* __restrict__ s, int64_
     e[3] = ~0ull;
 }
 
-__global__ void morton_batch_kernel(const double2* __restrict__ pos, int64_t n, Batch b,
-                                    const DeviceScalars* __restrict__ s,
-                                    uint64_t* __restrict__ key0, uint64_t* __restrict__ key1,
-                                    uint32_t* __restrict__ val0, uint32_t* __restrict__ val1,
+__global__ void morton_batch_kernel(const double2* pos, int64_t n, Batch b,
+                                    const DeviceScalars* s,
+                                    uint64_t* key0, uint64_t* key1,
+                                    uint32_t* val0, uint32_t* val1,
                                     SortState z) {
     chain_begin();
-    reset_sort(z, s->sort_passes);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    // (cluster sorts read buffer 0)
-    const bool odd = z.hist && (s->sort_passes & 1);
-    uint64_t* __restrict__ key = odd ? key1 : key0;
-    uint32_t* __restrict__ val = odd ? val1 : val0;
+    const int passes = s->sort_passes;
+    if (i >= n) {
+        reset_sort(z, passes);
+        return;
+    }
     const int u = b.uid[i];
     const double2 lo = b.lo[u];
     const double inv_w = b.inv_w[u];
-    const double2 p = __ldg(pos + i);
+    const double2 p = pos[i];
+    reset_sort(z, passes);
+    // (cluster sorts read buffer 0)
+    const bool odd = z.hist && (passes & 1);
+    uint64_t* key = odd ? key1 : key0;
+    uint32_t* val = odd ? val1 : val0;
     const double scale = (double)(1u << kBatchMortonBits);
     const double top = scale - 1.0;
     const uint32_t ix = __double2uint_rd(fmin(fmax((p.x - lo.x) * inv_w * scale, 0.0), top));
@@ -509,9 +514,9 @@ __device__ __forceinline__ void cluster_wait() {
 
 template <int kItems, int kSrc>
 __global__ void __launch_bounds__(kClusterThreads, 1)
-cluster_sort(const double2* __restrict__ pos, int64_t n, DeviceScalars* __restrict__ s, int adaptive,
+cluster_sort(const double2* pos, int64_t n, DeviceScalars* s, int adaptive,
              int new_step, int fixed_passes, const uint64_t* key_in, uint64_t* key_out,
-             uint32_t* __restrict__ val_out, unsigned long long* mark0, unsigned long long* mark1) {
+             uint32_t* val_out, unsigned long long* mark0, unsigned long long* mark1) {
     chain_begin();
     mark_start(mark0);
     constexpr int kTile = kClusterThreads * kItems;
@@ -535,7 +540,7 @@ cluster_sort(const double2* __restrict__ pos, int64_t n, DeviceScalars* __restri
         double2 p[kItems];
 #pragma unroll
         for (int k = 0; k < kItems; ++k)
-            p[k] = first + 32 * k < n ? __ldg(pos + first + 32 * k) : make_double2(0.0, 0.0);
+            p[k] = first + 32 * k < n ? pos[first + 32 * k] : make_double2(0.0, 0.0);
         RootBox box;
         {
             double v[4] = {INFINITY, -INFINITY, INFINITY, -INFINITY};
@@ -695,7 +700,7 @@ constexpr int kCountItems = kCountTile / kCountThreads;
 constexpr int kCountWarps = kCountThreads / 32;
 
 __global__ void __launch_bounds__(kCountThreads)
-count_digits(const uint64_t* __restrict__ key, int64_t n, int pass, uint16_t* __restrict__ counts) {
+count_digits(const uint64_t* key, int64_t n, int pass, uint16_t* counts) {
     chain_begin();
     __shared__ uint32_t hist[4][256];  // one per quarter of the block
     const int tid = threadIdx.x, part = tid >> 8;
@@ -717,9 +722,9 @@ count_digits(const uint64_t* __restrict__ key, int64_t n, int pass, uint16_t* __
 }
 
 __global__ void __launch_bounds__(kCountThreads, 1)
-count_scatter(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ val_in,
-              uint64_t* __restrict__ key_out, uint32_t* __restrict__ val_out, int64_t n, int pass,
-              const uint16_t* __restrict__ counts, int tiles) {
+count_scatter(const uint64_t* key_in, const uint32_t* val_in,
+              uint64_t* key_out, uint32_t* val_out, int64_t n, int pass,
+              const uint16_t* counts, int tiles) {
     chain_begin();
     __shared__ uint16_t whist[kCountWarps][256];  // per warp, then exclusive within its part
     __shared__ uint32_t match[kCountWarps][256];  // per warp and digit: the row's lanes with it
@@ -838,13 +843,13 @@ constexpr int kLook = 4;  // words in flight (8 and 16: 4M sort 289 -> 297, 304 
 constexpr int kHistRows = 4;
 
 __global__ void __launch_bounds__(kSortThreads)
-onesweep_histogram(const uint64_t* __restrict__ key0, const uint64_t* __restrict__ key1, int64_t n,
-                   const DeviceScalars* __restrict__ s, uint32_t* __restrict__ hist,
+onesweep_histogram(const uint64_t* key0, const uint64_t* key1, int64_t n,
+                   const DeviceScalars* s, uint32_t* hist,
                    unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
     // the Morton pass wrote the codes where the first radix pass reads them
-    const uint64_t* __restrict__ key = (s->sort_passes & 1) ? key1 : key0;
+    const uint64_t* key = (s->sort_passes & 1) ? key1 : key0;
     const int dmin = 8 - s->sort_passes;  // digits below are not sorted by a pass
     __shared__ uint32_t h[8][256];
     for (int k = threadIdx.x; k < 8 * 256; k += kSortThreads) (&h[0][0])[k] = 0;
@@ -859,7 +864,7 @@ onesweep_histogram(const uint64_t* __restrict__ key0, const uint64_t* __restrict
 #pragma unroll
         for (int r = 0; r < kHistRows; ++r) {
             const int64_t i = row0 + 32 * r + lane;
-            k[r] = i < n ? __ldg(key + i) : 0ull;
+            k[r] = i < n ? key[i] : 0ull;
         }
 #pragma unroll
         for (int r = 0; r < kHistRows; ++r) {
@@ -947,11 +952,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar) {
 // once; passes == nullptr runs every pass.
 template <int kItems>
 __global__ void __launch_bounds__(kSortThreads, 4)
-onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ val_in,
-              uint64_t* __restrict__ key_out, uint32_t* __restrict__ val_out, int64_t n, int shift,
-              const uint32_t* __restrict__ hist, uint32_t* __restrict__ status,
-              unsigned* __restrict__ tile_counter, unsigned* __restrict__ err,
-              const int32_t* __restrict__ passes, int tiles) {
+onesweep_pass(const uint64_t* key_in, const uint32_t* val_in,
+              uint64_t* key_out, uint32_t* val_out, int64_t n, int shift,
+              const uint32_t* hist, uint32_t* status,
+              unsigned* tile_counter, unsigned* err,
+              const int32_t* passes, int tiles) {
     chain_begin();
     constexpr int kTile = kItems * kSortThreads;
     constexpr int kMatch = 256 * kWarps;  // the match words, in the values' place
@@ -1127,8 +1132,8 @@ onesweep_pass(const uint64_t* __restrict__ key_in, const uint32_t* __restrict__ 
 // ping-pong buffers.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-tie_mark(const uint64_t* __restrict__ key, int64_t n, DeviceScalars* __restrict__ s,
-         uint2* __restrict__ small, uint2* __restrict__ big) {
+tie_mark(const uint64_t* key, int64_t n, DeviceScalars* s,
+         uint2* small, uint2* big) {
     chain_begin();
     const int passes = s->sort_passes;
     if (passes >= 8) return;
@@ -1185,9 +1190,9 @@ tie_mark(const uint64_t* __restrict__ key, int64_t n, DeviceScalars* __restrict_
 constexpr int kTieWarps = 4;
 
 __global__ void __launch_bounds__(kTieWarps * 32)
-tie_sort(uint64_t* __restrict__ key0, uint32_t* __restrict__ val0, uint64_t* __restrict__ key1,
-         uint32_t* __restrict__ val1, const uint2* __restrict__ small, const uint2* __restrict__ big,
-         const DeviceScalars* __restrict__ s) {
+tie_sort(uint64_t* key0, uint32_t* val0, uint64_t* key1,
+         uint32_t* val1, const uint2* small, const uint2* big,
+         const DeviceScalars* s) {
     chain_begin();
     const int passes = s->sort_passes;
     if (passes >= 8) return;
@@ -1280,23 +1285,24 @@ tie_sort(uint64_t* __restrict__ key0, uint32_t* __restrict__ val0, uint64_t* __r
 
 // CU:135-147: gather the bodies into Morton order.  In SPLIT mode it also
 // writes the FP32 source record of each body relative to the box centre.
-__global__ void gather_kernel(const uint32_t* __restrict__ order, int64_t n, BodyBuffers src,
-                              BodyBuffers dst, float4* __restrict__ body4,
-                              const DeviceScalars* __restrict__ s, Batch bt,
+__global__ void gather_kernel(const uint32_t* order, int64_t n, BodyBuffers src,
+                              BodyBuffers dst, float4* body4,
+                              const DeviceScalars* s, Batch bt,
                               unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t j = __ldg(order + i);
-    const double2 p = __ldg(src.pos + j);
-    const double m = __ldg(src.mass + j);
+    const uint32_t j = order[i];
+    const double2 p = src.pos[j], v = src.vel[j];
+    const double m = src.mass[j];
+    const int32_t o = src.orig[j];
+    const double2 c = body4 ? frame_center(s, bt, (int)i) : make_double2(0.0, 0.0);
     dst.pos[i] = p;
-    dst.vel[i] = __ldg(src.vel + j);
+    dst.vel[i] = v;
     dst.mass[i] = m;
-    dst.orig[i] = __ldg(src.orig + j);
+    dst.orig[i] = o;
     if (body4) {
-        const double2 c = frame_center(s, bt, (int)i);
         body4[i] = make_float4((float)(p.x - c.x), (float)(p.y - c.y), (float)m,
                                __int_as_float((int)i));
     }

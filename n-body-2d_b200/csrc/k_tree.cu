@@ -136,8 +136,8 @@ constexpr int kWideTiles = 148;
 
 template <int kBlock>
 __global__ void __launch_bounds__(kBlock)
-tree_lcp(const uint64_t* __restrict__ key, int n, uint8_t* __restrict__ lcp8,
-         TileTable tab, unsigned* __restrict__ lcp_hist,
+tree_lcp(const uint64_t* key, int n, uint8_t* lcp8,
+         TileTable tab, unsigned* lcp_hist,
          unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
@@ -197,7 +197,7 @@ tree_lcp(const uint64_t* __restrict__ key, int n, uint8_t* __restrict__ lcp8,
 // with a level below v, tile_first the first of tiles t..tiles-1.
 constexpr int kTileScanThreads = 1024;
 __global__ void __launch_bounds__(kTileScanThreads)
-tree_ansv_tiles(int tiles, int32_t* __restrict__ tile_first, int32_t* __restrict__ tile_last) {
+tree_ansv_tiles(int tiles, int32_t* tile_first, int32_t* tile_last) {
     chain_begin();
     __shared__ int wagg[kTileScanThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -329,7 +329,7 @@ __device__ __forceinline__ int cell_id(const Tree& t, int boundary) {
 // when those equal c_i.
 template <int kBlock>
 __global__ void __launch_bounds__(kBlock)
-tree_ansv(Tree t, int n, int tiles, TileTable tab, DeviceScalars* __restrict__ s) {
+tree_ansv(Tree t, int n, int tiles, TileTable tab, DeviceScalars* s) {
     chain_begin();
     constexpr int kItems = kAnsvTile / kBlock, kWarps = kBlock / 32;
     // masks[r][v]: row r's ballot of "level < v" (v = 1..30; 0 elsewhere).
@@ -642,9 +642,9 @@ constexpr int kLinkBlocks = kAnsvTile / kThreads;
 
 template <bool kMono>
 __global__ void __launch_bounds__(kThreads, 5)
-tree_link(const uint64_t* __restrict__ key, int n, const double2* __restrict__ pos,
-          const double* __restrict__ mass, Tree t, DeviceScalars* __restrict__ s,
-          const double4* __restrict__ prefix, Batch bt, float accept_scale, int gsize, int fill,
+tree_link(const uint64_t* key, int n, const double2* pos,
+          const double* mass, Tree t, DeviceScalars* s,
+          const double4* prefix, Batch bt, float accept_scale, int gsize, int fill,
           int small) {
     chain_begin();
     const int tile = blockIdx.x / kLinkBlocks;
@@ -837,8 +837,8 @@ struct MomentSmem {
 
 template <bool kSplit, bool kSecond>
 __global__ void __launch_bounds__(kMomentThreads, 2)
-tree_moments(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
-             const double* __restrict__ mass, int n, Tree t, Batch bt, float accept_scale,
+tree_moments(DeviceScalars* s, const double2* pos,
+             const double* mass, int n, Tree t, Batch bt, float accept_scale,
              unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
@@ -1064,7 +1064,7 @@ __device__ double4 block_exclusive_d4(double4 v, double4* part, double4& total) 
 // Many tiles: exclusive scan of the totals (one block, chunks of kThreads *
 // kScanItems tiles in order); tiles[ntiles] = the grand total.
 __global__ void __launch_bounds__(kThreads)
-prefix_tiles_scan(double4* __restrict__ tiles, int ntiles) {
+prefix_tiles_scan(double4* tiles, int ntiles) {
     chain_begin();
     __shared__ double4 part[kThreads];
     double4 carry = make_double4(0.0, 0.0, 0.0, 0.0);
@@ -1089,8 +1089,8 @@ prefix_tiles_scan(double4* __restrict__ tiles, int ntiles) {
 
 // Phase 1: per tile of kScanTile bodies, the total.
 __global__ void __launch_bounds__(kThreads)
-prefix_reduce(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
-              const DeviceScalars* __restrict__ s, Batch bt, double4* __restrict__ tiles,
+prefix_reduce(const double2* pos, const double* mass, int n,
+              const DeviceScalars* s, Batch bt, double4* tiles,
               unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
@@ -1113,9 +1113,9 @@ prefix_reduce(const double2* __restrict__ pos, const double* __restrict__ mass, 
 template <bool kFew>
 // (four blocks per SM, 64 registers: 300k bodies 14.5 -> 12.0 us, 4M as with 80)
 __global__ void __launch_bounds__(kThreads + (kFew ? 32 : 0), kFew ? 1 : 4)
-prefix_apply(const double2* __restrict__ pos, const double* __restrict__ mass, int n,
-             const DeviceScalars* __restrict__ s, Batch bt, const double4* __restrict__ tiles,
-             int ntiles, double4* __restrict__ prefix) {
+prefix_apply(const double2* pos, const double* mass, int n,
+             const DeviceScalars* s, Batch bt, const double4* tiles,
+             int ntiles, double4* prefix) {
     chain_begin();
     __shared__ double4 wtot[kThreads / 32], tile_off;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1257,8 +1257,8 @@ __device__ __forceinline__ void add_shifted(float m, float dx, float dy, const f
 // A block deals its cells to its threads by size, so that the lanes of a warp
 // sum over about as many bodies each (in id order 9 of 32 lanes were active).
 __global__ void __launch_bounds__(kThreads)
-learned_features(DeviceScalars* __restrict__ s, const double2* __restrict__ pos,
-                 const double* __restrict__ mass, Tree t, Batch bt) {
+learned_features(DeviceScalars* s, const double2* pos,
+                 const double* mass, Tree t, Batch bt) {
     chain_begin();
     const int id0 = blockIdx.x * blockDim.x;
     const int cells = s->cells;
@@ -1431,8 +1431,8 @@ static_assert(kAnsvTile <= 1 << kCellBits && kCellBits + kSmallBits < 31, "a lis
 
 template <bool kSmall>  // small groups are listed apart
 __global__ void __launch_bounds__(kThreads, kSmall ? 4 : 5)
-tree_groups_write(int n, int gsize, int fill, int small, Tree t, DeviceScalars* __restrict__ s,
-                  Batch bt, const uint64_t* __restrict__ key, unsigned long long* mark) {
+tree_groups_write(int n, int gsize, int fill, int small, Tree t, DeviceScalars* s,
+                  Batch bt, const uint64_t* key, unsigned long long* mark) {
     chain_begin();
     mark_start(mark);
     const int tile = blockIdx.x;
@@ -1538,7 +1538,7 @@ tree_groups_write(int n, int gsize, int fill, int small, Tree t, DeviceScalars* 
 
 // Root reference of each universe: the cell whose body range is exactly the
 // universe's (found like a child cell in tree_link), or its single leaf.
-__global__ void batch_roots(const uint64_t* __restrict__ key, Tree t, Batch bt) {
+__global__ void batch_roots(const uint64_t* key, Tree t, Batch bt) {
     chain_begin();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= bt.nuni) return;

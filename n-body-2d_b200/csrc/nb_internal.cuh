@@ -313,7 +313,11 @@ __device__ __forceinline__ int choose_sort_passes(const unsigned* hist, int64_t 
 // writes are visible, and then lets the next kernel's blocks be launched as
 // soon as all blocks of this one have come that far.  Nothing is read or
 // written before that wait, so the order of memory accesses is that of plain
-// launches.
+// launches.  A kernel's lifetime does begin before it, while the kernel before
+// may still write: `__ldg` and parameters marked `__restrict__` promise memory
+// that nobody writes for that long, and the compiler may then load it through
+// the non-coherent path or ahead of the wait.  Chained kernels use neither; the
+// wait's memory clobber holds plain loads behind it.
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
