@@ -22,7 +22,6 @@ constexpr int kThreads = 128;
 constexpr int kTile = 256;    // sources staged in shared memory at a time
 
 using nb::m_over_r3;
-using nb::normal_range;
 
 // Pair weight w of a_i += w (p_j - p_i).  kCpuLaw: the law of
 // Simulation::force, m / (d (d^2 + eps2)) (Simulation.cpp:74-80, G applied
@@ -47,7 +46,7 @@ __device__ __forceinline__ double pair_weight_any(double m, double r2, double ep
 // bodies 0.92 -> 0.38 ms).  Several targets per thread share the loads and
 // the loop.  Only a tile that holds one of the warp's own sources tests for
 // it; a tile whose sums are not finite (a square that is zero, subnormal or
-// infinite) is summed again with full-range functions.
+// infinite, or a term that overflows) is summed again with full-range functions.
 template <bool kCpuLaw, int kPer>
 __device__ __forceinline__ void sum_sources(const double2* __restrict__ pos,
                                             const double* __restrict__ mass, int64_t s0, int64_t s1,

@@ -66,7 +66,8 @@ __device__ __forceinline__ double dist2(double dx, double dy) {
 __device__ __forceinline__ void plummer(double dx, double dy, double m, double eps2, double& ax,
                                         double& ay) {
     const double d2 = dist2(dx, dy) + eps2;
-    const double a = normal_range(d2) ? m_over_r3(m, d2) : m_over_r3_any(m, d2);
+    double a = m_over_r3(m, d2);
+    if (!isfinite(a)) a = m_over_r3_any(m, d2);
     ax += dx * a;
     ay += dy * a;
 }
@@ -149,8 +150,9 @@ force_fp64(const double2* pos, const double* mass, double2* vel,
     __syncwarp();
 
     // Both lists below take the first cnt <= 32 entries.  A term whose d2 is
-    // zero, subnormal or infinite comes out as NaN: such a batch (almost never)
-    // is summed again with the full-range 1/sqrt.
+    // zero, subnormal or infinite, or that overflows, comes out infinite or NaN:
+    // such a batch (almost never) is summed again, these terms with the
+    // full-range 1/sqrt.
     auto sum_full = [&](int cnt) {
         const double ax0 = ax, ay0 = ay;
 #pragma unroll 4

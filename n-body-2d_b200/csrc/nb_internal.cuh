@@ -257,8 +257,9 @@ __device__ __forceinline__ double cell_width2(const DeviceScalars* s, const Batc
 // m r^-3 from r^2 (FP64): the hardware's approximate 1/sqrt y (about 20 bits),
 // corrected by the binomial series of (1 - e)^(-3/2), e = 1 - r^2 y^2, to its
 // second-order term; e^3 is below 2^-57.  Seven FP64 instructions.  y has so
-// few bits that y^2 is exact, so e carries one rounding.  For r^2 in
-// normal_range(); m_over_r3_any() takes the rest.
+// few bits that y^2 is exact, so e carries one rounding.  A zero, subnormal or
+// infinite r^2 and an overflow give an infinity or NaN (inf * e - inf), never a
+// finite value: m_over_r3_any() then says which.
 __device__ __forceinline__ double m_over_r3(double m, double r2) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
@@ -277,9 +278,6 @@ __device__ __forceinline__ double m_over_r_s(double m, double r2, double s) {
     const double e = __fma_rn(-__dmul_rn(r2, v), v, 1.0);
     const double w = __dmul_rn(m, u);
     return __fma_rn(w, __dmul_rn(e, __fma_rn(0.375, e, 0.5)), w);
-}
-__device__ __forceinline__ bool normal_range(double x) {  // positive, normal and finite
-    return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u;
 }
 __device__ __forceinline__ double m_over_r3_any(double m, double r2) {
     const double inv = rsqrt(r2);
