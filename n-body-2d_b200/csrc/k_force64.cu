@@ -251,7 +251,8 @@ force_fp64(const double2* pos, const double* mass, double2* vel,
                 // nearest and farthest side of the box
                 const double x0 = bx0 - c.x, x1 = c.x - bx1, y0 = by0 - c.y, y1 = c.y - by1;
                 const double xn = x0 > x1 ? x0 : x1, yn = y0 > y1 ? y0 : y1;
-                const double near2 = dist2(xn > 0.0 ? xn : 0.0, yn > 0.0 ? yn : 0.0);
+                // (an undefined centre keeps its NaN, which fails both tests below)
+                const double near2 = dist2(xn < 0.0 ? 0.0 : xn, yn < 0.0 ? 0.0 : yn);
                 if (w < theta_sq * near2) {
                     accept = mask;
                 } else if (kG == 1) {
