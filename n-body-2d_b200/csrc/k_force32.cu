@@ -587,8 +587,10 @@ void launch_split_soft(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_ac
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &blocks, force_split<kQuad, kBPL, kLearned, kZeroSoft, kShare>, kWarpsPerBlock * 32, 0) !=
                     cudaSuccess ||
-            blocks < 1)
+            blocks < 1) {
+            cudaGetLastError();
             blocks = 4;
+        }
         grid = c->sm_count * blocks;
     }
     const float theta2 = (float)(c->p.theta * c->p.theta);

@@ -1221,8 +1221,10 @@ void launch_mlp_correct(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_a
         int blocks = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, mlp_correct_kick,
                                                           kCorrWarps * 32, smem) != cudaSuccess ||
-            blocks < 1)
+            blocks < 1) {
+            cudaGetLastError();
             blocks = 2;
+        }
         c->corr_blocks_per_sm = blocks;
     }
     mlp_correct_kick<<<c->sm_count * c->corr_blocks_per_sm, kCorrWarps * 32, smem, c->stream>>>(

@@ -295,11 +295,20 @@ unsigned active_phases(const nb_ctx* c) {
 
 int capture_graph(nb_ctx* c, int parity) {
     cudaGraph_t g = nullptr;
+    cudaGetLastError();  // (an error that an earlier call left behind)
     NB_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     const uint64_t before = c->launches;
     enqueue_step(c, parity, true, false, true);
     c->kernels_per_step = c->launches - before;
+    // the launchers return nothing: what failed is the last error.  A capture
+    // with a launch missing still ends well, as a graph without that kernel.
+    const cudaError_t launched = cudaGetLastError();
     const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+    if (launched != cudaSuccess) {
+        if (e == cudaSuccess) cudaGraphDestroy(g);
+        cudaGetLastError();
+        return fail(c, NB_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(launched));
+    }
     if (e != cudaSuccess) return fail(c, NB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     const cudaError_t e2 = cudaGraphInstantiate(&c->graph[parity], g, 0);
     cudaGraphDestroy(g);

@@ -1,0 +1,100 @@
+"""Failed launches are reported: the library's host side on a fake CUDA runtime
+(fake_cudart.c) that runs no kernel and fails the calls it is told to."""
+import ctypes as C
+import importlib
+import pathlib
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = pathlib.Path(__file__).resolve().parent
+LAUNCH, ATTRIBUTE, CLUSTERS = range(3)
+NB_ERR_CUDA = 2
+
+
+@pytest.fixture(scope="module")
+def fake(nbp, tmp_path_factory):
+    """libnbody_b200's own objects, linked with the fake runtime."""
+    build = importlib.import_module(nbp.__name__ + ".build")
+    build.build()
+    objects = sorted(build.OBJ / (s.stem + ".o") for s in build.CSRC.glob("*.cu"))
+    so = tmp_path_factory.mktemp("fake") / "libnbody_fake.so"
+    cuda = pathlib.Path(build.nvcc()).resolve().parents[1]
+    fake_o = so.with_suffix(".o")
+    subprocess.run(["gcc", "-c", "-O1", "-fPIC", "-fvisibility=hidden", "-I", str(cuda / "include"),
+                    str(HERE / "fake_cudart.c"), "-o", str(fake_o)], check=True)
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined", "-o", str(so),
+                    *map(str, objects), str(fake_o)], check=True)
+    lib = C.CDLL(str(so))
+    lib.nb_last_error.restype = C.c_char_p
+    lib.nb_last_error.argtypes = [C.c_void_p]
+    lib.fake_calls.restype = C.c_long
+    lib.fake_fail.argtypes = [C.c_int, C.c_long]
+    return lib
+
+
+# (mode, flags, bodies, universes): one context per chain of kernels
+KINDS = {
+    "fp64 cluster": (0, 0, 1000, 0), "fp64 onesweep": (0, 0, 40000, 0),
+    "fp64 wide": (0, 0, 400000, 0),
+    "split cluster": (1, 0, 1000, 0), "split onesweep": (1, 0, 140000, 0),
+    "split scanned tiles": (1, 0, 600000, 0),
+    "quad": (1, 1, 1000, 0), "learned": (1, 2, 1000, 0), "learned quad": (1, 3, 40000, 0),
+    "batch cluster": (1, 0, 1000, 4), "batch onesweep": (1, 0, 40000, 4),
+    "allpairs": (2, 0, 1000, 0), "allpairs cpu law": (2, 4, 1000, 0),
+}
+
+
+class Context:
+    def __init__(self, nbp, lib, kind):
+        mode, flags, n, universes = KINDS[kind]
+        p = nbp.NbParams()
+        lib.nb_params_default(C.byref(p))
+        p.mode, p.flags = mode, flags
+        self.lib, self.h, self.n = lib, C.c_void_p(), n
+        m, x = np.ones(n), np.zeros((n, 2))
+        lib.fake_reset()
+        args = (m.ctypes.data_as(C.c_void_p), x.ctypes.data_as(C.c_void_p),
+                x.ctypes.data_as(C.c_void_p), C.byref(self.h))
+        if universes:
+            counts = (C.c_uint64 * universes)(*[n // universes] * universes)
+            rc = lib.nb_batch_create(C.byref(p), universes, counts, *args)
+        else:
+            rc = lib.nb_create(C.byref(p), C.c_uint64(n), *args)
+        assert rc == 0
+        if flags & 2:
+            w = np.zeros(5123, np.float32)
+            assert lib.nb_set_mlp_weights(self.h, w.ctypes.data_as(C.c_void_p)) == 0
+        lib.fake_reset()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        assert self.lib.nb_destroy(self.h) == 0
+
+    def step(self, n=1):
+        return self.lib.nb_step(self.h, n)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_failed_launch_fails_the_step(nbp, fake, kind):
+    with Context(nbp, fake, kind) as ctx:
+        assert ctx.step() == 0
+        calls = [fake.fake_calls(LAUNCH), fake.fake_calls(ATTRIBUTE)]
+    assert calls[0] >= 6
+    for what in (LAUNCH, ATTRIBUTE):
+        for k in range(calls[what]):
+            with Context(nbp, fake, kind) as ctx:
+                fake.fake_fail(what, k)
+                launched = fake.fake_graph_launches()
+                assert ctx.step() == NB_ERR_CUDA, (what, k)
+                assert fake.fake_graph_launches() == launched  # nothing ran
+                assert b"launch" in fake.nb_last_error(ctx.h)
+                assert fake.fake_open_captures() == 0 and fake.fake_live_graphs() == 0
+                assert fake.fake_last_error() == 0
+                # the next step captures what is missing and runs
+                assert ctx.step(3) == 0
+                assert fake.fake_graph_launches() == launched + 3
+
