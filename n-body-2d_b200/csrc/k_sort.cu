@@ -1316,62 +1316,64 @@ inline unsigned blocks_for(int64_t n, int threads) {
 
 namespace {
 
-// Launches cluster_sort over n keys with kItems keys per thread.
-template <int kItems, int kSrc>
-cudaError_t launch_cluster(cudaStream_t st, bool chained, int blocks, int cluster, const double2* pos,
-                           int64_t n, DeviceScalars* s, int adaptive, int new_step, int fixed_passes,
-                           const uint64_t* key_in, uint64_t* key_out, uint32_t* val_out,
-                           unsigned long long* mark0, unsigned long long* mark1) {
-    auto* kernel = cluster_sort<kItems, kSrc>;
-    const size_t smem = sizeof(ClusterSmem<kItems>);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    return chain_launch(st, chained, kernel, blocks, kClusterThreads, smem, cluster, pos, n, s, adaptive,
-                        new_step, fixed_passes, key_in, key_out, val_out, mark0, mark1);
-}
-
 // As few keys per thread as one cluster allows (a pass ranks them one after
 // the other), then as few blocks as hold them.
+inline int cluster_items(int64_t n) { return n <= (int64_t)kClusterMost * kClusterThreads ? 1 : 2; }
+inline int cluster_blocks(int64_t n) {
+    const int64_t tile = (int64_t)cluster_items(n) * kClusterThreads;
+    int blocks = 1;
+    while (blocks * tile < n) blocks *= 2;
+    return blocks;
+}
+
+// cluster_sorts() has set the kernel's attributes.
 template <int kSrc>
 cudaError_t launch_cluster_sort(cudaStream_t st, bool chained, const double2* pos, int64_t n,
                                 DeviceScalars* s, int adaptive, int new_step, int fixed_passes,
                                 const uint64_t* key_in, uint64_t* key_out, uint32_t* val_out,
                                 unsigned long long* mark0, unsigned long long* mark1) {
-    const int items = n <= (int64_t)kClusterMost * kClusterThreads ? 1 : 2;
-    const int tiles = (int)((n + items * kClusterThreads - 1) / (items * kClusterThreads));
-    int cluster = 1;
-    while (cluster < tiles) cluster *= 2;
-    auto* launch = items == 1 ? launch_cluster<1, kSrc> : launch_cluster<2, kSrc>;
-    return launch(st, chained, cluster, cluster, pos, n, s, adaptive, new_step, fixed_passes, key_in,
-                  key_out, val_out, mark0, mark1);
+    const bool one = cluster_items(n) == 1;
+    const int blocks = cluster_blocks(n);
+    return chain_launch(st, chained, one ? cluster_sort<1, kSrc> : cluster_sort<2, kSrc>, blocks,
+                        kClusterThreads, one ? sizeof(ClusterSmem<1>) : sizeof(ClusterSmem<2>), blocks,
+                        pos, n, s, adaptive, new_step, fixed_passes, key_in, key_out, val_out, mark0,
+                        mark1);
+}
+
+// Sets a kernel's attributes and asks whether one cluster of it fits the device.
+template <int kItems, int kSrc>
+bool cluster_fits(int blocks) {
+    auto* kernel = cluster_sort<kItems, kSrc>;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)blocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = blocks;
+    cfg.blockDim = kClusterThreads;
+    cfg.dynamicSmemBytes = sizeof(ClusterSmem<kItems>);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess)
+        return clusters > 0;
+    cudaGetLastError();  // answered: the caller sorts by passes over global memory
+    return false;
 }
 
 inline bool by_cluster(const nb_ctx* c) { return c->sort.hist == nullptr; }
 
 }  // namespace
 
-// The largest clusters that the sort launches must fit the device.
-int64_t cluster_sort_size() {
-    auto* kernel = cluster_sort<2, kSrcBodies>;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kClusterMost;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = kClusterMost;
-    cfg.blockDim = kClusterThreads;
-    cfg.dynamicSmemBytes = sizeof(ClusterSmem<2>);
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)cfg.dynamicSmemBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess)
-        clusters = 0;
-    return clusters > 0 ? kClusterSortMax : 0;
+bool cluster_sorts(int64_t n, bool from_keys) {
+    if (n > kClusterSortMax) return false;
+    const bool one = cluster_items(n) == 1;
+    auto* fits = from_keys ? (one ? cluster_fits<1, kSrcKeys> : cluster_fits<2, kSrcKeys>)
+                           : (one ? cluster_fits<1, kSrcBodies> : cluster_fits<2, kSrcBodies>);
+    return fits(cluster_blocks(n));
 }
 
 void launch_bbox(nb_ctx* c, const double2* pos, bool new_step) {
@@ -1494,7 +1496,7 @@ cudaError_t launch_morton_sort_raw(const double2* pos, int64_t n, uint64_t* cons
                                    uint32_t* const val[2], uint64_t* key_out, uint32_t* val_out,
                                    uint16_t* counts, double* partials, int bbox_blocks,
                                    DeviceScalars* scal, cudaStream_t st) {
-    if (n <= cluster_sort_size())
+    if (cluster_sorts(n, false))
         return launch_cluster_sort<kSrcBodies>(st, false, pos, n, scal, 0, 0, 8, nullptr, key_out,
                                                val_out, nullptr, nullptr);
     const int tiles = (int)count_tiles(n);

@@ -61,7 +61,7 @@ int check_params(const nb_params* p) {
     return NB_OK;
 }
 
-int alloc_all(nb_ctx* c) {
+int alloc_all(nb_ctx* c, bool batch) {
     const size_t n = (size_t)c->n;
     for (int k = 0; k < 2; ++k) {
         NB_CUDA(c, dalloc(&c->buf[k].pos, n));
@@ -73,7 +73,7 @@ int alloc_all(nb_ctx* c) {
     }
     const int tile_keys = nb::sort_tile_items(c->n, c->sm_count) * nb::kSortThreads;
     c->sort.tiles = (int)((n + tile_keys - 1) / tile_keys);
-    if (c->n > nb::cluster_sort_size()) {  // onesweep passes
+    if (!nb::cluster_sorts(c->n, batch)) {  // onesweep passes
         NB_CUDA(c, dalloc(&c->sort.hist, 8 * 256));
         NB_CUDA(c, dalloc(&c->sort.status, (size_t)8 * 256 * nb::sort_status_rows(c->sort.tiles)));
         NB_CUDA(c, dalloc(&c->sort.tile_counter, 8));
@@ -442,7 +442,7 @@ int create_context(const nb_params* p, uint64_t n, const double* mass, const dou
         cudaEventCreateWithFlags(&c->copied, cudaEventDisableTiming) != cudaSuccess) {
         rc = NB_ERR_CUDA;
     }
-    if (rc == NB_OK) rc = alloc_all(c);
+    if (rc == NB_OK) rc = alloc_all(c, counts != nullptr);
     if (rc == NB_OK && counts) rc = alloc_batch(c, nuni, counts);
     if (rc == NB_OK) rc = nb_upload(c, mass, pos_xy, vel_xy);
     if (rc != NB_OK) {

@@ -420,10 +420,11 @@ void launch_scatter(nb_ctx* c, const BodyBuffers& b, double2* out_pos, double2* 
 void launch_identity(nb_ctx* c, int32_t* orig);
 
 // Up to kClusterSortMax bodies are sorted by one cluster of blocks that holds
-// all keys in shared memory; cluster_sort_size() is the most that this device
-// sorts so (0 where it cannot run such a cluster).
+// all keys in shared memory.  cluster_sorts() says whether the current device
+// can run the cluster that n bodies take, from their positions or (batched
+// universes) from keys, and readies the kernel for its launches there.
 constexpr int64_t kClusterSortMax = 32768;
-int64_t cluster_sort_size();
+bool cluster_sorts(int64_t n, bool from_keys);
 
 // The bounding-box, Morton and radix-sort stage on caller-provided buffers
 // (no context): key/val ping-pong scratch of n entries each, counts of

@@ -13,7 +13,9 @@ enum { CALL_LAUNCH, CALL_ATTRIBUTE, CALL_CLUSTERS, CALL_KINDS };
 static cudaError_t last_error = cudaSuccess;
 static long calls[CALL_KINDS];
 static long fail_at[CALL_KINDS] = {-1, -1, -1}; /* index of the call that fails, -1: none */
-static long open_captures, live_graphs, graph_launches;
+static long open_captures, live_graphs, graph_launches, unprobed_clusters;
+static const void* probed[16]; /* kernels that occupancy was asked for, in clusters */
+static int probes;
 
 static cudaError_t done(cudaError_t e) {
     if (e != cudaSuccess) last_error = e;
@@ -27,13 +29,17 @@ static cudaError_t counted(int kind, cudaError_t e) {
 API void fake_reset(void) {
     for (int k = 0; k < CALL_KINDS; ++k) calls[k] = 0, fail_at[k] = -1;
     last_error = cudaSuccess;
+    unprobed_clusters = 0;
 }
+API void fake_forget_probes(void) { probes = 0; }
 API void fake_fail(int kind, long index) { fail_at[kind] = index; }
 API long fake_calls(int kind) { return calls[kind]; }
 API int fake_last_error(void) { return last_error; }
 API long fake_open_captures(void) { return open_captures; }
 API long fake_live_graphs(void) { return live_graphs; }
 API long fake_graph_launches(void) { return graph_launches; }
+/* launches of a cluster of blocks whose kernel has not been asked for */
+API long fake_unprobed_clusters(void) { return unprobed_clusters; }
 
 /* what compiled .cu objects register */
 void** __cudaRegisterFatBinary(void* f) { (void)f; return calloc(1, sizeof(void*)); }
@@ -61,7 +67,13 @@ cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** a, size_t s, 
     return counted(CALL_LAUNCH, cudaErrorLaunchOutOfResources);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) {
-    (void)c, (void)f, (void)a;
+    (void)a;
+    for (unsigned k = 0; k < c->numAttrs; ++k)
+        if (c->attrs[k].id == cudaLaunchAttributeClusterDimension) {
+            int known = 0;
+            for (int q = 0; q < probes; ++q) known |= probed[q] == f;
+            unprobed_clusters += !known;
+        }
     return counted(CALL_LAUNCH, cudaErrorLaunchOutOfResources);
 }
 cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v) {
@@ -69,7 +81,8 @@ cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v)
     return counted(CALL_ATTRIBUTE, cudaErrorInvalidValue);
 }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void* f, const cudaLaunchConfig_t* c) {
-    (void)f, (void)c;
+    (void)c;
+    if (probes < 16) probed[probes++] = f;
     *n = 0;
     const cudaError_t e = counted(CALL_CLUSTERS, cudaErrorInvalidClusterSize);
     if (e == cudaSuccess) *n = 8;

@@ -47,7 +47,7 @@ KINDS = {
 
 
 class Context:
-    def __init__(self, nbp, lib, kind):
+    def __init__(self, nbp, lib, kind, fail=None):
         mode, flags, n, universes = KINDS[kind]
         p = nbp.NbParams()
         lib.nb_params_default(C.byref(p))
@@ -55,6 +55,9 @@ class Context:
         self.lib, self.h, self.n = lib, C.c_void_p(), n
         m, x = np.ones(n), np.zeros((n, 2))
         lib.fake_reset()
+        lib.fake_forget_probes()
+        if fail:
+            lib.fake_fail(*fail)
         args = (m.ctypes.data_as(C.c_void_p), x.ctypes.data_as(C.c_void_p),
                 x.ctypes.data_as(C.c_void_p), C.byref(self.h))
         if universes:
@@ -66,6 +69,7 @@ class Context:
         if flags & 2:
             w = np.zeros(5123, np.float32)
             assert lib.nb_set_mlp_weights(self.h, w.ctypes.data_as(C.c_void_p)) == 0
+        assert lib.fake_last_error() == 0  # nothing left for the next call to trip over
         lib.fake_reset()
 
     def __enter__(self):
@@ -98,3 +102,43 @@ def test_a_failed_launch_fails_the_step(nbp, fake, kind):
                 assert ctx.step(3) == 0
                 assert fake.fake_graph_launches() == launched + 3
 
+
+@pytest.mark.parametrize("kind", [k for k in KINDS if KINDS[k][2] <= 32768 and KINDS[k][0] < 2])
+def test_without_clusters_the_sort_takes_passes(nbp, fake, kind):
+    """A device that cannot run the cluster sort (or an error while asking)."""
+    with Context(nbp, fake, kind) as ctx:
+        assert ctx.step() == 0
+        clustered = fake.fake_calls(LAUNCH)
+    for what, k in ((CLUSTERS, 0), (ATTRIBUTE, 0), (ATTRIBUTE, 1)):
+        with Context(nbp, fake, kind, fail=(what, k)) as ctx:
+            assert ctx.step() == 0
+            assert fake.fake_calls(LAUNCH) > clustered
+
+
+@pytest.mark.parametrize("n", [1025, 16384, 16385, 32768])
+@pytest.mark.parametrize("universes", [0, 4])
+def test_the_cluster_kernel_that_runs_was_asked_for(nbp, fake, n, universes):
+    KINDS["probe"] = (1, 0, n - n % max(1, universes), universes)
+    with Context(nbp, fake, "probe") as ctx:
+        assert ctx.step() == 0
+        assert fake.fake_unprobed_clusters() == 0
+    del KINDS["probe"]
+
+
+@pytest.mark.parametrize("n", [1000, 32768, 32769, 262144])
+def test_static_sort_asks_once_where_a_cluster_can_sort(fake, n):
+    buf = (C.c_double * (2 * n))()
+    out, order = (C.c_uint64 * n)(), (C.c_int32 * n)()
+    fake.fake_reset()
+    assert fake.nb_morton_sort_static(buf, C.c_uint64(n), out, order, None, None) == 0
+    assert fake.fake_calls(CLUSTERS) == (n <= 32768)
+    assert fake.fake_calls(ATTRIBUTE) == (2 if n <= 32768 else 0)
+    if n <= 32768:  # cannot: the counting passes, and no error left
+        for what in (CLUSTERS, ATTRIBUTE):
+            fake.fake_reset()
+            fake.fake_fail(what, 0)
+            assert fake.nb_morton_sort_static(buf, C.c_uint64(n), out, order, None, None) == 0
+            assert fake.fake_calls(LAUNCH) == 18 and fake.fake_last_error() == 0
+    fake.fake_reset()
+    fake.fake_fail(LAUNCH, 0)
+    assert fake.nb_morton_sort_static(buf, C.c_uint64(n), out, order, None, None) == NB_ERR_CUDA
