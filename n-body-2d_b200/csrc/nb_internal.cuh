@@ -193,7 +193,6 @@ struct nb_ctx {
     nb::SortBuffers sort;
     nb::Tree tree;
     nb::DeviceScalars* scal = nullptr;   // device
-    unsigned* host_error = nullptr;      // pinned: scal->error as last copied out
     double* bbox_partials = nullptr;     // [blocks][4]
     int bbox_blocks = 0;
     int split_blocks[64] = {};            // persistent grids of the SPLIT traversal variants

@@ -8,11 +8,11 @@
 
 #define API __attribute__((visibility("default")))
 
-enum { CALL_LAUNCH, CALL_ATTRIBUTE, CALL_CLUSTERS, CALL_KINDS };
+enum { CALL_LAUNCH, CALL_ATTRIBUTE, CALL_CLUSTERS, CALL_HOST_ALLOC, CALL_SYNC, CALL_KINDS };
 
 static cudaError_t last_error = cudaSuccess;
 static long calls[CALL_KINDS];
-static long fail_at[CALL_KINDS] = {-1, -1, -1}; /* index of the call that fails, -1: none */
+static long fail_at[CALL_KINDS] = {-1, -1, -1, -1, -1}; /* index of the call that fails, -1: none */
 static long open_captures, live_graphs, graph_launches, unprobed_clusters;
 static const void* probed[16]; /* kernels that occupancy was asked for, in clusters */
 static int probes;
@@ -115,8 +115,12 @@ cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr a, int d) {
 cudaError_t cudaMalloc(void** p, size_t n) {
     return done((*p = calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation);
 }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned f) { (void)f; return cudaMalloc(p, n); }
-cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned f) {
+    (void)f;
+    const cudaError_t e = counted(CALL_HOST_ALLOC, cudaErrorMemoryAllocation);
+    return e == cudaSuccess ? cudaMalloc(p, n) : e;
+}
+cudaError_t cudaMallocHost(void** p, size_t n) { return cudaHostAlloc(p, n, 0); }
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, enum cudaMemcpyKind k) {
@@ -154,7 +158,10 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned f) {
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    (void)s;
+    return counted(CALL_SYNC, cudaErrorLaunchFailure);
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) {
     (void)s, (void)e, (void)f;
     return cudaSuccess;

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 HERE = pathlib.Path(__file__).resolve().parent
-LAUNCH, ATTRIBUTE, CLUSTERS = range(3)
+LAUNCH, ATTRIBUTE, CLUSTERS, HOST_ALLOC, SYNC = range(5)
 NB_ERR_CUDA = 2
 
 
@@ -66,6 +66,7 @@ class Context:
         else:
             rc = lib.nb_create(C.byref(p), C.c_uint64(n), *args)
         assert rc == 0
+        self.host_allocs = lib.fake_calls(HOST_ALLOC)
         if flags & 2:
             w = np.zeros(5123, np.float32)
             assert lib.nb_set_mlp_weights(self.h, w.ctypes.data_as(C.c_void_p)) == 0
@@ -142,3 +143,17 @@ def test_static_sort_asks_once_where_a_cluster_can_sort(fake, n):
     fake.fake_reset()
     fake.fake_fail(LAUNCH, 0)
     assert fake.nb_morton_sort_static(buf, C.c_uint64(n), out, order, None, None) == NB_ERR_CUDA
+
+
+@pytest.mark.parametrize("kind", ["fp64 cluster", "split onesweep", "allpairs"])
+def test_a_context_pins_no_memory_and_a_download_waits_once(nbp, fake, kind):
+    """Pinned memory costs a context some 4 ms to get and to give back."""
+    with Context(nbp, fake, kind) as ctx:
+        assert ctx.host_allocs == 0
+        assert ctx.step() == 0
+        out = np.empty((ctx.n, 2))
+        fake.fake_reset()
+        assert fake.nb_download(ctx.h, out.ctypes.data_as(C.c_void_p), None) == 0
+        assert fake.fake_calls(SYNC) == 1
+        fake.fake_fail(SYNC, 1)  # what a failed kernel looks like to the host
+        assert fake.nb_download(ctx.h, out.ctypes.data_as(C.c_void_p), None) == NB_ERR_CUDA
