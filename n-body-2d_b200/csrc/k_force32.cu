@@ -616,7 +616,7 @@ void launch_split_kernel(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_
     // eps2 below the smallest normal float is treated like eps2 = 0
     const float eps2 = (float)c->p.epsilon_squared;
     constexpr bool kCanShare = kBPL == 1 && !kLearned;
-    const bool share = kCanShare && c->n <= kShareMax;
+    const bool share = kCanShare && bodies_on_148(c) <= kShareMax;
     if (eps2 >= FLT_MIN)
         share ? launch_split_soft<kQuad, kBPL, kLearned, false, kCanShare>(c, b, kick, store_acc, chained, eps2)
               : launch_split_soft<kQuad, kBPL, kLearned, false, false>(c, b, kick, store_acc, chained, eps2);

@@ -556,15 +556,18 @@ inline unsigned blocks_for(int64_t n, int threads) {
 void launch_force_fp64(nb_ctx* c, const BodyBuffers& b, bool kick, bool store_acc) {
     c->launches += 1;
     if (c->want_terms) return launch_walk64<32, true>(c, b, kick, store_acc);
-    // As few bodies per warp as keep the walk to one wave of resident warps
-    // (4,144 = 148 SMs x 28): a warp's walk is a chain of dependent loads, which
-    // a smaller group shortens, while a larger one shares each node among more
-    // bodies.  us at kG = 1 / 4 / 16 / 32: 1,001 bodies 26 / 32 / 45 / 63; 16,384
-    // 122 / 55 / 73 / 96; 65,536 624 / 206 / 120 / 132; 262,144 2212 / 665 / 358 /
-    // 303; 1,048,576 10599 / 2732 / 1351 / 1058 (one thread per body before: 303,
-    // 486, -, 1225, 3596; with a node's loads issued together the chosen sizes now
-    // take 19, 49, 117, - and 1037).
-    const int64_t per_warp = c->n / 4096;
+    // A warp's walk is a chain of dependent loads, which a smaller group shortens,
+    // while a larger one shares each node among more bodies: few enough bodies per
+    // warp that the walk is between one and two waves of the resident warps (4,144
+    // = 148 SMs x 28), two just below each switch.  Force, us, at kG = 1 / 2 / 4 / 8
+    // / 16 / 32, Plummer disc: 6,000 bodies 53 / 36 / 36 / 45 / 64 / 80; 8,191 61 /
+    // 42 / 41 / 48 / 69 / 82; 16,383 128 / 83 / 54 / 55 / 76 / 88; 32,767 293 / 174 /
+    // 104 / 74 / 89 / 101; 65,535 681 / 388 / 226 / 147 / 120 / 127; 131,071 1529 /
+    // 840 / 474 / 292 / 218 / 186; 200,003 2456 / 1330 / 737 / 446 / 317 / 269.  The
+    // next size would be the quicker one from about two thirds of the way to its
+    // switch on (at 8,191 41 instead of 61, at 32,767 74 instead of 104).  1,048,576
+    // bodies take 1,037 at kG = 32, 3,596 with one thread per body.
+    const int64_t per_warp = bodies_on_148(c) / 4096;
     if (per_warp < 2) return launch_walk64<1, false>(c, b, kick, store_acc);
     if (per_warp < 4) return launch_walk64<2, false>(c, b, kick, store_acc);
     if (per_warp < 8) return launch_walk64<4, false>(c, b, kick, store_acc);

@@ -132,7 +132,6 @@ constexpr int kFewTiles = 64;
 // kBlock threads per tile: 1,024 while every SM has at most one tile (a warp's
 // rows follow one another), else 256.
 constexpr int kWideThreads = 1024;
-constexpr int kWideTiles = 148;
 
 template <int kBlock>
 __global__ void __launch_bounds__(kBlock)
@@ -1624,7 +1623,7 @@ void launch_tree(nb_ctx* c, const BodyBuffers& b) {
     const bool few = tiles <= kFewTiles;
     c->launches += few ? 3 : 4;
     const TileTable tab{t.ansv_first, t.ansv_last, few ? 1 : tiles, few ? kAnsvLevels : 1};
-    const bool wide = tiles <= kWideTiles;
+    const bool wide = tiles <= c->sm_count;
     chain_launch(c->stream, true, wide ? tree_lcp<kWideThreads> : tree_lcp<kThreads>, tiles,
                  wide ? kWideThreads : kThreads, 0, 1, key, n, t.lcp8, tab, c->scal->lcp_hist,
                  mark_of(c, 4));

@@ -234,6 +234,10 @@ struct nb_ctx {
 
 namespace nb {
 
+// Rules that weigh bodies against SMs were measured on the B200's 148: the
+// number of bodies that would be as many per SM there.
+inline int64_t bodies_on_148(const nb_ctx* c) { return c->n * 148 / c->sm_count; }
+
 // Learned mode: opening angle of the plain walk whose extra openings the
 // network replaces (band cells: accepted at theta, opened at this angle).
 inline float band_theta(const nb_ctx* c) {

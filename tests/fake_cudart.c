@@ -16,6 +16,8 @@ static long fail_at[CALL_KINDS] = {-1, -1, -1, -1, -1}; /* index of the call tha
 static long open_captures, live_graphs, graph_launches, unprobed_clusters;
 static const void* probed[16]; /* kernels that occupancy was asked for, in clusters */
 static int probes;
+static struct { const void* kernel; unsigned grid, block; } launched[256]; /* since the reset */
+static int sms = 148;
 
 static cudaError_t done(cudaError_t e) {
     if (e != cudaSuccess) last_error = e;
@@ -32,6 +34,10 @@ API void fake_reset(void) {
     unprobed_clusters = 0;
 }
 API void fake_forget_probes(void) { probes = 0; }
+API void fake_set_sms(int n) { sms = n; }
+API const void* fake_launched(int k) { return launched[k].kernel; }
+API unsigned fake_grid(int k) { return launched[k].grid; }
+API unsigned fake_block(int k) { return launched[k].block; }
 API void fake_fail(int kind, long index) { fail_at[kind] = index; }
 API long fake_calls(int kind) { return calls[kind]; }
 API int fake_last_error(void) { return last_error; }
@@ -68,6 +74,11 @@ cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** a, size_t s, 
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) {
     (void)a;
+    if (calls[CALL_LAUNCH] < 256) {
+        launched[calls[CALL_LAUNCH]].kernel = f;
+        launched[calls[CALL_LAUNCH]].grid = c->gridDim.x;
+        launched[calls[CALL_LAUNCH]].block = c->blockDim.x;
+    }
     for (unsigned k = 0; k < c->numAttrs; ++k)
         if (c->attrs[k].id == cudaLaunchAttributeClusterDimension) {
             int known = 0;
@@ -107,7 +118,7 @@ cudaError_t cudaSetDevice(int d) { (void)d; return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr a, int d) {
     (void)a, (void)d;
-    *v = 148;
+    *v = sms;
     return cudaSuccess;
 }
 

@@ -31,6 +31,7 @@ def fake(nbp, tmp_path_factory):
     lib.nb_last_error.argtypes = [C.c_void_p]
     lib.fake_calls.restype = C.c_long
     lib.fake_fail.argtypes = [C.c_int, C.c_long]
+    lib.fake_launched.restype = C.c_void_p
     return lib
 
 
@@ -157,3 +158,32 @@ def test_a_context_pins_no_memory_and_a_download_waits_once(nbp, fake, kind):
         assert fake.fake_calls(SYNC) == 1
         fake.fake_fail(SYNC, 1)  # what a failed kernel looks like to the host
         assert fake.nb_download(ctx.h, out.ctypes.data_as(C.c_void_p), None) == NB_ERR_CUDA
+
+
+def launches_on(nbp, fake, sms, mode, n):
+    """(kernel, blocks, threads) of a step's launches on a device of so many SMs."""
+    KINDS["sms"] = (mode, 0, n, 0)
+    fake.fake_set_sms(sms)
+    try:
+        with Context(nbp, fake, "sms") as ctx:
+            assert ctx.step() == 0
+            per_step = fake.fake_calls(LAUNCH) // 2  # both parities were captured
+            return [(fake.fake_launched(k), fake.fake_grid(k), fake.fake_block(k))
+                    for k in range(per_step)]
+    finally:
+        fake.fake_set_sms(148)
+        del KINDS["sms"]
+
+
+@pytest.mark.parametrize("mode,n", [(0, 9000), (0, 40000), (0, 100000), (0, 250000), (1, 20000),
+                                    (1, 250000)])
+def test_rules_follow_the_sms(nbp, fake, mode, n):
+    """Half the SMs take n bodies as all of them take 2 n: the same walk, bodies
+    per warp, and threads per tile of the tree (where the rules end differs)."""
+    def rules(sms, n):
+        launches = launches_on(nbp, fake, sms, mode, n)
+        walk = max(k for k, (_, _, threads) in enumerate(launches) if threads == 128)
+        tiles = -(-n // 2048)
+        return launches[walk][0], any(launch[1:] == (tiles, 1024) for launch in launches[2:])
+    assert rules(74, n) == rules(148, 2 * n)
+    assert rules(74, n) != rules(148, n)
