@@ -74,12 +74,6 @@ __device__ __forceinline__ void put_entry(float4* xy, float2* m, int slot, float
     reinterpret_cast<float*>(m)[slot] = mass;
 }
 
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
 __device__ __forceinline__ int warp_exclusive_sum(int v, int& total) {
     const int lane = threadIdx.x & 31;
     int inc = v;

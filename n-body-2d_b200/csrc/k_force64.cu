@@ -37,26 +37,6 @@ struct Walk64 {
     double nw[32];               //   and squared width
 };
 
-// Lane v receives bit v of every lane's word x (bit l from lane l).
-__device__ __forceinline__ unsigned warp_transpose_bits(unsigned x) {
-    const int lane = threadIdx.x & 31;
-    constexpr unsigned keep[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const int j = 16 >> k;
-        const unsigned p = __shfl_xor_sync(kFull, x, j);
-        x = (lane & j) ? (x & ~keep[k]) | ((p >> j) & keep[k])
-                       : (x & keep[k]) | ((p << j) & ~keep[k]);
-    }
-    return x;
-}
-
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
 // The reference's squared distance (nvcc contracts CU:461 to this fma).
 // Rounding is monotone, so it never decreases when |dx| or |dy| grows.
 __device__ __forceinline__ double dist2(double dx, double dy) {

@@ -387,12 +387,6 @@ __global__ void morton_batch_kernel(const double2* pos, int64_t n, Batch b,
 // ---------------------------------------------------------------------------
 constexpr int kWarps = kSortThreads / 32;
 
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
 // Exclusive scan of one value per thread over a 256-thread block.
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* warp_tot,
                                                          uint32_t* total) {

@@ -90,28 +90,6 @@ constexpr int kAnsvRows = kAnsvTile / 32;           // 64 rows
 constexpr int kNoLevel = kMaxLevel + 1;             // past the last body: never below a level
 static_assert(kAnsvItems == 8 && kAnsvLevels == 32, "one lane per level, 8 rows per warp");
 
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
-// Lane v receives bit v of every lane's word x (bit l from lane l): the 32 x
-// 32 bit matrix of the warp's words transposed by swapping off-diagonal
-// blocks of 16, 8, 4, 2 and 1 between lane pairs.
-__device__ __forceinline__ unsigned warp_transpose_bits(unsigned x) {
-    const int lane = threadIdx.x & 31;
-    constexpr unsigned keep[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const int j = 16 >> k;
-        const unsigned p = __shfl_xor_sync(kFull, x, j);
-        x = (lane & j) ? (x & ~keep[k]) | ((p >> j) & keep[k])
-                       : (x & keep[k]) | ((p << j) & ~keep[k]);
-    }
-    return x;
-}
-
 // Bit v set for every v above level c (v = 0..31).
 __device__ __forceinline__ unsigned thermometer(int c) {
     return c >= 31 ? 0u : (0xFFFFFFFFu << (c + 1));

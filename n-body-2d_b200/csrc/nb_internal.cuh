@@ -13,7 +13,6 @@
 namespace nb {
 
 constexpr int kMaxLevel = 30;     // level-30 cells are leaves (BarnesHutCuda.cu:182)
-constexpr int kStackDepth = 96;   // >= 1 + 3 * 30 pending cells of a DFS
 constexpr int kSortThreads = 256;
 constexpr int kSortItemsMax = 12;
 // Keys per thread of a radix tile: 4 up to one tile of 1,024 keys per SM, 8 up to
@@ -304,6 +303,28 @@ __device__ __forceinline__ int choose_sort_passes(const unsigned* hist, int64_t 
     const bool few = (lane & 3) == 0 && lane >= 4 && from * 32 <= (unsigned long long)n;
     const unsigned ok = __ballot_sync(0xffffffffu, few);
     return ok ? (__ffs(ok) - 1) / 4 : 8;
+}
+
+__device__ __forceinline__ unsigned lanemask_lt() {
+    unsigned m;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
+}
+
+// Lane v receives bit v of every lane's word x (bit l from lane l): the 32 x
+// 32 bit matrix of the warp's words transposed by swapping off-diagonal
+// blocks of 16, 8, 4, 2 and 1 between lane pairs.
+__device__ __forceinline__ unsigned warp_transpose_bits(unsigned x) {
+    const int lane = threadIdx.x & 31;
+    constexpr unsigned keep[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const int j = 16 >> k;
+        const unsigned p = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? (x & ~keep[k]) | ((p >> j) & keep[k])
+                       : (x & keep[k]) | ((p << j) & ~keep[k]);
+    }
+    return x;
 }
 
 // ---- the step's kernel chain ----------------------------------------------
