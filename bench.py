@@ -83,11 +83,11 @@ def _package():
 
 # DRAM bytes one launch of the SPLIT monopole force kernel moves per body:
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one force_split launch
-# on the 1,048,576-body collision (83.6 MB + 12.3 MB = 95.9 MB, --clock-control
+# on the 1,048,576-body collision (85.2 MB + 11.9 MB = 97.1 MB, --clock-control
 # none).  Bodies and cells both grow linearly with N, so the figure scales by
 # N; it is a property of the kernel's access pattern, re-measured when the
 # kernel changes.
-FORCE_TRAFFIC_BYTES_PER_BODY = 95.9e6 / 1048576
+FORCE_TRAFFIC_BYTES_PER_BODY = 97.1e6 / 1048576
 
 
 def _peaks() -> tuple[dict, str]:
@@ -159,7 +159,11 @@ class ClockSampler:
             self.stop = threading.Event()
             self.thread = threading.Thread(target=self._poll, args=(pynvml, h), daemon=True)
             self.thread.start()
-            time.sleep(0.05)
+            # the first query of a fresh box can take longer than the timed region
+            limit = time.time() + 2.0
+            while not self.samples and self.thread.is_alive() and time.time() < limit:
+                time.sleep(0.005)
+            time.sleep(0.02)
             return self
         except Exception:
             self.nvml = None
