@@ -40,10 +40,10 @@ __device__ __forceinline__ double pair_weight_any(double m, double r2, double ep
 
 // Sums the sources [s0, s1) for the block's targets, kPer per thread: target
 // b of a thread is p[b], and self[b] its own source index, which is left out.
-// 13 FP64 instructions per pair (22 with the CPU law), each two issue cycles:
-// the FP64 pipe is the bound (1 / sqrt and its division took some 35: 65,536
-// targets of 1,048,576 bodies with their copies 205 -> 70 ms; a step of 20,011
-// bodies 0.92 -> 0.38 ms).  Several targets per thread share the loads and
+// 14 FP64 instructions per pair (15 and a second seed with the CPU law), each
+// two issue cycles: the FP64 pipe is the bound, 87% of its cycles active (1 /
+// sqrt and its division took some 35 instructions: 65,536 targets of 1,048,576
+// bodies with their copies 205 -> 66 ms; a step of 20,011 bodies 0.92 -> 0.37 ms).  Several targets per thread share the loads and
 // the loop.  Only a tile that holds one of the warp's own sources tests for
 // it; a tile whose sums are not finite (a square that is zero, subnormal or
 // infinite, or a term that overflows) is summed again with full-range functions.

@@ -64,10 +64,11 @@ __device__ __forceinline__ void plummer(double dx, double dy, double m, double e
 // Accepted nodes go to a shared-memory list, which the warp sums 32 entries at
 // a time: lane = (list slot, body), 32 / kG slots side by side.
 //
-// Bound by the FP64 pipe (13 instructions per body and list entry, each two
-// issue cycles).  One thread per body and one node at a time kept the pipe at
-// 16% and 18 of 32 lanes active: scattered loads behind every step of a serial
-// walk.
+// At 1M bodies issue is at 70% and the FP64 pipe at 50% of its cycles (14
+// instructions per body and list entry, each two issue cycles, and the opening
+// tests): no unit is full, fixed latencies and turns at issue take the rest.  One
+// thread per body and one node at a time kept the pipe at 16% and 18 of 32 lanes
+// active: scattered loads behind every step of a serial walk.
 // kTerms (nb_debug_interactions): per-body interaction counts and the depth
 // a depth-first walk's stack would reach.  A node's pending count (siblings
 // waiting at and above it) is a property of its path, so each node carries it.
