@@ -21,6 +21,7 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kBoxThreads = 512;
+constexpr double kBoxSeed = 1.7976931348623157e308;  // DBL_MAX
 
 __device__ __forceinline__ double warp_min(double v) {
     for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(kFull, v, o));
@@ -168,8 +169,7 @@ bbox_kernel(const double2* pos, int64_t n, double* partials,
     if (!last_block) return;
     __threadfence();
     // CU:649-654 seeds with +-DBL_MAX; folding from there is identical.
-    double bx0 = 1.7976931348623157e308, bx1 = -1.7976931348623157e308;
-    double by0 = 1.7976931348623157e308, by1 = -1.7976931348623157e308;
+    double bx0 = kBoxSeed, bx1 = -kBoxSeed, by0 = kBoxSeed, by1 = -kBoxSeed;
     for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
         const double* in = partials + 4 * b;
         bx0 = fmin(bx0, __ldcg(in + 0));
@@ -537,7 +537,9 @@ cluster_sort(const double2* pos, int64_t n, DeviceScalars* s, int adaptive,
             p[k] = first + 32 * k < n ? pos[first + 32 * k] : make_double2(0.0, 0.0);
         RootBox box;
         {
-            double v[4] = {INFINITY, -INFINITY, INFINITY, -INFINITY};
+            // (CU:649-654 seeds with +-DBL_MAX, which show where an axis has no
+            // finite value: nb_morton_sort_static takes any positions)
+            double v[4] = {kBoxSeed, -kBoxSeed, kBoxSeed, -kBoxSeed};
 #pragma unroll
             for (int k = 0; k < kItems; ++k)
                 if (first + 32 * k < n) {
