@@ -21,14 +21,13 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kTile = 256;    // sources staged in shared memory at a time
 
-using nb::m_over_r3;
-
 // Pair weight w of a_i += w (p_j - p_i).  kCpuLaw: the law of
 // Simulation::force, m / (d (d^2 + eps2)) (Simulation.cpp:74-80, G applied
 // with the kick); otherwise Plummer's m (d^2 + eps2)^-3/2.
 template <bool kCpuLaw>
 __device__ __forceinline__ double pair_weight(double m, double r2, double eps2) {
-    return kCpuLaw ? nb::m_over_r_s(m, r2, r2 + eps2) : m_over_r3(m, r2 + eps2);
+    return kCpuLaw ? nb::m_over_r_s(m, r2, r2 + eps2)
+                   : nb::m_over_r3<false>(m, r2 + eps2);
 }
 // The same for any r2: zero, subnormal or infinite squares.
 template <bool kCpuLaw>

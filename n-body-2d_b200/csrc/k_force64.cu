@@ -46,7 +46,7 @@ __device__ __forceinline__ double dist2(double dx, double dy) {
 __device__ __forceinline__ void plummer(double dx, double dy, double m, double eps2, double& ax,
                                         double& ay) {
     const double d2 = dist2(dx, dy) + eps2;
-    double a = m_over_r3(m, d2);
+    double a = m_over_r3<true>(m, d2);
     if (!isfinite(a)) a = m_over_r3_any(m, d2);
     ax += dx * a;
     ay += dy * a;
@@ -140,7 +140,7 @@ force_fp64(const double2* pos, const double* mass, double2* vel,
         for (int k = slot; k < cnt; k += kSlots) {
             const double2 p = L.fxy[k];
             const double dx = p.x - me.x, dy = p.y - me.y;
-            const double a = m_over_r3(L.fm[k], dist2(dx, dy) + eps2);
+            const double a = m_over_r3<true>(L.fm[k], dist2(dx, dy) + eps2);
             if (!kMasked || ((L.mask[k] >> body) & 1u)) {
                 ax = fma(dx, a, ax);
                 ay = fma(dy, a, ay);
@@ -180,7 +180,7 @@ force_fp64(const double2* pos, const double* mass, double2* vel,
             mine &= mine - 1;
             const double2 p = L.pxy[k];
             const double dx = p.x - me.x, dy = p.y - me.y;
-            const double a = m_over_r3(L.pm[k], dist2(dx, dy) + eps2);
+            const double a = m_over_r3<true>(L.pm[k], dist2(dx, dy) + eps2);
             ax = fma(dx, a, ax);
             ay = fma(dy, a, ay);
         }

@@ -261,13 +261,17 @@ __device__ __forceinline__ double cell_width2(const DeviceScalars* s, const Batc
 // second-order term; e^3 is below 2^-57.  Seven FP64 instructions.  y has so
 // few bits that y^2 is exact, so e carries one rounding.  A zero, subnormal or
 // infinite r^2 and an overflow give an infinity or NaN (inf * e - inf), never a
-// finite value: m_over_r3_any() then says which.
+// finite value: m_over_r3_any() then says which.  kMassLast: r^-3 is formed
+// first and over- and underflows by itself, as in the reference's GPU law
+// (CU:428-430), which the FP64 walk follows; otherwise only m r^-3 does, as in
+// the all-pairs sums' m / r / r / r.
+template <bool kMassLast>
 __device__ __forceinline__ double m_over_r3(double m, double r2) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
     const double t = __dmul_rn(y, y);
     const double e = __fma_rn(-r2, t, 1.0);
-    const double w = __dmul_rn(__dmul_rn(m, y), t);
+    const double w = kMassLast ? __dmul_rn(m, __dmul_rn(y, t)) : __dmul_rn(__dmul_rn(m, y), t);
     return __fma_rn(w, __dmul_rn(e, __fma_rn(1.875, e, 1.5)), w);
 }
 // m / (sqrt(r2) s), s > 0 normal (FP64): approximate 1/sqrt and reciprocal, then
